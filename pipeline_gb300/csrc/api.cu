@@ -409,8 +409,9 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
           "build: radix tree");
   mark(rec, s);
   const OctTags tags = oct_tags_carve(w + L.tags_off, out->nodes_capacity);
+  const bool slots = n <= kSlotTagMaxPoints;
   OCT_TRY(launch_prefix_sum_clear_tags(n, m.unique, out->edge_count, out->prefix_sum, m.max_slot,
-                                       w + L.tree_off, m.status, tags, s),
+                                       w + L.tree_off, m.status, tags, slots, s),
           "build: prefix sum");
   mark(rec, s);
   if (out->nodes_capacity > 0) {
@@ -430,7 +431,8 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
     a.n_brt_host = n;
     a.d_unique = m.unique;
     a.d_max_slot = m.max_slot;
-    OCT_TRY(launch_octree(kOctMake | kOctLink | kOctFresh, a, tags, m.status, s, rec, true),
+    OCT_TRY(launch_octree(kOctMake | kOctLink | kOctFresh, a, tags, m.status, s, rec, true,
+                          slots),
             "build: octree");
   } else {
     for (int k = 0; k < 2; ++k) mark(rec, s);

@@ -31,6 +31,7 @@
 // build is a fixed launch sequence that CUDA graphs capture.
 #include <stdio.h>
 
+#include <algorithm>
 #include <new>
 #include <vector>
 
@@ -212,6 +213,26 @@ __device__ __forceinline__ int next_tile(uint32_t* queue, int& round, int* s_til
 }
 
 // ------------------------------------------------------------ prefix sum --
+// The same with slot tags (octree.cuh).
+__global__ void __launch_bounds__(kPfThreads, 5)
+    batch_prefix_slots_kernel(BatchDev B, const int* __restrict__ unique_c,
+                              const int* __restrict__ ec, int* __restrict__ ps_out,
+                              int* __restrict__ max_slot_c,
+                              const uint32_t* __restrict__ tile_prefix, OctTags tags,
+                              uint32_t* __restrict__ queue) {
+  __shared__ __align__(16) PrefixSmem S;
+  __shared__ int s_tile;
+  int round = 0;
+  for (int t = next_tile(queue, round, &s_tile); t < B.T4; t = next_tile(queue, round, &s_tile)) {
+    const int4 d = B.tiles4k[t];
+    const int c = d.z, cs = B.start[c], ns = B.node_start[c];
+    const int n = max(unique_c[c] - 1, 0), lo = d.x - cs;
+    if (lo >= n) continue;
+    prefix_slots_tile(S, ec + cs, ps_out + cs, n, lo, tile_prefix[t] - tile_prefix[d.w],
+                      slot_tags(tags, ns, B.node_start[c + 1] - ns), max_slot_c + c);
+  }
+}
+
 // Inclusive prefix sum of each cloud's edge counts (written by the tree
 // kernels with their per-tile sums, scanned into tile_prefix), and each
 // cloud's largest octree slot.
@@ -428,15 +449,86 @@ __global__ void __launch_bounds__(kFinThreads, 6)
   }
 }
 
-__global__ void batch_publish_kernel(BatchDev B, BatchOctDev O, const uint32_t* status,
-                                     int* __restrict__ counts) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < B.C; c += gridDim.x * blockDim.x) {
+// The same stages with slot tags (octree.cuh).
+__global__ void __launch_bounds__(256, 6)
+    batch_slot_emit_kernel(BatchDev B, BatchOctDev O, uint32_t* __restrict__ status,
+                           uint32_t* __restrict__ queue) {
+  __shared__ int s_tile;
+  int round = 0;
+  for (int k = next_tile(queue, round, &s_tile); k < B.T4; k = next_tile(queue, round, &s_tile)) {
+    const int4 d = B.tiles4k[k];
+    const int c = d.z;
     const CloudSizes z = cloud_sizes(B, O, c);
-    counts[4 * c + 0] = O.unique_c[c];
-    counts[4 * c + 1] = z.n_brt;
-    counts[4 * c + 2] = z.n_oct;
-    counts[4 * c + 3] = (int)((z.fits ? 0u : kStatusCapacity) | (*status & ~kStatusCapacity));
+    if (!z.fits) {
+      if (k == d.w && threadIdx.x == 0) raise_status(status, kStatusCapacity);
+      continue;
+    }
+    const int cs = B.start[c];
+    const int end = min(d.y - cs, z.n_brt);
+    const OctArgs a = cloud_view(B, O, z);
+    const SlotTags t = slot_tags(O.tags, z.ns, z.cap);
+    for (int i = d.x - cs + (int)threadIdx.x; i < end; i += 256)
+      emit_slots(i, a, t, z.n_brt, z.n_oct);
   }
+}
+
+// The clouds' written slots in blocks of 256: block first_block[c] is cloud
+// c's first. Without a queue each CTA of one wave takes a contiguous run of
+// the blocks and finds its first cloud once; with one, blocks come from the
+// queue. A CTA per 256 slots of the capacity (289,490 CTAs on the 512-cloud
+// batch, more than half of them past their cloud's last node) took
+// 0.970 ms there (with node tags), this 0.731 ms.
+__global__ void __launch_bounds__(kFinThreads, 6)
+    batch_slot_finalize_kernel(BatchDev B, BatchOctDev O, const int* __restrict__ first_block,
+                               uint32_t* __restrict__ queue) {
+  __shared__ __align__(16) int s_nodes[kFinThreads * kNodeWords];
+  __shared__ int s_tile;
+  const int blocks = first_block[B.C];
+  int round = 0;
+  int k = (int)((long long)blocks * blockIdx.x / gridDim.x);
+  const int end = (int)((long long)blocks * (blockIdx.x + 1) / gridDim.x);
+  int c = -1;
+  for (;; ++k) {
+    if (queue) k = next_tile(queue, round, &s_tile);
+    if (k >= (queue ? blocks : end)) break;
+    if (c < 0 || queue) c = cloud_of(first_block, B.C, k);
+    while (k >= first_block[c + 1]) ++c;
+    const CloudSizes z = cloud_sizes(B, O, c);
+    const int p0 = (k - first_block[c]) * kFinThreads;
+    const int count = min(kFinThreads, z.n_oct - p0);
+    const OctArgs a = cloud_view(B, O, z);
+    if ((int)threadIdx.x < count)
+      finalize_slots(p0 + (int)threadIdx.x, a, slot_tags(O.tags, z.ns, z.cap), z.n_brt,
+                     a.prefix_n[0] / 3, s_nodes + threadIdx.x * kNodeWords);
+    store_node_block(s_nodes, a.nodes + p0, count);
+  }
+  if (threadIdx.x == 0) bulk_wait_all();
+}
+
+// One CTA: every cloud's counts, and the scan of the clouds' slot blocks.
+__global__ void __launch_bounds__(1024)
+    batch_publish_kernel(BatchDev B, BatchOctDev O, const uint32_t* status,
+                         int* __restrict__ counts, int* __restrict__ first_block) {
+  __shared__ int warp_tot[32];
+  __shared__ int total;
+  int before = 0;
+  for (int c0 = 0; c0 < B.C; c0 += 1024) {
+    const int c = c0 + (int)threadIdx.x;
+    int blocks = 0;
+    if (c < B.C) {
+      const CloudSizes z = cloud_sizes(B, O, c);
+      counts[4 * c + 0] = O.unique_c[c];
+      counts[4 * c + 1] = z.n_brt;
+      counts[4 * c + 2] = z.n_oct;
+      counts[4 * c + 3] = (int)((z.fits ? 0u : kStatusCapacity) | (*status & ~kStatusCapacity));
+      blocks = z.fits ? (z.n_oct + kFinThreads - 1) / kFinThreads : 0;
+    }
+    const int ex = block_exclusive_sum<1024>(blocks, warp_tot, &total);
+    if (c < B.C) first_block[c] = before + ex;
+    before += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) first_block[B.C] = before;
 }
 
 }  // namespace octgb
@@ -446,6 +538,7 @@ struct oct_batch_plan {
   int C = 0;
   int N = 0;
   int total_cap = 0;
+  bool slots = true;  // slot tags: no cloud above kSlotTagMaxPoints
   octgb::SortPlan sp{};
   std::vector<int> start, node_start, cloud_tile0;
   std::vector<int4> sort_tiles, tiles4k, slot_tiles;
@@ -454,7 +547,7 @@ struct oct_batch_plan {
          tables_bytes = 0;
   // workspace offsets
   size_t w_status = 0, w_queue = 0, w_unique = 0, w_maxslot = 0, w_hist = 0,
-         zero_bytes = 0, w_tree = 0, w_base = 0, w_th = 0, w_keys_a = 0, w_keys_b = 0,
+         zero_bytes = 0, w_tree = 0, w_base = 0, w_th = 0, w_blocks = 0, w_keys_a = 0, w_keys_b = 0,
          w_tags = 0, ws_bytes = 0;
 };
 
@@ -528,6 +621,7 @@ OCT_API oct_batch_plan* oct_batch_plan_create(int n_clouds, const int32_t* h_siz
     }
     P->start[c] = (int)N;
     P->node_start[c] = (int)cap;
+    P->slots = P->slots && h_sizes[c] <= kSlotTagMaxPoints;
     N += h_sizes[c];
     cap += h_node_caps ? h_node_caps[c] : h_sizes[c];
     if (N > OCT_MAX_N || cap > OCT_MAX_N) {
@@ -578,6 +672,7 @@ OCT_API oct_batch_plan* oct_batch_plan_create(int n_clouds, const int32_t* h_siz
   P->zero_bytes = o;
   P->w_tree = take(tree_scratch_bytes_tiles((int)P->tiles4k.size()));
   P->w_base = take(4 * (size_t)n_clouds * passes * bins);
+  P->w_blocks = take(4 * (size_t)(n_clouds + 1));
   P->w_th = take(4 * (P->sort_tiles.size() + 1) * bins);
   P->w_keys_a = take(4 * (size_t)std::max(P->N, 1));
   P->w_keys_b = take(4 * (size_t)std::max(P->N, 1));
@@ -740,8 +835,14 @@ int batch_build(const oct_batch_plan* P, const void* d_tables, const oct_vec4* p
     if (e != cudaSuccess) return batch_fail(e, "batch: tree");
     const OctTags tags = oct_tags_carve(w + P->w_tags, std::max(P->total_cap, 1));
     uint32_t* queue = g_batch_queue ? reinterpret_cast<uint32_t*>(w + P->w_queue) : nullptr;
-    batch_prefix_sum_kernel<<<queue_grid(batch_prefix_sum_kernel, 256, B.T4, queue), 256, 0, s>>>(
-        B, unique_c, out->edge_count, out->prefix_sum, max_slot_c, TS.tile_prefix, tags, queue);
+    if (P->slots)
+      batch_prefix_slots_kernel<<<queue_grid(batch_prefix_slots_kernel, kPfThreads, B.T4, queue),
+                                  kPfThreads, 0, s>>>(B, unique_c, out->edge_count,
+                                                      out->prefix_sum, max_slot_c, TS.tile_prefix,
+                                                      tags, queue);
+    else
+      batch_prefix_sum_kernel<<<queue_grid(batch_prefix_sum_kernel, 256, B.T4, queue), 256, 0, s>>>(
+          B, unique_c, out->edge_count, out->prefix_sum, max_slot_c, TS.tile_prefix, tags, queue);
     BatchOctDev O;
     O.nodes = out->nodes;
     O.offsets = out->prefix_sum;
@@ -755,12 +856,23 @@ int batch_build(const oct_batch_plan* P, const void* d_tables, const oct_vec4* p
     O.unique_c = unique_c;
     O.max_slot_c = max_slot_c;
     O.tags = tags;
-    batch_oct_emit_kernel<<<queue_grid(batch_oct_emit_kernel, 256, B.T4, queue), 256, 0, s>>>(
-        B, O, status, queue ? queue + 4 : nullptr);
-    if (B.Tn > 0)
+    uint32_t* emit_queue = queue ? queue + 4 : nullptr;
+    uint32_t* fin_queue = queue ? queue + 8 : nullptr;
+    int* first_block = reinterpret_cast<int*>(w + P->w_blocks);
+    if (P->slots)
+      batch_slot_emit_kernel<<<queue_grid(batch_slot_emit_kernel, 256, B.T4, queue), 256, 0, s>>>(
+          B, O, status, emit_queue);
+    else
+      batch_oct_emit_kernel<<<queue_grid(batch_oct_emit_kernel, 256, B.T4, queue), 256, 0, s>>>(
+          B, O, status, emit_queue);
+    batch_publish_kernel<<<1, 1024, 0, s>>>(B, O, status, d_cloud_counts, first_block);
+    if (P->slots) {
+      const int grid = std::max(1, std::min(B.Tn, sms * 6));
+      batch_slot_finalize_kernel<<<grid, kFinThreads, 0, s>>>(B, O, first_block, fin_queue);
+    } else if (B.Tn > 0) {
       batch_oct_finalize_kernel<<<queue_grid(batch_oct_finalize_kernel, kFinThreads, B.Tn, queue),
-                                  kFinThreads, 0, s>>>(B, O, queue ? queue + 8 : nullptr);
-    batch_publish_kernel<<<(P->C + 255) / 256, 256, 0, s>>>(B, O, status, d_cloud_counts);
+                                  kFinThreads, 0, s>>>(B, O, fin_queue);
+    }
   } else {
     e = cudaMemsetAsync(d_cloud_counts, 0, 16 * (size_t)P->C, s);
   }

@@ -280,6 +280,14 @@ struct OctTags {
 size_t oct_tags_bytes(int cap);
 OctTags oct_tags_carve(void* base, int cap);
 
+// Whole and batched builds up to this many points (per cloud) use slot tags
+// (octree.cuh), whose slot numbers have 27 bits. A cell of level l needs two
+// codes sharing 3 l - 1 bits, so a cloud of U codes has at most
+// sum over l of min(2^(3 l - 1), U / 2) octree nodes: for U = 120M that is
+// 2 * 60M + 2^23 + 2^20 + ... < 2^27, however the codes lie. Larger clouds
+// take the node tags of the stage entries.
+constexpr int kSlotTagMaxPoints = 120000000;
+
 // Zeroes the tags of slots [lo, hi] (inclusive) with `nthreads` threads of
 // index `tid`: consecutive threads take consecutive 16-byte child words, so
 // every warp store fills whole sectors.
@@ -292,6 +300,41 @@ __device__ __forceinline__ void clear_tag_range(const OctTags& t, size_t lo, siz
   for (size_t p = lo + (size_t)tid; p <= hi; p += (size_t)nthreads) {
     t.owner[p] = 0;
     t.mask[p] = 0;
+  }
+}
+
+// The slot tags' view of the same arrays: child tags as above, in place of
+// the owners the radix node whose prefix is the slot (0: none), one mask byte
+// per slot. `at` is the cloud's first slot (0 for a single cloud); slots are
+// cloud-local.
+struct SlotTags {
+  uint32_t* child;  // [cap * 8]
+  uint32_t* node;   // [cap] (radix node << 4) | step, kNoNode, or 0: open
+  uint8_t* mask;    // [cap]
+  int at, cap;
+  __device__ __forceinline__ uint32_t* mask_word(int slot, int& shift) const {
+    const uint32_t g = (uint32_t)at + (uint32_t)slot;
+    shift = (int)(g & 3u) * 8;
+    return reinterpret_cast<uint32_t*>(mask) + (g >> 2);
+  }
+};
+__host__ __device__ static inline SlotTags slot_tags(const OctTags& t, int at, int cap) {
+  return SlotTags{t.child + (size_t)at * 8, t.owner + at, reinterpret_cast<uint8_t*>(t.mask), at,
+                  cap};
+}
+
+// Zeroes the mask bytes of the cloud's slots [lo, hi] (inclusive); bytes
+// outside the range may be another tile's.
+__device__ __forceinline__ void clear_mask_range(const SlotTags& t, int lo, int hi, int tid,
+                                                 int nthreads) {
+  const uint32_t b0 = (uint32_t)t.at + (uint32_t)lo, b1 = (uint32_t)t.at + (uint32_t)hi + 1u;
+  const uint32_t w0 = (b0 + 3u) >> 2, w1 = b1 >> 2;  // whole words inside the range
+  for (uint32_t w = w0 + (uint32_t)tid; w < w1; w += (uint32_t)nthreads)
+    reinterpret_cast<uint32_t*>(t.mask)[w] = 0u;
+  const uint32_t head = w0 <= w1 ? 4u * w0 : b1, tail = w0 <= w1 ? 4u * w1 : b1;
+  if (tid < 4) {  // the bytes before and after them
+    if (b0 + (uint32_t)tid < head) t.mask[b0 + tid] = 0;
+    if (tail + (uint32_t)tid < b1) t.mask[tail + tid] = 0;
   }
 }
 
@@ -314,22 +357,26 @@ struct OctArgs {
   int n_oct_host;          // used when d_max_slot == nullptr
   const int* d_max_slot;   // largest slot on the device (n_oct = max_slot + 1)
 };
-// tags_clear: the tags of [0, M) are already zero (launch_prefix_sum_clear_tags).
+// tags_clear: the tags of [0, M) are already zero and, with slot tags, the
+// slots' nodes written (launch_prefix_sum_clear_tags); slots: slot tags (mode
+// kOctMake | kOctLink | kOctFresh only).
 cudaError_t launch_octree(int mode, const OctArgs& a, const OctTags& t, uint32_t* status,
-                          cudaStream_t s, Recorder* rec = nullptr, bool tags_clear = false);
+                          cudaStream_t s, Recorder* rec = nullptr, bool tags_clear = false,
+                          bool slots = false);
 
 // Inclusive prefix sum of the edge counts written by launch_radix_tree_sorted
 // (which also summed them per 4,096-node tile into the scratch) that also
 // clears the octree tags of every slot stages 7-8 can touch, up to the tags'
-// capacity: one small kernel scans the tile sums, then every tile scans its
-// own nodes from its prefix (no inter-tile waits).
+// capacity (slots: also writes each slot's radix node): one small kernel scans
+// the tile sums, then every tile scans its own nodes from its prefix (no
+// inter-tile waits).
 // Exclusive scan of tiles per-tile sums (one CTA).
 cudaError_t launch_tile_sums_scan(int tiles, const int* tile_sum, uint32_t* tile_prefix,
                                   cudaStream_t s);
 
 cudaError_t launch_prefix_sum_clear_tags(int n_host, const int* d_unique, int* ec, int* ps,
                                          int* d_max_slot, void* tree_scratch, uint32_t* status,
-                                         const OctTags& tags, cudaStream_t s);
+                                         const OctTags& tags, bool slots, cudaStream_t s);
 
 // Copies U, B, M, status into out[4] (device).
 cudaError_t launch_publish_counts(const int* d_unique, const int* d_max_slot,

@@ -1169,9 +1169,10 @@ OCT_API int oct_build_octree_learned(const oct_vec4* points, int n, float min_co
                                  out->tree.left_child, out->tree.parent, out->edge_count,
                                  w + L.tree_off, s);
   const OctTags tags = oct_tags_carve(w + L.tags_off, out->nodes_capacity);
+  const bool slots = n <= kSlotTagMaxPoints;
   if (e == cudaSuccess)
     e = launch_prefix_sum_clear_tags(n, d_unique, out->edge_count, out->prefix_sum, d_max_slot,
-                                     w + L.tree_off, status, tags, s);
+                                     w + L.tree_off, status, tags, slots, s);
   if (e == cudaSuccess && out->nodes_capacity > 0) {
     OctArgs a{};
     a.nodes = out->nodes;
@@ -1189,7 +1190,8 @@ OCT_API int oct_build_octree_learned(const oct_vec4* points, int n, float min_co
     a.n_brt_host = n;
     a.d_unique = d_unique;
     a.d_max_slot = d_max_slot;
-    e = launch_octree(kOctMake | kOctLink | kOctFresh, a, tags, status, s, nullptr, true);
+    e = launch_octree(kOctMake | kOctLink | kOctFresh, a, tags, status, s, nullptr, true,
+                      slots);
   }
   if (e == cudaSuccess) e = launch_publish_counts(d_unique, d_max_slot, status, out->d_counts, s);
   if (e == cudaSuccess && d_stats)

@@ -81,41 +81,43 @@ __global__ void __launch_bounds__(kFinThreads, 8) oct_finalize_kernel(int mode, 
   if (!z.fits || z.n_brt < 1) return;
   const int root_level = a.prefix_n[0] / 3;
   const bool fresh = mode & kOctFresh;
-  int* out_words = reinterpret_cast<int*>(a.nodes);
   for (int blk = blockIdx.x * kFinThreads; blk < z.n_oct; blk += gridDim.x * kFinThreads) {
     const int p = blk + threadIdx.x;
-    const int count = min(kFinThreads, z.n_oct - blk);
     if (p < z.n_oct) finalize_slot(fresh, p, a, t, root_level, s_nodes + threadIdx.x * kNodeWords);
-    bulk_fence_writes();
-    __syncthreads();
-    int* dst = out_words + (size_t)blk * kNodeWords;
-    // 256 nodes are 960 16-byte words; blk is a multiple of 256, so dst is
-    // 16-byte aligned whenever the node array is.
-    const int words = count * kNodeWords;
-    if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (words & 3) == 0) {
-      // one bulk copy of the staged block (the TMA engine writes it)
-      if (threadIdx.x == 0) {
-        bulk_store_s2g(dst, s_nodes, (uint32_t)words * 4u);
-        bulk_wait_read();  // the stage is free for the next block
-      }
-    } else {
-      int k0 = 0;
-      if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        const int quads = words >> 2;
-        const uint4* src4 = reinterpret_cast<const uint4*>(s_nodes);
-        uint4* dst4 = reinterpret_cast<uint4*>(dst);
-        for (int k = threadIdx.x; k < quads; k += kFinThreads) dst4[k] = src4[k];
-        k0 = quads << 2;
-      }
-      for (int k = k0 + threadIdx.x; k < words; k += kFinThreads) dst[k] = s_nodes[k];
-    }
-    __syncthreads();
+    store_node_block(s_nodes, a.nodes + blk, min(kFinThreads, z.n_oct - blk));
+  }
+  if (threadIdx.x == 0) bulk_wait_all();
+}
+
+// The same stages with slot tags (whole builds): launch bounds and grids as above.
+__global__ void __launch_bounds__(256, 8)
+    slot_emit_kernel(OctArgs a, SlotTags t, uint32_t* __restrict__ status) {
+  chain_enter();
+  const Sizes z = read_sizes(a);
+  if (!z.fits) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) raise_status(status, kStatusCapacity);
+    return;
+  }
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < z.n_brt) emit_slots(i, a, t, z.n_brt, z.n_oct);
+}
+
+__global__ void __launch_bounds__(kFinThreads, 8) slot_finalize_kernel(OctArgs a, SlotTags t) {
+  chain_enter();
+  __shared__ __align__(16) int s_nodes[kFinThreads * kNodeWords];
+  const Sizes z = read_sizes(a);
+  if (!z.fits || z.n_brt < 1) return;
+  const int root_level = a.prefix_n[0] / 3;
+  for (int blk = blockIdx.x * kFinThreads; blk < z.n_oct; blk += gridDim.x * kFinThreads) {
+    const int p = blk + threadIdx.x;
+    if (p < z.n_oct) finalize_slots(p, a, t, z.n_brt, root_level, s_nodes + threadIdx.x * kNodeWords);
+    store_node_block(s_nodes, a.nodes + blk, min(kFinThreads, z.n_oct - blk));
   }
   if (threadIdx.x == 0) bulk_wait_all();
 }
 
 cudaError_t launch_octree(int mode, const OctArgs& a, const OctTags& t, uint32_t* status,
-                          cudaStream_t s, Recorder* rec, bool tags_clear) {
+                          cudaStream_t s, Recorder* rec, bool tags_clear, bool slots) {
   cudaError_t e;
   if (!tags_clear) {
     const int zgrid = device_sm_count() * 8;
@@ -126,7 +128,12 @@ cudaError_t launch_octree(int mode, const OctArgs& a, const OctTags& t, uint32_t
   int nb = a.d_unique ? a.n_brt_host : a.n_brt_host;
   int egrid = (nb + 255) / 256;
   if (egrid < 1) egrid = 1;
-  e = launch_chained(oct_emit_kernel, dim3(egrid), dim3(256), 0, s, mode, a, t, status, tags_clear);
+  if (slots)
+    e = launch_chained(slot_emit_kernel, dim3(egrid), dim3(256), 0, s, a, slot_tags(t, 0, a.cap),
+                       status);
+  else
+    e = launch_chained(oct_emit_kernel, dim3(egrid), dim3(256), 0, s, mode, a, t, status,
+                       tags_clear);
   if (e != cudaSuccess) return e;
   mark(rec, s);
   // One wave at 8 CTAs per SM, each walking the 256-slot blocks: the node
@@ -135,7 +142,11 @@ cudaError_t launch_octree(int mode, const OctArgs& a, const OctTags& t, uint32_t
   int fgrid = (a.cap + kFinThreads - 1) / kFinThreads;
   fgrid = std::min(fgrid, device_sm_count() * 8);
   if (fgrid < 1) fgrid = 1;
-  e = launch_chained(oct_finalize_kernel, dim3(fgrid), dim3(kFinThreads), 0, s, mode, a, t);
+  if (slots)
+    e = launch_chained(slot_finalize_kernel, dim3(fgrid), dim3(kFinThreads), 0, s, a,
+                       slot_tags(t, 0, a.cap));
+  else
+    e = launch_chained(oct_finalize_kernel, dim3(fgrid), dim3(kFinThreads), 0, s, mode, a, t);
   if (e == cudaSuccess) mark(rec, s);
   return e;
 }

@@ -160,6 +160,316 @@ __device__ __forceinline__ float cell_size(float range, int k) {
   return __fdiv_rn(range, (float)(1 << k));
 }
 
+// ------------------------------------------------------------- slot tags --
+// The whole and batched builds' form of the same tags (trees built by this
+// library, stages 7 and 8 together, up to kSlotTagMaxPoints points). Two facts
+// let finalize turn a tag into its value without looking anything up:
+//   - among radix nodes with octree nodes (k >= 1) the inclusive prefix grows
+//     by at least one from each to the next, so (prefix, step) orders their
+//     writes as (node, step) does, and names the value: prefix + step;
+//   - a leaf lies at its parent's own index or at the far end of the parent's
+//     range, usually a few codes away, so a link tag carries that distance
+//     behind its order key.
+//   MakeOctNodes  step j of the node with prefix s : (s << 4) | j     (s < 2^27, s >= 1)
+//   LinkLeafNodes of node i : 0x80000000 | (i << (b + 1)) | (2^b + off), the
+//     leaf being i + off, off <= 0 for the left leaf and >= 0 for the right
+//     one (never 0 for both: i is one end of the node's range). The field's
+//     ends, 0 and all ones, stand for a leaf too far off: read left_child[i].
+//     b is what the cloud's node numbers leave (6 bits at 16.7M points, where
+//     about one slot in a hundred looks up)
+// The corner's writer needs no tag either: slots [s, s + k) belong to the node
+// with prefix s, later nodes overwrite, and the prefix sum's tiles note each
+// slot's node and step (SlotTags::node). The masks take one byte per slot.
+// Against node tags (owner tag, 4-byte mask, two table reads per child):
+// emit 0.202 -> 0.186 ms (285 -> 236 warp instructions per 32 nodes; bound by its
+// dependent loads), finalize 0.152 -> 0.132 ms (416 -> 288 per 32 slots; bound by
+// DRAM, 5.8 TB/s) at 16.7M uniform points.
+constexpr uint32_t kNoNode = 15u;  // SlotTags::node: no node's slots reach this one (0: open)
+
+__device__ __forceinline__ int link_off_bits(int n_brt) {
+  return min(__clz(n_brt) - 2, 16);  // 31 tag bits, one of them the side
+}
+
+__device__ __forceinline__ void slot_put(const SlotTags& t, int slot, uint32_t which,
+                                         uint32_t tag) {
+  atomicMax(t.child + ((uint32_t)slot * 8u + which), tag);
+}
+__device__ __forceinline__ void slot_mark(const SlotTags& t, int slot, uint32_t which) {
+  int sh;
+  uint32_t* w = t.mask_word(slot, sh);
+  atomicOr(w, 1u << (sh + (int)which));
+}
+
+// Inclusive prefix sum of one tile of 4,096 edge counts of a cloud, with the
+// slot tags' preparation of the slots it covers: child tags and masks zeroed,
+// each slot's radix node written. The tile's own slots are (ex, ex + total];
+// the next nine may hold the last node's further steps and are cleared as
+// well (the next tile clears them again: zeros either way, and nothing else
+// writes tags in this kernel).
+//
+// Bound: DRAM writes (the tags take 33 B per slot beside 8 B per node). The
+// child tags are zeroed by bulk copies of a zeroed 4 KB block (the TMA engine
+// writes them), which leaves the load/store units to the counts: 0.084 -> 0.067 ms
+// at 16.7M uniform points against the node tags and 16-byte stores.
+constexpr int kPfThreads = 256;
+constexpr int kPfItems = 16;
+constexpr int kPfTile = kPfThreads * kPfItems;  // the radix-tree tiles
+constexpr int kPfZero = 4096;                   // bytes of the zero block
+constexpr int kMaxSteps = 10;                   // octree levels one radix node can span
+
+struct PrefixSmem {
+  uint4 zero[kPfZero / 16];
+  uint32_t node[kPfTile];  // by slot after the tile's prefix: (tile's node + 1) << 4 | step
+  int v[kPfTile + kPfTile / 32];  // padded: entry j at j + j / 32
+  uint32_t warp[32];
+  uint32_t total;
+  int max_slot;
+};
+
+__device__ __forceinline__ int pf_pad(int j) { return j + (j >> 5); }
+
+// ec, ps: the cloud's arrays; the tile's nodes are [lo, min(lo + 4096, n)), its
+// exclusive prefix ex. max_slot: raised to the largest slot stages 7-8 write.
+// All threads call it; ends with a barrier.
+__device__ __forceinline__ void prefix_slots_tile(PrefixSmem& S, const int* __restrict__ ec,
+                                                  int* __restrict__ ps, int n, int lo, uint32_t ex,
+                                                  const SlotTags& t, int* max_slot) {
+  const int tid = threadIdx.x;
+  const int valid = min(kPfTile, n - lo);
+#pragma unroll
+  for (int k = 0; k < kPfItems; ++k) {
+    const int j = k * kPfThreads + tid;
+    S.v[pf_pad(j)] = j < valid ? ec[lo + j] : 0;
+  }
+  S.zero[tid] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int q = 0; q < kPfTile / 4 / kPfThreads; ++q)
+    reinterpret_cast<uint4*>(S.node)[tid + q * kPfThreads] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid == 0) S.max_slot = 0;
+  bulk_fence_writes();
+  __syncthreads();
+  int v[kPfItems];
+  uint32_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < kPfItems; ++k) {
+    v[k] = S.v[pf_pad(tid * kPfItems + k)];
+    sum += (uint32_t)v[k];
+  }
+  const uint32_t off = block_exclusive_sum<kPfThreads>(sum, S.warp, &S.total);
+  const uint32_t total = S.total;
+  const uint32_t cap = (uint32_t)t.cap;
+  if (ex < cap) {
+    const uint32_t hi = min(ex + min(total, cap) + (uint32_t)(kMaxSteps - 1), cap - 1u);
+    if (tid == 0) {
+      char* dst = reinterpret_cast<char*>(t.child + (size_t)ex * 8);
+      const size_t bytes = ((size_t)hi - ex + 1) * 32;
+      for (size_t b = 0; b < bytes; b += kPfZero)
+        bulk_store_s2g(dst + b, S.zero, (uint32_t)min((size_t)kPfZero, bytes - b));
+    }
+    clear_mask_range(t, (int)ex, (int)hi, tid, kPfThreads);
+  }
+  // (Bounds on run and v: counts of a malformed tree, see emit_slots.)
+  // a tile covers at most its nodes' slots; more than the stage holds only
+  // when many nodes span several levels
+  const bool staged = total <= (uint32_t)kPfTile;
+  uint32_t run = ex + off;
+  int mx = 0;
+  uint32_t multi = 0;  // items that span several levels
+#pragma unroll
+  for (int k = 0; k < kPfItems; ++k) {
+    const int j = tid * kPfItems + k;
+    run += (uint32_t)v[k];
+    S.v[pf_pad(j)] = (int)run;  // each thread rewrites only its own entries
+    const int i = lo + j;
+    const uint32_t q = run - ex - 1u;
+    const bool makes = i > 0 && v[k] > 0;  // entries past the last node are 0
+    if (makes) mx = max(mx, (int)run + v[k] - 1);
+    if (makes && v[k] > 1) multi |= 1u << k;
+    // the node's own slot: later nodes win over earlier nodes' further steps
+    if (makes && q < (uint32_t)kPfTile) atomicMax(&S.node[q], (uint32_t)(j + 1) << 4);
+    if (i == n - 1) mx = max(mx, (int)run);
+  }
+  // further steps, one such node of each lane at a time
+  while (staged && multi) {
+    const int j = tid * kPfItems + __ffs(multi) - 1;
+    multi &= multi - 1u;
+    const uint32_t q = (uint32_t)S.v[pf_pad(j)] - ex - 1u;
+    const uint32_t k = (uint32_t)min(ec[lo + j], kMaxSteps);
+    for (uint32_t h = 1; h < k && q + h < total; ++h)
+      atomicMax(&S.node[q + h], ((uint32_t)(j + 1) << 4) | h);
+  }
+  if (!staged) {
+    // the node's own slot only, none for those up to the one before it
+#pragma unroll 1
+    for (int k = 0; k < kPfItems; ++k) {
+      const int j = tid * kPfItems + k;
+      const uint32_t r = (uint32_t)S.v[pf_pad(j)];
+      const int kk = j < valid && lo + j > 0 ? min(ec[lo + j], kMaxSteps) : 0;
+      for (int h = 1; h < kk; ++h)
+        if (r - (uint32_t)h < cap) t.node[r - (uint32_t)h] = 0u;
+      if (kk > 0 && r < cap) t.node[r] = (uint32_t)(lo + j) << 4;
+    }
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((tid & 31) == 0 && mx > 0) atomicMax(&S.max_slot, mx);
+  __syncthreads();
+  if (tid == 0) atomicMax(max_slot, S.max_slot);
+#pragma unroll
+  for (int k = 0; k < kPfItems; ++k) {
+    const int j = k * kPfThreads + tid;
+    if (j < valid) ps[lo + j] = S.v[pf_pad(j)];
+  }
+  if (staged) {
+    for (uint32_t q = tid; q < total; q += kPfThreads) {
+      const uint32_t slot = ex + 1u + q;
+      const uint32_t e = S.node[q];
+      // the tile before may reach its first few slots: left open
+      const uint32_t none = q < (uint32_t)kMaxSteps && lo > 0 ? 0u : kNoNode;
+      if (slot < cap) t.node[slot] = e ? e + ((uint32_t)(lo - 1) << 4) : none;
+    }
+  }
+  // slot 0 (the root's) and the slots after the last node's prefix have none
+  if (lo == 0 && tid == 0 && cap > 0) t.node[0] = 0u;
+  if (lo + kPfTile >= n && tid < kMaxSteps) {
+    const uint32_t slot = ex + total + 1u + (uint32_t)tid;
+    if (slot < cap) t.node[slot] = 0u;
+  }
+  if (tid == 0) bulk_wait_read();  // the zero block may go
+  __syncthreads();
+}
+
+// Every write radix node i makes. The tree is this library's own, so a walk
+// ends at a node with octree nodes or at node 0 after at most 30 steps, every
+// index is below n_brt and every slot below n_oct (n_oct - 1 is the largest
+// slot written). The clamps only matter after a status bit was raised (a
+// sort whose look-back timed out leaves no tree): nothing goes out of bounds.
+__device__ __forceinline__ void emit_slots(int i, const OctArgs& a, const SlotTags& t, int n_brt,
+                                           int n_oct) {
+  const uint32_t last = (uint32_t)n_brt - 1u, top_slot = (uint32_t)n_oct - 1u;
+  const uint32_t pn = a.prefix_n[i];
+  const int k = min(a.counts[i], kMaxSteps);
+  const uint32_t par = min((uint32_t)a.parent[i], last);
+  const bool ll = a.hll[i] != 0, lr = a.hlr[i] != 0;
+  const bool make = k > 0 && i >= 1, link = ll || lr;
+  int base = 0;
+  uint32_t lc = 0, code = 0;
+  if (make) {
+    base = a.offsets[i];
+    code = a.codes[i];
+  }
+  if (link) lc = min((uint32_t)a.left_child[i], last);
+  const int L = (int)(pn / 3u);
+  // The first radix node with octree nodes, from the parent (MakeOctNodes, or
+  // the links of a node without any) or the node itself.
+  uint32_t rn = (uint32_t)i;
+  if (make || (link && k == 0 && i != 0)) {
+    rn = par;
+    int c = a.counts[rn];
+    uint32_t next = (uint32_t)a.parent[rn];
+    for (int step = 0; c == 0 && rn != 0u && step < 32; ++step) {
+      rn = min(next, last);
+      c = a.counts[rn];
+      next = (uint32_t)a.parent[rn];
+    }
+  }
+  uint32_t cl = 0, cr = 0;
+  if (ll) cl = a.codes[lc];
+  if (lr) cr = a.codes[lc + 1u];
+  const int up = (int)min((uint32_t)a.offsets[rn], top_slot);
+  if (make) {
+    // include/shared/oct.h:24-90
+    const uint32_t s16 = (uint32_t)base << 4;
+    for (int j = 0; j < k - 1; ++j) {
+      const uint32_t which = (code >> (30 - 3 * (L - j))) & 7u;
+      const int slot = (int)min((uint32_t)(base + j + 1), top_slot);
+      slot_put(t, slot, which, s16 | (uint32_t)j);
+      slot_mark(t, slot, which);
+    }
+    const uint32_t which = (code >> (30 - 3 * (L - k + 1))) & 7u;
+    slot_put(t, up, which, s16 | (uint32_t)(k - 1));
+    slot_mark(t, up, which);
+  }
+  if (link) {
+    // include/shared/oct.h:92-134, walk ended at radix node 0
+    const int dst = make ? (int)min((uint32_t)base, top_slot) : up;
+    const uint32_t sh = (uint32_t)(27 - 3 * L) & 31u;
+    const int b = link_off_bits(n_brt);
+    const uint32_t mid = 1u << b;
+    const uint32_t key = kLinkTag | ((uint32_t)i << (b + 1));
+    if (ll) slot_put(t, dst, (cl >> sh) & 7u, key | (mid - min((uint32_t)i - lc, mid)));
+    if (lr)
+      slot_put(t, dst, (cr >> sh) & 7u, key | (mid + min(lc + 1u - (uint32_t)i, mid - 1u)));
+  }
+}
+
+// The 15 words of slot p, from the slot tags.
+__device__ __forceinline__ void finalize_slots(int p, const OctArgs& a, const SlotTags& t,
+                                               int n_brt, int root_level, int* w) {
+  const uint32_t last = (uint32_t)n_brt - 1u;
+  const uint4* c4 = reinterpret_cast<const uint4*>(t.child);
+  const uint4 ta = c4[2 * (uint32_t)p], tb = c4[2 * (uint32_t)p + 1u];
+  const uint32_t m = t.mask[(uint32_t)t.at + (uint32_t)p];
+  uint32_t own = p > 0 ? t.node[p] : 0u;
+  if (own == 0u && p > 0) {
+    // not in a tile's own slots (a tile's first few, or one with more slots
+    // than it stages): the nearest node before it whose slots reach p
+    for (int d = 1; d < kMaxSteps && d < p; ++d) {
+      const uint32_t e = t.node[p - d];
+      if ((e & 15u) == 0u && e != 0u && a.counts[min(e >> 4, last)] > d) {
+        own = e + (uint32_t)d;
+        break;
+      }
+    }
+  }
+  const int j = (int)(own & 15u);
+  own = min(own >> 4, last);  // 0: none
+  // slot 0 is the root's: the corner of node 0's cell, the whole range
+  const bool owned = own != 0u || p == 0;
+  int pn = 0;
+  uint32_t code = 0;
+  if (owned) {
+    pn = a.prefix_n[own];
+    code = a.codes[own];
+  }
+  const uint32_t tags[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
+  const int b = link_off_bits(n_brt);
+  const uint32_t field = (2u << b) - 1u;
+  uint32_t far = 0;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    // both kinds by selects (a warp holds both): 0 for no tag
+    const uint32_t g = tags[c];
+    const bool link = (int)g < 0;
+    const uint32_t x = g & ~kLinkTag;
+    const uint32_t m = link ? field : 15u;
+    const uint32_t low = x & m;
+    const uint32_t high = x >> (link ? b + 1 : 4);
+    w[c] = (int)(high + low - (link ? 1u << b : 0u));
+    far |= link && ((low + 1u) & m) < 2u ? 1u << c : 0u;
+  }
+  while (far) {
+    const int c = __ffs(far) - 1;
+    far &= far - 1u;
+    const uint32_t g = t.child[(uint32_t)p * 8u + (uint32_t)c];
+    w[c] = a.left_child[min((g & ~kLinkTag) >> (b + 1), last)] + (int)(g & 1u);
+  }
+  float4 corner = make_float4(0.f, 0.f, 0.f, 0.f);
+  float cell = 0.f;
+  if (owned) {
+    const int level = p == 0 ? root_level : pn / 3 - j;
+    const int sh = 30 - 3 * level;
+    corner = decode_corner((code >> sh) << sh, a.min_coord, a.range);
+    cell = p == 0 ? a.range : cell_size(a.range, level - root_level);
+  }
+  w[8] = __float_as_int(corner.x);
+  w[9] = __float_as_int(corner.y);
+  w[10] = __float_as_int(corner.z);
+  w[11] = __float_as_int(corner.w);
+  w[12] = __float_as_int(cell);
+  w[13] = (int)m;
+  w[14] = 0;
+}
+
 // One thread per slot computes the node; the block stages its 256 nodes
 // (15 KB) in shared memory and writes them as consecutive 32-bit words, so
 // every warp store is one contiguous 128-byte line.
@@ -238,6 +548,31 @@ __device__ __forceinline__ void finalize_slot(bool fresh, int p, const OctArgs& 
     w[13] = nd->child_node_mask | (int)m;
     w[14] = nd->child_leaf_mask & ~(int)link_bits;
   }
+}
+
+// The block's staged nodes to dst[0, count): one bulk copy (the TMA engine
+// writes it) when dst is 16-byte aligned and the block a whole number of
+// 16-byte words, else vector and word stores. The block's threads call it
+// after staging; the stage is free again when it returns.
+__device__ __forceinline__ void store_node_block(const int* s_nodes, oct_node* nodes, int count) {
+  bulk_fence_writes();
+  __syncthreads();
+  int* dst = reinterpret_cast<int*>(nodes);
+  const int words = count * kNodeWords;
+  const bool aligned = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+  if (aligned && (words & 3) == 0) {
+    if (threadIdx.x == 0) {
+      bulk_store_s2g(dst, s_nodes, (uint32_t)words * 4u);
+      bulk_wait_read();
+    }
+  } else {
+    const int quads = aligned ? words >> 2 : 0;
+    const uint4* src4 = reinterpret_cast<const uint4*>(s_nodes);
+    uint4* dst4 = reinterpret_cast<uint4*>(dst);
+    for (int k = threadIdx.x; k < quads; k += blockDim.x) dst4[k] = src4[k];
+    for (int k = 4 * quads + threadIdx.x; k < words; k += blockDim.x) dst[k] = s_nodes[k];
+  }
+  __syncthreads();
 }
 
 }  // namespace octgb

@@ -18,6 +18,7 @@
 // (include/kernels/06_partial_sum.hpp:6-9; the reference GPU driver does this
 // scan on the host, apps/gpu_demo/main.cu:308-310). Fused, one read of
 // prefix_n/parent produces both arrays and the octree node count.
+#include "octree.cuh"
 #include "tree.cuh"
 
 namespace octgb {
@@ -393,16 +394,32 @@ __global__ void __launch_bounds__(kTsThreads)
   if (total_out && threadIdx.x == 0) *total_out = (int)s_total;
 }
 
+// Prefix sum of the whole build with slot tags (octree.cuh).
+__global__ void __launch_bounds__(kPfThreads, 5)
+    prefix_slots_kernel(int n_host, const int* __restrict__ d_unique, const int* __restrict__ ec,
+                        int* __restrict__ ps, int* __restrict__ d_max_slot,
+                        const uint32_t* __restrict__ tile_prefix, SlotTags t) {
+  chain_enter();
+  __shared__ __align__(16) PrefixSmem S;
+  const int n = d_unique ? max(*d_unique - 1, 0) : n_host;
+  const int lo = blockIdx.x * kPfTile;
+  if (lo >= n) return;
+  prefix_slots_tile(S, ec, ps, n, lo, tile_prefix[blockIdx.x], t, d_max_slot);
+}
+
 cudaError_t launch_prefix_sum_clear_tags(int n_host, const int* d_unique, int* ec, int* ps,
                                          int* d_max_slot, void* tree_scratch, uint32_t* status,
-                                         const OctTags& tags, cudaStream_t s) {
-  static_assert(kEsTile == 4096, "scan tiles are the radix-tree tiles");
+                                         const OctTags& tags, bool slots, cudaStream_t s) {
+  static_assert(kEsTile == 4096 && kPfTile == 4096, "scan tiles are the radix-tree tiles");
   if (n_host <= 0) return cudaSuccess;
   const TreeScratch S = tree_scratch_carve(tree_scratch, n_host);
   cudaError_t e = launch_chained(tile_sums_scan_kernel, dim3(1), dim3(kTsThreads), 0, s, 0, n_host,
                                  d_unique, S.tile_sum, S.tile_prefix, nullptr, nullptr);
   if (e != cudaSuccess) return e;
   const int tiles = (n_host + kEsTile - 1) / kEsTile;
+  if (slots)
+    return launch_chained(prefix_slots_kernel, dim3(tiles), dim3(kPfThreads), 0, s, n_host,
+                          d_unique, ec, ps, d_max_slot, S.tile_prefix, slot_tags(tags, 0, tags.cap));
   return launch_chained(edge_scan_kernel, dim3(tiles), dim3(kEsThreads), 0, s, kScanOnly, n_host,
                         d_unique, nullptr, nullptr, ec, ps, d_max_slot, nullptr, nullptr, status,
                         tags.cap > 0 ? tags : OctTags{}, S.tile_prefix);

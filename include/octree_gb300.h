@@ -281,7 +281,8 @@ OCT_API int oct_build_octree(const oct_vec4* points, int n, float min_coord, flo
 
 /* Which form stages 2-3 took in the last whole build of n points with this
  * workspace (read back after that build has finished): 0 the LSD radix passes
- * and run-head unique (clouds below 2^22 points), 1 the MSD form (top-digit
+ * and run-head unique (clouds below 2^22 points; also reported for clouds
+ * built by one launch, which sorts its own way), 1 the MSD form (top-digit
  * scatter, per-bucket bitmaps, pack), 2 the LSD form chosen by the device
  * because the top-digit buckets were too uneven. Both give the same bytes. */
 #define OCT_SORT_FORM_LSD 0
@@ -289,7 +290,8 @@ OCT_API int oct_build_octree(const oct_vec4* points, int n, float min_coord, flo
 #define OCT_SORT_FORM_LSD_FALLBACK 2
 OCT_API int oct_build_sort_form(const void* workspace, int n, int nodes_capacity, int* form);
 
-/* Timed build for measurement: the same launches as oct_build_octree, with
+/* Timed build for measurement: the stage-by-stage launches (those of
+ * oct_build_octree for clouds it does not build in one launch), with
  * caller-created CUDA events (cudaEvent_t, passed as void*) recorded on the
  * stream at each step boundary: events[k] after step k of
  * oct_build_step_name(k) for k < oct_build_step_count() (step 0 is the start).

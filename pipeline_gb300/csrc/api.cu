@@ -5,6 +5,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "kernels.cuh"
 
 using namespace octgb;
@@ -53,6 +55,7 @@ BuildLayout build_layout(int n, int cap) {
   L.tree_off = align_up(L.keys_b_off + sizeof(uint32_t) * (size_t)(n > 0 ? n : 1), 256);
   L.tags_off = align_up(L.tree_off + tree_scratch_bytes(n), 256);
   L.total = align_up(L.tags_off + oct_tags_bytes(cap), 256);
+  if (n > 0 && n <= fused_max_points()) L.total = std::max(L.total, fused_workspace_bytes(n, cap));
   return L;
 }
 
@@ -360,6 +363,30 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
   const BuildLayout L = build_layout(n, out->nodes_capacity);
   if (workspace_bytes < L.total) return OCT_ERR_WORKSPACE;
   char* w = static_cast<char*>(workspace);
+  OctArgs a{};
+  a.nodes = out->nodes;
+  a.cap = out->nodes_capacity;
+  a.offsets = out->prefix_sum;
+  a.counts = out->edge_count;
+  a.codes = out->codes;
+  a.prefix_n = out->tree.prefix_n;
+  a.hll = out->tree.has_leaf_left;
+  a.hlr = out->tree.has_leaf_right;
+  a.parent = out->tree.parent;
+  a.left_child = out->tree.left_child;
+  a.min_coord = min_coord;
+  a.range = range;
+  a.n_brt_host = n;
+  if (!rec && n <= fused_max_points()) {
+    const cudaError_t e = launch_fused_build(reinterpret_cast<const float4*>(points), n, min_coord,
+                                             range, out->codes, a, out->edge_count,
+                                             out->prefix_sum, out->d_counts, w, s);
+    if (e != cudaErrorCooperativeLaunchTooLarge) {
+      OCT_TRY(e, "build: fused");
+      return OCT_OK;
+    }
+    (void)cudaGetLastError();  // a context with fewer SMs: stage by stage
+  }
   const Misc m = misc_at(w + L.misc_off);
   uint32_t* keys_a = reinterpret_cast<uint32_t*>(w + L.keys_a_off);
   uint32_t* keys_b = reinterpret_cast<uint32_t*>(w + L.keys_b_off);
@@ -415,20 +442,6 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
           "build: prefix sum");
   mark(rec, s);
   if (out->nodes_capacity > 0) {
-    OctArgs a{};
-    a.nodes = out->nodes;
-    a.cap = out->nodes_capacity;
-    a.offsets = out->prefix_sum;
-    a.counts = out->edge_count;
-    a.codes = out->codes;
-    a.prefix_n = out->tree.prefix_n;
-    a.hll = out->tree.has_leaf_left;
-    a.hlr = out->tree.has_leaf_right;
-    a.parent = out->tree.parent;
-    a.left_child = out->tree.left_child;
-    a.min_coord = min_coord;
-    a.range = range;
-    a.n_brt_host = n;
     a.d_unique = m.unique;
     a.d_max_slot = m.max_slot;
     OCT_TRY(launch_octree(kOctMake | kOctLink | kOctFresh, a, tags, m.status, s, rec, true,

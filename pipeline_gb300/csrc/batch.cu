@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kPfThreads, 5)
                               int* __restrict__ max_slot_c,
                               const uint32_t* __restrict__ tile_prefix, OctTags tags,
                               uint32_t* __restrict__ queue) {
-  __shared__ __align__(16) PrefixSmem S;
+  __shared__ PrefixSmem<kPfThreads, kPfItems> S;
   __shared__ int s_tile;
   int round = 0;
   for (int t = next_tile(queue, round, &s_tile); t < B.T4; t = next_tile(queue, round, &s_tile)) {

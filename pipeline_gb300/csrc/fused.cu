@@ -1,0 +1,645 @@
+// The whole build of a small or medium cloud as one cooperative launch.
+//
+// Launched stage by stage, such a build is a chain of some twenty kernels of
+// 2 to 17 us that each leave most of the chip idle: launches, tail waits and
+// latencies, not work. Here one grid of at most one CTA per SM runs the stages
+// as phases with a grid barrier between them (1 to 2 us; up to eight CTAs are
+// one cluster with its hardware barrier, about half that). Launched on a
+// stream, before and after: 130 -> 33 us at 4,096 uniform points, 147 -> 47 at
+// a lidar frame of 122,880, 188 -> 103 at 1,048,576, 228 -> 162 at 1.8M. What
+// is left is the phases' latencies (2 to 4 us each) up to some 100,000 points
+// and the half-full SMs after that. The limit of 12,288 points per SM leaves
+// a quarter of the sort's 16,384 codes for the bucket that straddles the end
+// of a CTA's share; the build is still the faster one there.
+//
+//   codes    each CTA's points to Morton codes, kept in registers; a code
+//            equal to the one before it in its warp is dropped (only unique
+//            codes are needed, and scan-ordered clouds repeat them in runs);
+//            counts per top-12-bit bucket, the CTA's place in each bucket
+//            taken from the global count's atomic add
+//   scatter  bucket bases (every CTA scans the 4,096 counts), the codes to
+//            their buckets
+//   sort     a CTA takes the buckets that start in its share of the codes:
+//            sorted in shared memory and made unique; a bucket too large for
+//            that by a bitmap over its 2^18 values, which takes any number of
+//            codes, so a cloud that falls into few buckets costs time only
+//   codes    every run to its place (a scan of the CTAs' counts), the deltas
+//            of adjacent codes and the tiles' smallest
+//   tree     tree_nodes_tile, one tile per CTA (1,024 positions at least)
+//   prefix   prefix_slots_tile over the same tiles, each CTA summing the tile
+//            sums before its own
+//   emit, finalize  emit_slots per radix node, finalize_slots per slot
+//
+// The outputs are those of the tiled kernels, byte for byte.
+//
+// Grid barriers are bounded like every other wait: a CTA that gives up raises
+// OCT_STATUS_SPIN_TIMEOUT and returns, and so do the others in turn. Memory
+// that the kernel itself wrote is read through plain loads only (no
+// read-only-cache loads): the barrier's acquire makes it visible.
+#include <algorithm>
+
+#include "octree.cuh"
+#include "smem_sort.cuh"
+#include "tree_tile.cuh"
+
+namespace octgb {
+
+constexpr int kFuThreads = 1024;
+constexpr int kFuWarps = kFuThreads / 32;
+constexpr int kFuItems = 16;                       // codes per thread at most
+constexpr int kFuCap = kFuThreads * kFuItems;      // codes a CTA sorts in shared memory
+constexpr int kFuShare = 12288;                    // codes per CTA at most (the rest is slack)
+constexpr int kFuBucketBits = 12;
+constexpr int kFuBuckets = 1 << kFuBucketBits;
+constexpr int kFuSpanBits = 30 - kFuBucketBits;    // values of a bucket: a 32 KiB bitmap
+constexpr int kFuTile = 1024;                      // tree and prefix tiles: multiples of this
+constexpr uint32_t kFuBinMost = 48;  // codes in a bin before the radix sort takes over
+constexpr uint32_t kFuBinFew = 12;   // codes in a bin up to which neighbours are compared blindly
+constexpr int kFuMaxGrid = 256;
+constexpr int kFuMaxCluster = 8;                   // the portable cluster size
+constexpr int kFuMinPer = 1024;                    // points per CTA at least
+
+struct FusedLayout {
+  size_t misc_off, hist_off, zero_bytes, cta_off, keys_off, min_off, sum_off, d_off, tags_off,
+      total;
+};
+
+static FusedLayout fused_layout(int n, int cap) {
+  FusedLayout L{};
+  const size_t tiles = ((size_t)n + kFuTile - 1) / kFuTile + 1;
+  size_t o = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = o;
+    o = align_up(o + bytes, 256);
+    return at;
+  };
+  L.misc_off = take(256);
+  L.hist_off = take(4 * (size_t)kFuBuckets);
+  L.zero_bytes = o;
+  L.cta_off = take(8 * (size_t)kFuMaxGrid);
+  L.keys_off = take(4 * (size_t)n);
+  L.min_off = take(align_up(tiles, kTtMinBlock));
+  L.sum_off = take(4 * tiles);
+  L.d_off = take((size_t)n + kFuShare + 512);  // the last tile is read whole
+  L.tags_off = take(oct_tags_bytes(cap));
+  L.total = o;
+  return L;
+}
+
+struct FusedArgs {
+  const float4* pts;
+  int n;
+  float min_coord, range;
+  uint32_t* bar;     // grid barrier arrivals
+  uint32_t* hist;    // [kFuBuckets] zeroed
+  uint32_t* status;
+  int* max_slot;
+  uint32_t* cta_count;  // [grid] unique codes of a CTA's run
+  uint32_t* cta_first;  // [grid] its first code
+  uint32_t* keys;       // [n] bucketed codes
+  TreeScratch S;        // at most one tile per CTA
+  TreeOut tree;
+  uint32_t* codes;
+  int* ps;
+  OctArgs oct;
+  SlotTags tags;
+  int* d_counts;
+};
+
+struct FusedSort {
+  uint32_t a[kFuCap], b[kFuCap];
+  uint32_t base[kFuBuckets];       // counts, then the CTA's place in each bucket
+  uint32_t start[kFuBuckets + 1];  // first position of each bucket
+  RadixSmem<kFuWarps> radix;
+};
+union FusedSmem {
+  FusedSort s;
+  TreeSmem<kFuShare, kFuThreads> tree;
+  PrefixSmem<kFuThreads, kFuShare / kFuThreads> prefix;
+  int nodes[kFuThreads * kNodeWords];
+  uint32_t spread[1024];
+};
+
+// All CTAs have passed every earlier phase, and what they wrote is visible.
+// False (in every thread) when the wait ran out. A grid of one cluster uses
+// the cluster's hardware barrier.
+template <bool CLUSTER>
+__device__ __forceinline__ bool grid_barrier(const FusedArgs& A, uint32_t phase, int* s_ok) {
+  if (CLUSTER) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return true;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    red_release_add_u32(A.bar, 1u);  // after the barrier above: the whole CTA's writes
+    const uint32_t want = phase * gridDim.x;
+    WaitBound wait(kWaitLimitNs);
+    int ok = 1;
+    while (ld_acquire_u32(A.bar) < want) {
+      if (wait.expired()) {
+        raise_status(A.status, kStatusSpinTimeout);
+        atomicOr(reinterpret_cast<uint32_t*>(A.d_counts) + 3, kStatusSpinTimeout);
+        ok = 0;
+        break;
+      }
+    }
+    *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+// Heads of the sorted keys a[0, cnt) (first of each run of equal keys) to
+// dst, in order; returns their number. All threads call it.
+__device__ __forceinline__ uint32_t fused_unique(const uint32_t* a, int cnt, uint32_t* dst,
+                                                 uint32_t* warp_tot, uint32_t* total) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = ((cnt + kFuWarps - 1) / kFuWarps + 31) & ~31;
+  const int seg0 = min(wid * per, cnt), seg1 = min(seg0 + per, cnt);
+  const uint32_t mine = heads_emit(a, seg0, seg1, false, 0, nullptr);
+  const uint32_t ex = block_exclusive_sum<kFuThreads>(lane == 0 ? mine : 0u, warp_tot, total);
+  const uint32_t base = __shfl_sync(kFull, ex, 0);
+  heads_emit(a, seg0, seg1, true, base, dst);
+  __syncthreads();
+  return *total;
+}
+
+// Sorted unique codes of a bucket of any size by bitmap (bm: 2^18 bits of
+// shared memory), over the front of its own range keys[0, cnt).
+__device__ uint32_t fused_bitmap_bucket(uint32_t* keys, uint32_t cnt, uint32_t* bm,
+                                        uint32_t* warp_tot, uint32_t* total) {
+  constexpr int kWords = 1 << (kFuSpanBits - 5);
+  constexpr int kPer = kWords / kFuThreads;
+  constexpr uint32_t kMask = (1u << kFuSpanBits) - 1u;
+  const int tid = threadIdx.x;
+  for (int w = tid; w < kWords; w += kFuThreads) bm[w] = 0u;
+  const uint32_t top = keys[0] & ~kMask;
+  __syncthreads();
+  for (uint32_t i0 = tid; i0 < cnt; i0 += 4 * kFuThreads) {
+    uint32_t k[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t i = i0 + (uint32_t)q * kFuThreads;
+      k[q] = i < cnt ? keys[i] & kMask : 0xffffffffu;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (k[q] != 0xffffffffu) atomicOr(&bm[k[q] >> 5], 1u << (k[q] & 31u));
+  }
+  __syncthreads();
+  uint32_t own = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) own += __popc(bm[tid * kPer + q]);
+  uint32_t pos = block_exclusive_sum<kFuThreads>(own, warp_tot, total);
+#pragma unroll 1
+  for (int q = 0; q < kPer; ++q) {
+    uint32_t bits = bm[tid * kPer + q];
+    while (bits) {
+      const int bit = __ffs(bits) - 1;
+      bits &= bits - 1u;
+      keys[pos++] = top | ((uint32_t)(tid * kPer + q) << 5) | (uint32_t)bit;
+    }
+  }
+  __syncthreads();
+  return *total;
+}
+
+// The codes keys[0, cnt) of whole buckets (cnt <= kFuCap; global positions
+// from lo on) sorted in M.a or M.b. Every bucket has as many bins as codes,
+// spread evenly over its values, so the bins follow the cloud's density and
+// hold about one code each: one count, one scan and one scatter bring a code
+// to its bin, where it finds its place by comparing with the others. (At 7,000
+// codes a CTA 18 us by three 8-bit radix passes, 12 us so.) Codes too
+// concentrated for that, more than kFuBinMost in a bin, take the radix sort.
+__device__ __forceinline__ uint32_t* fused_sort(const uint32_t* keys, int cnt, uint32_t lo,
+                                                FusedSort& M, uint32_t* warp_tot, uint32_t* total,
+                                                uint32_t* s_span) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int items = (cnt + kFuThreads - 1) / kFuThreads;
+  auto bin_of = [&](uint32_t k) {
+    const uint32_t b = k >> kFuSpanBits, s = M.start[b], c = M.start[b + 1] - s;
+    return s - lo + (((k & ((1u << kFuSpanBits) - 1u)) * c) >> kFuSpanBits);
+  };
+  uint32_t key[kFuItems], rank2[kFuItems / 2];
+  for (int j = tid; j < items * kFuThreads; j += kFuThreads) M.a[j] = 0u;
+#pragma unroll
+  for (int it = 0; it < kFuItems; ++it) {
+    if (it >= items) break;
+    const int j = it * kFuThreads + tid;
+    key[it] = j < cnt ? keys[j] : 0u;
+  }
+  __syncthreads();
+  uint32_t most = 0;
+#pragma unroll
+  for (int it = 0; it < kFuItems; ++it) {
+    if (it >= items) break;
+    uint32_t r = 0;
+    if (it * kFuThreads + tid < cnt) r = atomicAdd(&M.a[bin_of(key[it])], 1u);
+    most = max(most, r);
+    if (it & 1) rank2[it / 2] |= r << 16;
+    else rank2[it / 2] = r;
+  }
+  most = __reduce_max_sync(kFull, most);
+  if (lane == 0) M.radix.warp_tot[tid >> 5] = most;
+  __syncthreads();
+  most = __reduce_max_sync(kFull, M.radix.warp_tot[lane]);
+  if (most >= kFuBinMost) {
+    uint32_t kmin = 0xffffffffu, kmax = 0;
+#pragma unroll
+    for (int it = 0; it < kFuItems; ++it) {
+      if (it >= items) break;
+      const int j = it * kFuThreads + tid;
+      if (j < cnt) {
+        M.a[j] = key[it];
+        kmin = min(kmin, key[it]);
+        kmax = max(kmax, key[it]);
+      }
+    }
+    if (tid == 0) {
+      s_span[0] = 0xffffffffu;
+      s_span[1] = 0u;
+    }
+    __syncthreads();
+    kmin = __reduce_min_sync(kFull, kmin);
+    kmax = __reduce_max_sync(kFull, kmax);
+    if (lane == 0) {
+      atomicMin(&s_span[0], kmin);
+      atomicMax(&s_span[1], kmax);
+    }
+    __syncthreads();
+    kmin = s_span[0];
+    return smem_radix_sort<kFuWarps, kFuItems>(M.a, M.b, cnt, kmin, 32 - __clz(s_span[1] - kmin),
+                                               M.radix);
+  }
+  // bin counts to bin starts
+  uint32_t sum = 0;
+  for (int k = 0; k < items; ++k) sum += M.a[tid * items + k];
+  uint32_t ex = block_exclusive_sum<kFuThreads>(sum, warp_tot, total);
+  for (int k = 0; k < items; ++k) {
+    const uint32_t c = M.a[tid * items + k];
+    M.a[tid * items + k] = ex;
+    ex += c;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < kFuItems; ++it) {
+    if (it >= items) break;
+    if (it * kFuThreads + tid < cnt)
+      M.b[M.a[bin_of(key[it])] + ((rank2[it / 2] >> (16 * (it & 1))) & 0xffffu)] = key[it];
+  }
+  __syncthreads();
+  // place among the bin's codes (equal ones in the order they lie)
+#pragma unroll
+  for (int it = 0; it < kFuItems; ++it) {
+    if (it >= items) break;
+    const int j = it * kFuThreads + tid;
+    uint32_t place = 0;
+    if (j < cnt && most < kFuBinFew) {
+      // codes of other bins compare the right way round, so the neighbours
+      // within the largest bin's reach are all there is to look at
+      const uint32_t* at = M.b + j;
+      const uint32_t x = at[0];
+      // (reads past either end stay inside M and don't count)
+      const int after = cnt - 1 - j;
+      int p = j;
+#pragma unroll 4
+      for (int d = 1; d <= (int)most; ++d) {
+        p += (int)(at[d] < x) & (int)(d <= after);
+        p -= (int)(at[-d] > x) & (int)(d <= j);
+      }
+      place = (uint32_t)p;
+      key[it] = x;
+    } else if (j < cnt) {
+      const uint32_t x = M.b[j];
+      const uint32_t bin = bin_of(x);
+      const int s = (int)M.a[bin];
+      const int e = (int)bin + 1 < cnt ? (int)M.a[bin + 1] : cnt;
+      place = (uint32_t)s;
+      for (int q = s; q < e; ++q) {
+        const uint32_t y = M.b[q];
+        place += y < x || (y == x && q < j) ? 1u : 0u;
+      }
+      key[it] = x;
+    }
+    if (it & 1) rank2[it / 2] |= place << 16;
+    else rank2[it / 2] = place;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < kFuItems; ++it) {
+    if (it >= items) break;
+    if (it * kFuThreads + tid < cnt) M.a[(rank2[it / 2] >> (16 * (it & 1))) & 0xffffu] = key[it];
+  }
+  __syncthreads();
+  return M.a;
+}
+
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  FusedSmem& M = *reinterpret_cast<FusedSmem*>(sm_raw);
+  __shared__ uint32_t s_warp[32], s_total;
+  __shared__ uint32_t s_cut[4];  // lo, hi, start of the straddling bucket
+  __shared__ uint32_t s_off[kFuMaxGrid];
+  __shared__ int s_next, s_ok;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t G = gridDim.x, cta = blockIdx.x;
+  uint32_t phase = 0;
+
+  // ---- codes and bucket counts
+  const int per = (int)(((uint32_t)A.n + G - 1u) / G);
+  const int t0 = (int)min((long long)cta * per, (long long)A.n), t1 = min(t0 + per, A.n);
+  uint32_t code[kFuItems];
+  uint32_t rank2[kFuItems / 2];  // 16-bit ranks in the bucket, 0xffff: dropped
+  {
+    uint32_t* cnt = M.s.base;
+    uint32_t* lut = M.spread;
+    for (int b = tid; b < kFuBuckets; b += kFuThreads) cnt[b] = 0u;
+    if (CLUSTER) {  // no memset was launched
+      for (int b = (int)cta * kFuThreads + tid; b < kFuBuckets; b += (int)G * kFuThreads)
+        A.hist[b] = 0u;
+      if (cta == 0 && tid == 0) {
+        *A.status = 0u;
+        *A.max_slot = 0;
+      }
+    }
+    fill_spread_lut(lut);
+    // tile sums and minima start empty (used three barriers later)
+    const int pad = (int)align_up((size_t)A.S.tiles, kTtMinBlock);
+    for (int k = (int)cta * kFuThreads + tid; k < pad; k += (int)G * kFuThreads) {
+      A.S.tile_min[k] = (uint8_t)kTtAbsent;
+      if (k < A.S.tiles) A.S.tile_sum[k] = 0;
+    }
+    __syncthreads();
+    const float scale = __fdiv_rn(1024.0f, A.range);
+    bool bad = false;
+#pragma unroll
+    for (int h = 0; h < kFuItems; h += 4) {
+      if (h * kFuThreads < per) {
+        float4 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = t0 + (h + u) * kFuThreads + tid;
+          if (i < t1) p[u] = ld_stream_f4(A.pts + i);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = t0 + (h + u) * kFuThreads + tid;
+          uint32_t c = 0, r = 0xffffu;
+          if (i < t1) {
+            bool ok;
+            c = morton_code_lut(p[u].x, p[u].y, p[u].z, A.min_coord, A.range, scale, lut, ok);
+            bad |= !ok;
+          }
+          // the valid lanes are a prefix of the warp
+          const uint32_t prev = __shfl_up_sync(kFull, c, 1);
+          if (i < t1 && (lane == 0 || prev != c)) r = atomicAdd(&cnt[c >> kFuSpanBits], 1u);
+          code[h + u] = c;
+          if (u & 1) rank2[(h + u) / 2] |= r << 16;
+          else rank2[(h + u) / 2] = r;
+        }
+      }
+    }
+    const bool any_bad = __syncthreads_or(bad);
+    if (CLUSTER) grid_barrier<CLUSTER>(A, 0, &s_ok);  // the counts are cleared
+    if (any_bad && tid == 0) raise_status(A.status, kStatusRange);
+    // the CTA's place in each bucket
+#pragma unroll
+    for (int k = 0; k < kFuBuckets / kFuThreads; ++k) {
+      const int b = k * kFuThreads + tid;
+      const uint32_t c = cnt[b];
+      if (c) cnt[b] = atomicAdd(A.hist + b, c);
+    }
+  }
+  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+
+  // ---- scatter into buckets; this CTA's share of them
+  uint32_t lo, hi, cut, share;
+  {
+    constexpr int kPer = kFuBuckets / kFuThreads;
+    static_assert(kPer == 4, "one 16-byte load of counts per thread");
+    const uint4 q = reinterpret_cast<const uint4*>(A.hist)[tid];
+    const uint32_t c[kPer] = {q.x, q.y, q.z, q.w};
+    uint32_t ex = block_exclusive_sum<kFuThreads>(c[0] + c[1] + c[2] + c[3], s_warp, &s_total);
+    const uint32_t kept = s_total;
+    share = (kept + G - 1u) / G;
+    const uint32_t w0 = min(cta * share, kept), w1 = min(w0 + share, kept);
+    if (tid == 0) {
+      s_cut[0] = w0 == 0 ? 0u : kept;
+      s_cut[1] = kept;
+      s_cut[2] = kept;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      // a boundary inside or at the end of this bucket moves to its end
+      if (ex < w0 && w0 <= ex + c[k]) s_cut[0] = ex + c[k];
+      if (ex < w1 && w1 <= ex + c[k]) {
+        s_cut[1] = ex + c[k];
+        s_cut[2] = ex;
+      }
+      M.s.start[kPer * tid + k] = ex;
+      M.s.base[kPer * tid + k] += ex;
+      ex += c[k];
+    }
+    if (tid == kFuThreads - 1) M.s.start[kFuBuckets] = ex;
+    __syncthreads();
+    lo = s_cut[0];
+    hi = max(s_cut[1], lo);
+    cut = max(s_cut[2], lo);
+#pragma unroll
+    for (int it = 0; it < kFuItems; ++it) {
+      if (it * kFuThreads >= per) break;
+      const uint32_t r = (rank2[it / 2] >> (16 * (it & 1))) & 0xffffu;
+      if (r != 0xffffu) A.keys[M.s.base[code[it] >> kFuSpanBits] + r] = code[it];
+    }
+  }
+  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+
+  // ---- sort and unique: [lo, cut) with the straddling bucket [cut, hi), which
+  // goes alone by bitmap (a few us whatever it holds) when it is large beside
+  // the CTA's share or both do not fit
+  const uint32_t* run;
+  uint32_t u_small, u_big = 0;
+  {
+    const bool big = hi - lo > (uint32_t)kFuCap ||
+                     (hi - cut > 2u * (uint32_t)kFuThreads && hi - cut > 2u * share);
+    const int cnt = (int)min((big ? cut : hi) - lo, (uint32_t)kFuCap);
+    uint32_t* sorted = fused_sort(A.keys + lo, cnt, lo, M.s, s_warp, &s_total, s_cut);
+    uint32_t* other = sorted == M.s.a ? M.s.b : M.s.a;
+    u_small = fused_unique(sorted, cnt, other, s_warp, &s_total);
+    run = other;
+    __syncthreads();
+    if (big) u_big = fused_bitmap_bucket(A.keys + cut, hi - cut, sorted, s_warp, &s_total);
+    if (tid == 0) {
+      A.cta_count[cta] = u_small + u_big;
+      A.cta_first[cta] = u_small ? run[0] : u_big ? A.keys[cut] : 0u;
+    }
+  }
+  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+
+  // ---- unique codes and deltas to their places
+  int n_unique, tile;
+  {
+    const uint32_t mine = tid < (int)G ? A.cta_count[tid] : 0u;
+    uint32_t* tmin = M.s.base;  // smallest deltas of the tiles this run touches
+    for (int k = tid; k < kFuBuckets; k += kFuThreads) tmin[k] = kTtAbsent;
+    if (tid == 0) s_next = 0x7fffffff;
+    const uint32_t ex = block_exclusive_sum<kFuThreads>(mine, s_warp, &s_total);
+    if (tid < (int)G) s_off[tid] = ex;
+    if (tid < (int)G && tid > (int)cta && mine > 0) atomicMin(&s_next, tid);
+    __syncthreads();
+    n_unique = (int)s_total;
+    // one tile per CTA where that fills the chip
+    tile = (int)((s_total + G * kFuTile - 1u) / (G * kFuTile)) * kFuTile;
+    const uint32_t off = s_off[cta], u = u_small + u_big;
+    const uint32_t after = s_next < (int)G ? A.cta_first[s_next] : 0u;
+    const uint32_t* far = A.keys + cut;
+    auto at = [&](uint32_t j) { return j < u_small ? run[j] : far[j - u_small]; };
+    const uint32_t t_first = off / (uint32_t)tile;
+    uint32_t ta = t_first, ta_end = (t_first + 1u) * (uint32_t)tile;
+    for (uint32_t j0 = tid & ~31u; j0 < u; j0 += kFuThreads) {
+      const uint32_t j = j0 + lane;
+      uint32_t d = kTtAbsent;
+      const uint32_t pos = off + j;
+      if (j < u) {
+        const uint32_t c = at(j);
+        A.codes[pos] = c;
+        if (pos + 1u < (uint32_t)n_unique) {
+          d = tt_delta(c, j + 1u < u ? at(j + 1u) : after);
+          A.S.D[pos] = (uint8_t)d;
+        }
+      }
+      // the warp's 32 positions lie in one tile or two
+      while (off + j0 >= ta_end) {
+        ++ta;
+        ta_end += (uint32_t)tile;
+      }
+      const uint32_t ma = __reduce_min_sync(kFull, pos < ta_end ? d : kTtAbsent);
+      const uint32_t mb = __reduce_min_sync(kFull, pos < ta_end ? kTtAbsent : d);
+      if (lane == 0 && ma < kTtAbsent) atomicMin(&tmin[ta - t_first], ma);
+      if (lane == 0 && mb < kTtAbsent) atomicMin(&tmin[ta + 1u - t_first], mb);
+    }
+    __syncthreads();
+    const uint32_t touched = u ? (off + u - 1u) / (uint32_t)tile - t_first + 1u : 0u;
+    for (uint32_t k = tid; k < touched; k += kFuThreads)
+      if (tmin[k] < kTtAbsent) atomic_min_u8(A.S.tile_min + t_first + k, tmin[k]);
+  }
+  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+
+  // ---- radix tree and edge counts
+  const int n_brt = max(n_unique - 1, 0);
+  const int tiles = (n_brt + tile - 1) / tile;  // at most one per CTA
+  if ((int)cta < tiles) {
+    const TileInfo I{(int)cta, 0, tiles - 1, n_brt, (int)cta * tile, 0};
+    tree_nodes_tile(M.tree, SizedTile{tile}, I, A.codes, A.S, A.tree);
+  }
+  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+
+  // ---- prefix sums, octree tags
+  if ((int)cta < tiles) {
+    const uint32_t sum = tid < (int)cta ? (uint32_t)A.S.tile_sum[tid] : 0u;
+    block_exclusive_sum<kFuThreads>(sum, s_warp, &s_total);
+    const uint32_t before = s_total;
+    __syncthreads();
+    prefix_slots_tile(M.prefix, A.tree.ec, A.ps, n_brt, (int)cta * tile, before, A.tags,
+                      A.max_slot, tile / kFuThreads);
+    if (tid == 0) bulk_wait_all();
+  }
+  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+
+  // ---- octree
+  const int n_oct = n_brt >= 1 ? *A.max_slot + 1 : 0;
+  const bool octree = A.oct.cap > 0;
+  const bool fits = n_oct <= A.oct.cap;
+  if (octree) {
+    if (!fits) {
+      if (cta == 0 && tid == 0) raise_status(A.status, kStatusCapacity);
+    } else {
+      for (int i = (int)cta * kFuThreads + tid; i < n_brt; i += (int)G * kFuThreads)
+        emit_slots(i, A.oct, A.tags, n_brt, n_oct);
+    }
+    if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+  }
+  if (cta == 0 && tid == kFuThreads - 1) {  // every status bit is up
+    A.d_counts[0] = n_unique;
+    A.d_counts[1] = n_brt;
+    A.d_counts[2] = n_oct;
+    A.d_counts[3] = (int)*reinterpret_cast<volatile uint32_t*>(A.status);
+  }
+  if (octree) {
+    if (fits && n_brt >= 1) {
+      const int root_level = A.tree.prefix_n[0] / 3;
+      for (int blk = (int)cta * kFuThreads; blk < n_oct; blk += (int)G * kFuThreads) {
+        const int p = blk + tid;
+        if (p < n_oct)
+          finalize_slots(p, A.oct, A.tags, n_brt, root_level, M.nodes + tid * kNodeWords);
+        store_node_block(M.nodes, A.oct.nodes + blk, min(kFuThreads, n_oct - blk));
+      }
+      if (tid == 0) bulk_wait_all();
+    }
+  }
+}
+
+size_t fused_workspace_bytes(int n, int cap) { return fused_layout(n, cap).total; }
+
+int fused_max_points() { return device_sm_count() * kFuShare; }
+
+cudaError_t launch_fused_build(const float4* pts, int n, float min_coord, float range,
+                               uint32_t* codes, const OctArgs& oct, int* ec, int* ps,
+                               int* d_counts, void* workspace, cudaStream_t s) {
+  const FusedLayout L = fused_layout(n, oct.cap);
+  char* w = static_cast<char*>(workspace);
+  const int grid = std::max(1, std::min((n + kFuMinPer - 1) / kFuMinPer,
+                                        std::min(device_sm_count(), kFuMaxGrid)));
+  FusedArgs A{};
+  A.pts = pts;
+  A.n = n;
+  A.min_coord = min_coord;
+  A.range = range;
+  A.status = reinterpret_cast<uint32_t*>(w + L.misc_off);
+  A.bar = A.status + 1;
+  A.max_slot = reinterpret_cast<int*>(A.status + 2);
+  A.hist = reinterpret_cast<uint32_t*>(w + L.hist_off);
+  A.cta_count = reinterpret_cast<uint32_t*>(w + L.cta_off);
+  A.cta_first = A.cta_count + kFuMaxGrid;
+  A.keys = reinterpret_cast<uint32_t*>(w + L.keys_off);
+  A.S.D = reinterpret_cast<uint8_t*>(w + L.d_off);
+  A.S.tile_min = reinterpret_cast<uint8_t*>(w + L.min_off);
+  A.S.tile_sum = reinterpret_cast<int*>(w + L.sum_off);
+  A.S.tiles = (n + kFuTile - 1) / kFuTile;
+  A.tree = TreeOut{const_cast<uint8_t*>(oct.prefix_n), const_cast<uint8_t*>(oct.hll),
+                   const_cast<uint8_t*>(oct.hlr), const_cast<int*>(oct.left_child),
+                   const_cast<int*>(oct.parent), ec};
+  A.codes = codes;
+  A.ps = ps;
+  A.oct = oct;
+  A.tags = slot_tags(oct_tags_carve(w + L.tags_off, oct.cap), 0, oct.cap);
+  A.d_counts = d_counts;
+  const int smem = (int)sizeof(FusedSmem);
+  const bool cluster = grid <= kFuMaxCluster;
+  auto kernel = cluster ? fused_build_kernel<true> : fused_build_kernel<false>;
+  cudaError_t e = set_smem_limit(kernel, smem);
+  if (e != cudaSuccess) return e;
+  if (!cluster) e = cudaMemsetAsync(w + L.misc_off, 0, L.zero_bytes, s);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(kFuThreads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  if (cluster) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {(unsigned)grid, 1u, 1u};
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  }
+  c.attrs = at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, A);
+}
+
+}  // namespace octgb

@@ -378,6 +378,15 @@ cudaError_t launch_prefix_sum_clear_tags(int n_host, const int* d_unique, int* e
                                          int* d_max_slot, void* tree_scratch, uint32_t* status,
                                          const OctTags& tags, bool slots, cudaStream_t s);
 
+// The whole build of a cloud of at most fused_max_points() points in one
+// cooperative launch (fused.cu). oct holds the tree's output arrays as well.
+// cudaErrorCooperativeLaunchTooLarge: the grid does not fit this context.
+int fused_max_points();
+size_t fused_workspace_bytes(int n, int cap);
+cudaError_t launch_fused_build(const float4* pts, int n, float min_coord, float range,
+                               uint32_t* codes, const OctArgs& oct, int* ec, int* ps,
+                               int* d_counts, void* workspace, cudaStream_t s);
+
 // Copies U, B, M, status into out[4] (device).
 cudaError_t launch_publish_counts(const int* d_unique, const int* d_max_slot,
                                   const uint32_t* status, int* out, cudaStream_t s);

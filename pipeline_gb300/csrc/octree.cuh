@@ -200,7 +200,7 @@ __device__ __forceinline__ void slot_mark(const SlotTags& t, int slot, uint32_t 
   atomicOr(w, 1u << (sh + (int)which));
 }
 
-// Inclusive prefix sum of one tile of 4,096 edge counts of a cloud, with the
+// Inclusive prefix sum of one tile of edge counts of a cloud, with the
 // slot tags' preparation of the slots it covers: child tags and masks zeroed,
 // each slot's radix node written. The tile's own slots are (ex, ex + total];
 // the next nine may hold the last node's further steps and are cleared as
@@ -217,10 +217,12 @@ constexpr int kPfTile = kPfThreads * kPfItems;  // the radix-tree tiles
 constexpr int kPfZero = 4096;                   // bytes of the zero block
 constexpr int kMaxSteps = 10;                   // octree levels one radix node can span
 
+template <int THREADS, int ITEMS>
 struct PrefixSmem {
-  uint4 zero[kPfZero / 16];
-  uint32_t node[kPfTile];  // by slot after the tile's prefix: (tile's node + 1) << 4 | step
-  int v[kPfTile + kPfTile / 32];  // padded: entry j at j + j / 32
+  static constexpr int kTile = THREADS * ITEMS;
+  __align__(16) uint4 zero[kPfZero / 16];
+  __align__(16) uint32_t node[kTile];  // by slot after the tile's prefix: (tile's node + 1) << 4 | step
+  int v[kTile + kTile / 32];  // padded: entry j at j + j / 32
   uint32_t warp[32];
   uint32_t total;
   int max_slot;
@@ -228,34 +230,37 @@ struct PrefixSmem {
 
 __device__ __forceinline__ int pf_pad(int j) { return j + (j >> 5); }
 
-// ec, ps: the cloud's arrays; the tile's nodes are [lo, min(lo + 4096, n)), its
+// ec, ps: the cloud's arrays; the tile's nodes are [lo, min(lo + kTile, n)), its
 // exclusive prefix ex. max_slot: raised to the largest slot stages 7-8 write.
 // All threads call it; ends with a barrier.
-__device__ __forceinline__ void prefix_slots_tile(PrefixSmem& S, const int* __restrict__ ec,
-                                                  int* __restrict__ ps, int n, int lo, uint32_t ex,
-                                                  const SlotTags& t, int* max_slot) {
+template <int THREADS, int ITEMS>
+__device__ __forceinline__ void prefix_slots_tile(PrefixSmem<THREADS, ITEMS>& S, const int* ec,
+                                                  int* ps, int n, int lo, uint32_t ex,
+                                                  const SlotTags& t, int* max_slot,
+                                                int items = ITEMS) {
+  constexpr int kTile = THREADS * ITEMS;  // at most; the tile has THREADS * items
   const int tid = threadIdx.x;
-  const int valid = min(kPfTile, n - lo);
+  const int valid = min(THREADS * items, n - lo);
 #pragma unroll
-  for (int k = 0; k < kPfItems; ++k) {
-    const int j = k * kPfThreads + tid;
+  for (int k = 0; k < ITEMS; ++k) {
+    if (k >= items) break;
+    const int j = k * THREADS + tid;
     S.v[pf_pad(j)] = j < valid ? ec[lo + j] : 0;
   }
-  S.zero[tid] = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-  for (int q = 0; q < kPfTile / 4 / kPfThreads; ++q)
-    reinterpret_cast<uint4*>(S.node)[tid + q * kPfThreads] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid < kPfZero / 16) S.zero[tid] = make_uint4(0u, 0u, 0u, 0u);
+  for (int q = tid; q < kTile / 4; q += THREADS)
+    reinterpret_cast<uint4*>(S.node)[q] = make_uint4(0u, 0u, 0u, 0u);
   if (tid == 0) S.max_slot = 0;
   bulk_fence_writes();
   __syncthreads();
-  int v[kPfItems];
+  int v[ITEMS];
   uint32_t sum = 0;
 #pragma unroll
-  for (int k = 0; k < kPfItems; ++k) {
-    v[k] = S.v[pf_pad(tid * kPfItems + k)];
+  for (int k = 0; k < ITEMS; ++k) {
+    v[k] = k < items ? S.v[pf_pad(tid * items + k)] : 0;
     sum += (uint32_t)v[k];
   }
-  const uint32_t off = block_exclusive_sum<kPfThreads>(sum, S.warp, &S.total);
+  const uint32_t off = block_exclusive_sum<THREADS>(sum, S.warp, &S.total);
   const uint32_t total = S.total;
   const uint32_t cap = (uint32_t)t.cap;
   if (ex < cap) {
@@ -266,18 +271,19 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem& S, const int* __re
       for (size_t b = 0; b < bytes; b += kPfZero)
         bulk_store_s2g(dst + b, S.zero, (uint32_t)min((size_t)kPfZero, bytes - b));
     }
-    clear_mask_range(t, (int)ex, (int)hi, tid, kPfThreads);
+    clear_mask_range(t, (int)ex, (int)hi, tid, THREADS);
   }
   // (Bounds on run and v: counts of a malformed tree, see emit_slots.)
   // a tile covers at most its nodes' slots; more than the stage holds only
   // when many nodes span several levels
-  const bool staged = total <= (uint32_t)kPfTile;
+  const bool staged = total <= (uint32_t)kTile;
   uint32_t run = ex + off;
   int mx = 0;
   uint32_t multi = 0;  // items that span several levels
 #pragma unroll
-  for (int k = 0; k < kPfItems; ++k) {
-    const int j = tid * kPfItems + k;
+  for (int k = 0; k < ITEMS; ++k) {
+    if (k >= items) break;
+    const int j = tid * items + k;
     run += (uint32_t)v[k];
     S.v[pf_pad(j)] = (int)run;  // each thread rewrites only its own entries
     const int i = lo + j;
@@ -286,12 +292,12 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem& S, const int* __re
     if (makes) mx = max(mx, (int)run + v[k] - 1);
     if (makes && v[k] > 1) multi |= 1u << k;
     // the node's own slot: later nodes win over earlier nodes' further steps
-    if (makes && q < (uint32_t)kPfTile) atomicMax(&S.node[q], (uint32_t)(j + 1) << 4);
+    if (makes && q < (uint32_t)kTile) atomicMax(&S.node[q], (uint32_t)(j + 1) << 4);
     if (i == n - 1) mx = max(mx, (int)run);
   }
   // further steps, one such node of each lane at a time
   while (staged && multi) {
-    const int j = tid * kPfItems + __ffs(multi) - 1;
+    const int j = tid * items + __ffs(multi) - 1;
     multi &= multi - 1u;
     const uint32_t q = (uint32_t)S.v[pf_pad(j)] - ex - 1u;
     const uint32_t k = (uint32_t)min(ec[lo + j], kMaxSteps);
@@ -301,8 +307,8 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem& S, const int* __re
   if (!staged) {
     // the node's own slot only, none for those up to the one before it
 #pragma unroll 1
-    for (int k = 0; k < kPfItems; ++k) {
-      const int j = tid * kPfItems + k;
+    for (int k = 0; k < items; ++k) {
+      const int j = tid * items + k;
       const uint32_t r = (uint32_t)S.v[pf_pad(j)];
       const int kk = j < valid && lo + j > 0 ? min(ec[lo + j], kMaxSteps) : 0;
       for (int h = 1; h < kk; ++h)
@@ -315,12 +321,13 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem& S, const int* __re
   __syncthreads();
   if (tid == 0) atomicMax(max_slot, S.max_slot);
 #pragma unroll
-  for (int k = 0; k < kPfItems; ++k) {
-    const int j = k * kPfThreads + tid;
+  for (int k = 0; k < ITEMS; ++k) {
+    if (k >= items) break;
+    const int j = k * THREADS + tid;
     if (j < valid) ps[lo + j] = S.v[pf_pad(j)];
   }
   if (staged) {
-    for (uint32_t q = tid; q < total; q += kPfThreads) {
+    for (uint32_t q = tid; q < total; q += THREADS) {
       const uint32_t slot = ex + 1u + q;
       const uint32_t e = S.node[q];
       // the tile before may reach its first few slots: left open
@@ -330,7 +337,7 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem& S, const int* __re
   }
   // slot 0 (the root's) and the slots after the last node's prefix have none
   if (lo == 0 && tid == 0 && cap > 0) t.node[0] = 0u;
-  if (lo + kPfTile >= n && tid < kMaxSteps) {
+  if (lo + THREADS * items >= n && tid < kMaxSteps) {
     const uint32_t slot = ex + total + 1u + (uint32_t)tid;
     if (slot < cap) t.node[slot] = 0u;
   }

@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(kPfThreads, 5)
                         int* __restrict__ ps, int* __restrict__ d_max_slot,
                         const uint32_t* __restrict__ tile_prefix, SlotTags t) {
   chain_enter();
-  __shared__ __align__(16) PrefixSmem S;
+  __shared__ PrefixSmem<kPfThreads, kPfItems> S;
   const int n = d_unique ? max(*d_unique - 1, 0) : n_host;
   const int lo = blockIdx.x * kPfTile;
   if (lo >= n) return;

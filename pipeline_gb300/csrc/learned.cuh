@@ -113,7 +113,8 @@ __device__ __forceinline__ uint32_t lcdf_bucket(const LcdfTables& t, uint32_t v)
 }
 
 cudaError_t launch_lcdf_fit(const uint32_t* sorted_sample, int S, int k_req, int steps, float lr,
-                            char* blob, const LcdfLayout& L, int nb, cudaStream_t s);
+                            char* blob, const LcdfLayout& L, int nb, void* moments,
+                            cudaStream_t s);
 cudaError_t launch_lcdf_train(const uint32_t* sorted_sample, int S, int steps, float lr, char* blob,
                               const LcdfLayout& L, cudaStream_t s);
 cudaError_t launch_lcdf_loss_grad(const uint32_t* sorted_sample, int S, char* blob,

@@ -449,12 +449,16 @@ __global__ void __launch_bounds__(kFinThreads, 6)
   }
 }
 
-// The same stages with slot tags (octree.cuh).
-__global__ void __launch_bounds__(256, 6)
+// The same stages with slot tags (octree.cuh): a CTA takes a 4,096-node tile in
+// four parts.
+__global__ void __launch_bounds__(kEmitThreads, 6)
     batch_slot_emit_kernel(BatchDev B, BatchOctDev O, uint32_t* __restrict__ status,
                            uint32_t* __restrict__ queue) {
+  __shared__ EmitSmem M;
   __shared__ int s_tile;
   int round = 0;
+  uint32_t phase = 0;
+  if (threadIdx.x == 0) mbar_init(&M.bar, 1);
   for (int k = next_tile(queue, round, &s_tile); k < B.T4; k = next_tile(queue, round, &s_tile)) {
     const int4 d = B.tiles4k[k];
     const int c = d.z;
@@ -467,40 +471,63 @@ __global__ void __launch_bounds__(256, 6)
     const int end = min(d.y - cs, z.n_brt);
     const OctArgs a = cloud_view(B, O, z);
     const SlotTags t = slot_tags(O.tags, z.ns, z.cap);
-    for (int i = d.x - cs + (int)threadIdx.x; i < end; i += 256)
-      emit_slots(i, a, t, z.n_brt, z.n_oct);
+    for (int lo = d.x - cs; lo < end; lo += kEmitTile) {
+      const int n = min(kEmitTile, end - lo);
+      bool ok;
+      const uint32_t shift = load_emit_tile(M, a, (uint32_t)cs, (uint32_t)lo, (uint32_t)n,
+                                            (uint32_t)B.N, phase, status, ok);
+      if (!ok) return;
+      phase ^= 1u;
+      emit_tile(M, a, t, (uint32_t)lo, (uint32_t)n, shift, z.n_brt, z.n_oct);
+      bulk_fence_writes();
+      __syncthreads();  // M is the next part's
+    }
   }
 }
 
 // The clouds' written slots in blocks of 256: block first_block[c] is cloud
 // c's first. Without a queue each CTA of one wave takes a contiguous run of
-// the blocks and finds its first cloud once; with one, blocks come from the
-// queue. A CTA per 256 slots of the capacity (289,490 CTAs on the 512-cloud
-// batch, more than half of them past their cloud's last node) took
-// 0.970 ms there (with node tags), this 0.731 ms.
-__global__ void __launch_bounds__(kFinThreads, 6)
+// the blocks and looks a cloud up once (its view is kept in shared memory);
+// with one, blocks come from the queue. A CTA per 256 slots of the capacity
+// (289,490 CTAs on the 512-cloud batch, more than half of them past their
+// cloud's last node) took 0.970 ms there (with node tags), this 0.635 ms.
+__global__ void __launch_bounds__(kFinThreads, 8)
     batch_slot_finalize_kernel(BatchDev B, BatchOctDev O, const int* __restrict__ first_block,
                                uint32_t* __restrict__ queue) {
   __shared__ __align__(16) int s_nodes[kFinThreads * kNodeWords];
-  __shared__ int s_tile;
+  __shared__ OctArgs s_a;
+  __shared__ SlotTags s_t;
+  __shared__ int s_tile, s_first, s_stop, s_brt, s_oct, s_level;
   const int blocks = first_block[B.C];
   int round = 0;
   int k = (int)((long long)blocks * blockIdx.x / gridDim.x);
-  const int end = (int)((long long)blocks * (blockIdx.x + 1) / gridDim.x);
-  int c = -1;
+  const int end = queue ? blocks : (int)((long long)blocks * (blockIdx.x + 1) / gridDim.x);
+  if (threadIdx.x == 0) s_first = s_stop = 0;
+  __syncthreads();
   for (;; ++k) {
     if (queue) k = next_tile(queue, round, &s_tile);
-    if (k >= (queue ? blocks : end)) break;
-    if (c < 0 || queue) c = cloud_of(first_block, B.C, k);
-    while (k >= first_block[c + 1]) ++c;
-    const CloudSizes z = cloud_sizes(B, O, c);
-    const int p0 = (k - first_block[c]) * kFinThreads;
-    const int count = min(kFinThreads, z.n_oct - p0);
-    const OctArgs a = cloud_view(B, O, z);
+    if (k >= end) break;
+    if (k < s_first || k >= s_stop) {  // another cloud (the same in every thread)
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        const int c = cloud_of(first_block, B.C, k);
+        const CloudSizes z = cloud_sizes(B, O, c);
+        s_a = cloud_view(B, O, z);
+        s_t = slot_tags(O.tags, z.ns, z.cap);
+        s_brt = z.n_brt;
+        s_oct = z.n_oct;
+        s_level = s_a.prefix_n[0] / 3;
+        s_first = first_block[c];
+        s_stop = first_block[c + 1];
+      }
+      __syncthreads();
+    }
+    const int p0 = (k - s_first) * kFinThreads;
+    const int count = min(kFinThreads, s_oct - p0);
     if ((int)threadIdx.x < count)
-      finalize_slots(p0 + (int)threadIdx.x, a, slot_tags(O.tags, z.ns, z.cap), z.n_brt,
-                     a.prefix_n[0] / 3, s_nodes + threadIdx.x * kNodeWords);
-    store_node_block(s_nodes, a.nodes + p0, count);
+      finalize_slots(p0 + (int)threadIdx.x, s_a, s_t, s_brt, s_level,
+                     s_nodes + threadIdx.x * kNodeWords);
+    store_node_block(s_nodes, s_a.nodes + p0, count);
   }
   if (threadIdx.x == 0) bulk_wait_all();
 }
@@ -867,7 +894,7 @@ int batch_build(const oct_batch_plan* P, const void* d_tables, const oct_vec4* p
           B, O, status, emit_queue);
     batch_publish_kernel<<<1, 1024, 0, s>>>(B, O, status, d_cloud_counts, first_block);
     if (P->slots) {
-      const int grid = std::max(1, std::min(B.Tn, sms * 6));
+      const int grid = std::max(1, std::min(B.Tn, sms * 8));
       batch_slot_finalize_kernel<<<grid, kFinThreads, 0, s>>>(B, O, first_block, fin_queue);
     } else if (B.Tn > 0) {
       batch_oct_finalize_kernel<<<queue_grid(batch_oct_finalize_kernel, kFinThreads, B.Tn, queue),

@@ -89,17 +89,25 @@ __global__ void __launch_bounds__(kFinThreads, 8) oct_finalize_kernel(int mode, 
   if (threadIdx.x == 0) bulk_wait_all();
 }
 
-// The same stages with slot tags (whole builds): launch bounds and grids as above.
-__global__ void __launch_bounds__(256, 8)
+// The same stages with slot tags (whole builds).
+__global__ void __launch_bounds__(kEmitThreads, 8)
     slot_emit_kernel(OctArgs a, SlotTags t, uint32_t* __restrict__ status) {
   chain_enter();
+  __shared__ EmitSmem M;
   const Sizes z = read_sizes(a);
   if (!z.fits) {
     if (blockIdx.x == 0 && threadIdx.x == 0) raise_status(status, kStatusCapacity);
     return;
   }
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < z.n_brt) emit_slots(i, a, t, z.n_brt, z.n_oct);
+  const int lo = (int)blockIdx.x * kEmitTile;
+  if (lo >= z.n_brt) return;
+  const int n = min(kEmitTile, z.n_brt - lo);
+  if (threadIdx.x == 0) mbar_init(&M.bar, 1);
+  bool ok;
+  const uint32_t shift = load_emit_tile(M, a, 0u, (uint32_t)lo, (uint32_t)n,
+                                        (uint32_t)a.n_brt_host, 0u, status, ok);
+  if (!ok) return;
+  emit_tile(M, a, t, (uint32_t)lo, (uint32_t)n, shift, z.n_brt, z.n_oct);
 }
 
 __global__ void __launch_bounds__(kFinThreads, 8) slot_finalize_kernel(OctArgs a, SlotTags t) {
@@ -129,8 +137,8 @@ cudaError_t launch_octree(int mode, const OctArgs& a, const OctTags& t, uint32_t
   int egrid = (nb + 255) / 256;
   if (egrid < 1) egrid = 1;
   if (slots)
-    e = launch_chained(slot_emit_kernel, dim3(egrid), dim3(256), 0, s, a, slot_tags(t, 0, a.cap),
-                       status);
+    e = launch_chained(slot_emit_kernel, dim3((std::max(nb, 1) + kEmitTile - 1) / kEmitTile),
+                       dim3(kEmitThreads), 0, s, a, slot_tags(t, 0, a.cap), status);
   else
     e = launch_chained(oct_emit_kernel, dim3(egrid), dim3(256), 0, s, mode, a, t, status,
                        tags_clear);

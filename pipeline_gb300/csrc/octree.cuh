@@ -181,7 +181,7 @@ __device__ __forceinline__ float cell_size(float range, int k) {
 // with prefix s, later nodes overwrite, and the prefix sum's tiles note each
 // slot's node and step (SlotTags::node). The masks take one byte per slot.
 // Against node tags (owner tag, 4-byte mask, two table reads per child):
-// emit 0.202 -> 0.186 ms (285 -> 236 warp instructions per 32 nodes; bound by its
+// emit 0.202 -> 0.186 ms (285 -> 236 warp instructions per 32 nodes; bound by its L2
 // dependent loads), finalize 0.152 -> 0.132 ms (416 -> 288 per 32 slots; bound by
 // DRAM, 5.8 TB/s) at 16.7M uniform points.
 constexpr uint32_t kNoNode = 15u;  // SlotTags::node: no node's slots reach this one (0: open)
@@ -345,67 +345,227 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem<THREADS, ITEMS>& S,
   __syncthreads();
 }
 
-// Every write radix node i makes. The tree is this library's own, so a walk
-// ends at a node with octree nodes or at node 0 after at most 30 steps, every
-// index is below n_brt and every slot below n_oct (n_oct - 1 is the largest
-// slot written). The clamps only matter after a status bit was raised (a
-// sort whose look-back timed out leaves no tree): nothing goes out of bounds.
+// The octree writes of one radix node. The tree is this library's own, so a
+// walk to the first node with octree nodes ends there or at node 0 after at
+// most 30 steps, every index is below n_brt and every slot below n_oct
+// (n_oct - 1 is the largest slot written). The clamps on indexes and slots only
+// matter after a status bit was raised (a sort whose look-back timed out leaves
+// no tree): nothing goes out of bounds.
+struct EmitNode {
+  int i, k, base;        // node, octree nodes, prefix
+  uint32_t code, level;  // the node's own code; prefix length / 3
+};
+
+// MakeOctNodes (include/shared/oct.h:24-90) of a node with octree nodes; up:
+// the slot of the first node above it that has some.
+__device__ __forceinline__ void emit_make(const EmitNode& e, uint32_t up, const SlotTags& t,
+                                          uint32_t top_slot) {
+  const uint32_t s16 = (uint32_t)e.base << 4;
+  for (int j = 0; j < e.k - 1; ++j) {
+    const uint32_t which = (e.code >> (30 - 3 * ((int)e.level - j))) & 7u;
+    const int slot = (int)min((uint32_t)(e.base + j + 1), top_slot);
+    slot_put(t, slot, which, s16 | (uint32_t)j);
+    slot_mark(t, slot, which);
+  }
+  const uint32_t which = (e.code >> (30 - 3 * ((int)e.level - e.k + 1))) & 7u;
+  const int slot = (int)min(up, top_slot);
+  slot_put(t, slot, which, s16 | (uint32_t)(e.k - 1));
+  slot_mark(t, slot, which);
+}
+
+// LinkLeafNodes (include/shared/oct.h:92-134, the walk ended at radix node 0)
+// of one leaf, code c: node i's left leaf is leaf i - back, its right one
+// i + ahead.
+__device__ __forceinline__ void emit_leaf(int i, uint32_t level, uint32_t dst, uint32_t c,
+                                          uint32_t field, int bits, const SlotTags& t,
+                                          uint32_t top_slot) {
+  const uint32_t sh = (uint32_t)(27 - 3 * (int)level) & 31u;
+  slot_put(t, (int)min(dst, top_slot), (c >> sh) & 7u,
+           kLinkTag | ((uint32_t)i << (bits + 1)) | field);
+}
+__device__ __forceinline__ uint32_t left_field(uint32_t back, int bits) {
+  return (1u << bits) - min(back, 1u << bits);
+}
+__device__ __forceinline__ uint32_t right_field(uint32_t ahead, int bits) {
+  return (1u << bits) + min(ahead, (1u << bits) - 1u);
+}
+
+// The slot of the first node with octree nodes from rn up, in global memory.
+__device__ __forceinline__ uint32_t root_slot(uint32_t rn, const OctArgs& a, uint32_t last) {
+  rn = min(rn, last);
+  int c = a.counts[rn];
+  uint32_t next = (uint32_t)a.parent[rn];
+  for (int step = 0; c == 0 && rn != 0u && step < 32; ++step) {
+    rn = min(next, last);
+    c = a.counts[rn];
+    next = (uint32_t)a.parent[rn];
+  }
+  return (uint32_t)a.offsets[rn];
+}
+
+// Node i straight from global memory (the fused build).
 __device__ __forceinline__ void emit_slots(int i, const OctArgs& a, const SlotTags& t, int n_brt,
                                            int n_oct) {
   const uint32_t last = (uint32_t)n_brt - 1u, top_slot = (uint32_t)n_oct - 1u;
-  const uint32_t pn = a.prefix_n[i];
-  const int k = min(a.counts[i], kMaxSteps);
-  const uint32_t par = min((uint32_t)a.parent[i], last);
+  EmitNode e;
+  e.i = i;
+  e.level = a.prefix_n[i] / 3u;
+  e.k = min(a.counts[i], kMaxSteps);
+  const uint32_t par = (uint32_t)a.parent[i];
   const bool ll = a.hll[i] != 0, lr = a.hlr[i] != 0;
-  const bool make = k > 0 && i >= 1, link = ll || lr;
-  int base = 0;
-  uint32_t lc = 0, code = 0;
+  const bool make = e.k > 0 && i >= 1;
+  e.base = 0;
+  uint32_t lc = 0;
   if (make) {
-    base = a.offsets[i];
-    code = a.codes[i];
+    e.base = a.offsets[i];
+    e.code = a.codes[i];
   }
-  if (link) lc = min((uint32_t)a.left_child[i], last);
-  const int L = (int)(pn / 3u);
-  // The first radix node with octree nodes, from the parent (MakeOctNodes, or
-  // the links of a node without any) or the node itself.
-  uint32_t rn = (uint32_t)i;
-  if (make || (link && k == 0 && i != 0)) {
-    rn = par;
-    int c = a.counts[rn];
-    uint32_t next = (uint32_t)a.parent[rn];
-    for (int step = 0; c == 0 && rn != 0u && step < 32; ++step) {
-      rn = min(next, last);
-      c = a.counts[rn];
-      next = (uint32_t)a.parent[rn];
-    }
-  }
+  if (ll || lr) lc = min((uint32_t)a.left_child[i], last);
+  uint32_t up = 0;
+  if (make || ((ll || lr) && e.k == 0 && i != 0)) up = root_slot(par, a, last);
   uint32_t cl = 0, cr = 0;
   if (ll) cl = a.codes[lc];
   if (lr) cr = a.codes[lc + 1u];
-  const int up = (int)min((uint32_t)a.offsets[rn], top_slot);
-  if (make) {
-    // include/shared/oct.h:24-90
-    const uint32_t s16 = (uint32_t)base << 4;
-    for (int j = 0; j < k - 1; ++j) {
-      const uint32_t which = (code >> (30 - 3 * (L - j))) & 7u;
-      const int slot = (int)min((uint32_t)(base + j + 1), top_slot);
-      slot_put(t, slot, which, s16 | (uint32_t)j);
-      slot_mark(t, slot, which);
+  if (make) emit_make(e, up, t, top_slot);
+  const uint32_t dst = make ? (uint32_t)e.base : up;
+  const int bits = link_off_bits(n_brt);
+  if (ll) emit_leaf(i, e.level, dst, cl, left_field((uint32_t)i - lc, bits), bits, t, top_slot);
+  if (lr)
+    emit_leaf(i, e.level, dst, cr, right_field(lc + 1u - (uint32_t)i, bits), bits, t, top_slot);
+}
+
+// A tile of radix nodes in shared memory: a node's parents and leaves lie close
+// to it (98% in its tile), so one round of bulk copies takes the place of four
+// to seven dependent rounds of loads, and what several nodes need is found once.
+constexpr int kEmitThreads = 256;
+constexpr int kEmitTile = 1024;  // nodes: four per thread
+constexpr int kEmitRoom = kEmitTile + 32;
+
+struct EmitSmem {
+  __align__(16) int counts[kEmitRoom];
+  __align__(16) int parent[kEmitRoom];
+  __align__(16) int offsets[kEmitRoom];
+  __align__(16) uint32_t codes[kEmitRoom];
+  __align__(16) int left[kEmitRoom];
+  __align__(16) uint8_t pn[kEmitRoom];
+  __align__(16) uint8_t hll[kEmitRoom];
+  __align__(16) uint8_t hlr[kEmitRoom];
+  unsigned long long bar;
+};
+
+// Brings nodes [lo, lo + n) (n <= kEmitTile, and the code after the last) of a
+// cloud into M. first: the cloud's place in the batch's arrays (`a` is the
+// cloud's view of them), total: entries of those arrays. Copies start at the
+// sixteenth entry at or before the tile, so every array's start is 16-byte
+// aligned when the arrays are; what the arrays' end leaves of the last sixteen,
+// or everything when they are not aligned, comes by plain loads. Returns the
+// tile's place in M; the block has passed a barrier. Thread 0 set M.bar up;
+// phase is the parity of earlier calls. False in ok when the wait ran out (the
+// caller returns).
+__device__ __forceinline__ uint32_t load_emit_tile(EmitSmem& M, const OctArgs& a, uint32_t first,
+                                                   uint32_t lo, uint32_t n, uint32_t total,
+                                                   uint32_t phase, uint32_t* status, bool& ok) {
+  const uint32_t start = first + lo;
+  const uint32_t shift = start & 15u;
+  const uint32_t need = shift + n + 1u;  // entries from start - shift on
+  const uintptr_t any = reinterpret_cast<uintptr_t>(a.counts - first) |
+                        reinterpret_cast<uintptr_t>(a.parent - first) |
+                        reinterpret_cast<uintptr_t>(a.offsets - first) |
+                        reinterpret_cast<uintptr_t>(a.codes - first) |
+                        reinterpret_cast<uintptr_t>(a.left_child - first) |
+                        reinterpret_cast<uintptr_t>(a.prefix_n - first) |
+                        reinterpret_cast<uintptr_t>(a.hll - first) |
+                        reinterpret_cast<uintptr_t>(a.hlr - first);
+  const uint32_t room = total - (start - shift);  // entries to the arrays' end
+  const uint32_t bulk = (any & 15u) ? 0u : min((need + 15u) & ~15u, room & ~15u);
+  const int o = (int)lo - (int)shift;  // the first copied entry, from the cloud's start
+  if (threadIdx.x == 0) {
+    mbar_expect(&M.bar, bulk * 23u);
+    if (bulk) {
+      bulk_load_g2s(M.counts, a.counts + o, bulk * 4u, &M.bar);
+      bulk_load_g2s(M.parent, a.parent + o, bulk * 4u, &M.bar);
+      bulk_load_g2s(M.offsets, a.offsets + o, bulk * 4u, &M.bar);
+      bulk_load_g2s(M.codes, a.codes + o, bulk * 4u, &M.bar);
+      bulk_load_g2s(M.left, a.left_child + o, bulk * 4u, &M.bar);
+      bulk_load_g2s(M.pn, a.prefix_n + o, bulk, &M.bar);
+      bulk_load_g2s(M.hll, a.hll + o, bulk, &M.bar);
+      bulk_load_g2s(M.hlr, a.hlr + o, bulk, &M.bar);
     }
-    const uint32_t which = (code >> (30 - 3 * (L - k + 1))) & 7u;
-    slot_put(t, up, which, s16 | (uint32_t)(k - 1));
-    slot_mark(t, up, which);
   }
-  if (link) {
-    // include/shared/oct.h:92-134, walk ended at radix node 0
-    const int dst = make ? (int)min((uint32_t)base, top_slot) : up;
-    const uint32_t sh = (uint32_t)(27 - 3 * L) & 31u;
-    const int b = link_off_bits(n_brt);
-    const uint32_t mid = 1u << b;
-    const uint32_t key = kLinkTag | ((uint32_t)i << (b + 1));
-    if (ll) slot_put(t, dst, (cl >> sh) & 7u, key | (mid - min((uint32_t)i - lc, mid)));
-    if (lr)
-      slot_put(t, dst, (cr >> sh) & 7u, key | (mid + min(lc + 1u - (uint32_t)i, mid - 1u)));
+  for (uint32_t j = bulk + threadIdx.x; j < min(need, room); j += kEmitThreads) {
+    const int q = o + (int)j;
+    M.counts[j] = a.counts[q];
+    M.parent[j] = a.parent[q];
+    M.offsets[j] = a.offsets[q];
+    M.codes[j] = a.codes[q];
+    M.left[j] = a.left_child[q];
+    M.pn[j] = a.prefix_n[q];
+    M.hll[j] = a.hll[q];
+    M.hlr[j] = a.hlr[q];
+  }
+  __syncthreads();
+  ok = true;
+  for (int tries = 0; tries < 2 && !mbar_try_wait(&M.bar, phase); ++tries) {
+    WaitBound wait(kWaitLimitNs);
+    bool done = false;
+    while (!done && !wait.expired()) done = mbar_try_wait(&M.bar, phase);
+    if (done) break;
+    // give up, but first wait once more for the copies to leave this memory
+    raise_status(status, kStatusSpinTimeout);
+    ok = false;
+  }
+  return shift;
+}
+
+// Every write of the tile's nodes [lo, lo + n), in M from place `shift` on
+// (load_emit_tile). Two rounds: first each node without octree nodes finds the
+// slot of the node above it that has some and keeps it in place of its own
+// prefix, which nobody needs; then every node's links go to its own entry and
+// its MakeOctNodes write to its parent's. At 16.7M uniform points 0.186 ->
+// 0.177 ms against one thread per node on global memory; bound by its L2
+// reductions (0.105 ms without them).
+__device__ __forceinline__ void emit_tile(EmitSmem& M, const OctArgs& a, const SlotTags& t,
+                                          uint32_t lo, uint32_t n, uint32_t shift, int n_brt,
+                                          int n_oct) {
+  const uint32_t last = (uint32_t)n_brt - 1u, top_slot = (uint32_t)n_oct - 1u;
+  const int bits = link_off_bits(n_brt);
+  for (uint32_t j = threadIdx.x; j < n; j += kEmitThreads) {
+    if (M.counts[shift + j] != 0 || lo + j == 0u) continue;
+    uint32_t rn = (uint32_t)M.parent[shift + j], slot = 0;
+    for (int step = 0;; ++step) {
+      const uint32_t u = rn - lo;
+      if (u >= n || step == 32) {
+        slot = root_slot(rn, a, last);
+        break;
+      }
+      if (M.counts[shift + u] != 0 || rn == 0u) {
+        slot = (uint32_t)M.offsets[shift + u];
+        break;
+      }
+      rn = (uint32_t)M.parent[shift + u];
+    }
+    M.offsets[shift + j] = (int)slot;
+  }
+  __syncthreads();
+  for (uint32_t j = threadIdx.x; j < n; j += kEmitThreads) {
+    const uint32_t at = shift + j;
+    EmitNode e;
+    e.i = (int)(lo + j);
+    e.k = min(M.counts[at], kMaxSteps);
+    e.base = M.offsets[at];  // or the slot its links go to
+    e.code = M.codes[at];
+    e.level = M.pn[at] / 3u;
+    if (e.k > 0 && e.i >= 1) {
+      const uint32_t par = (uint32_t)M.parent[at], u = par - lo;
+      emit_make(e, u < n ? (uint32_t)M.offsets[shift + u] : root_slot(par, a, last), t, top_slot);
+    }
+    const uint32_t lc = min((uint32_t)M.left[at], last), v = lc - lo;
+    if (M.hll[at])
+      emit_leaf(e.i, e.level, (uint32_t)e.base, v <= n ? M.codes[shift + v] : a.codes[lc],
+                left_field((uint32_t)e.i - lc, bits), bits, t, top_slot);
+    if (M.hlr[at])
+      emit_leaf(e.i, e.level, (uint32_t)e.base, v < n ? M.codes[shift + v + 1u] : a.codes[lc + 1u],
+                right_field(lc + 1u - (uint32_t)e.i, bits), bits, t, top_slot);
   }
 }
 

@@ -51,7 +51,9 @@ BuildLayout build_layout(int n, int cap) {
   L.ctrl_bytes = L.sort_off + L.sort.zero_bytes;
   L.msd_off = align_up(L.sort_off + L.sort.bytes, 256);
   L.keys_a_off = align_up(L.msd_off + msd_scratch_bytes(), 256);
-  L.keys_b_off = align_up(L.keys_a_off + sizeof(uint32_t) * (size_t)(n > 0 ? n : 1), 256);
+  // (the MSD form's runs start at multiples of four words: a little slack)
+  L.keys_b_off = align_up(
+      L.keys_a_off + sizeof(uint32_t) * ((size_t)(n > 0 ? n : 1) + msd_run_slack()), 256);
   L.tree_off = align_up(L.keys_b_off + sizeof(uint32_t) * (size_t)(n > 0 ? n : 1), 256);
   L.tags_off = align_up(L.tree_off + tree_scratch_bytes(n), 256);
   L.total = align_up(L.tags_off + oct_tags_bytes(cap), 256);
@@ -60,12 +62,13 @@ BuildLayout build_layout(int n, int cap) {
 }
 
 // misc area: [0] status, [1] n_unique, [2] max octree slot, [4..5] sort form
-// flags (MSD, LSD)
+// flags (MSD, LSD), [8..9] the MSD form's item counter and run cursor
 struct Misc {
   uint32_t* status;
   int* unique;
   int* max_slot;
   uint32_t* form;
+  uint32_t* msd;
 };
 Misc misc_at(char* base) {
   Misc m;
@@ -73,6 +76,7 @@ Misc misc_at(char* base) {
   m.unique = reinterpret_cast<int*>(base + 4);
   m.max_slot = reinterpret_cast<int*>(base + 8);
   m.form = reinterpret_cast<uint32_t*>(base + 16);
+  m.msd = reinterpret_cast<uint32_t*>(base + 32);
   return m;
 }
 
@@ -409,14 +413,15 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
                              (size_t)(L.sort.passes - 1) * L.sort.bins;
   const uint32_t* top_base = reinterpret_cast<const uint32_t*>(sort_ctrl + L.sort.base_off) +
                              (size_t)(L.sort.passes - 1) * L.sort.bins;
-  if (msd) OCT_TRY(launch_msd_gate(top_hist, n, m.form, s), "build: sort form");
+  if (msd) OCT_TRY(launch_msd_gate(top_hist, n, m.form, w + L.msd_off, s), "build: sort form");
   uint32_t* sorted = keys_a;
   OCT_TRY(launch_sort_passes_split(keys_a, keys_b, &L.sort, sort_ctrl, m.status,
                                    msd ? m.form : nullptr, msd ? m.form + 1 : nullptr, s, &sorted,
                                    rec),
           "build: sort");
   if (msd) {
-    OCT_TRY(launch_msd_buckets(keys_b, top_base, top_hist, w + L.msd_off, m.form, m.status, s),
+    OCT_TRY(launch_msd_buckets(keys_b, keys_a, top_base, top_hist, w + L.msd_off, m.msd, m.form,
+                               m.status, s),
             "build: msd buckets");
   }
   mark(rec, s);
@@ -424,8 +429,8 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
                                msd ? m.form + 1 : nullptr),
           "build: unique");
   if (msd) {
-    OCT_TRY(launch_msd_pack(keys_b, top_base, n, out->codes, m.unique, w + L.msd_off,
-                            w + L.tree_off, m.form, s),
+    OCT_TRY(launch_msd_pack(keys_a, n, out->codes, m.unique, w + L.msd_off, w + L.tree_off, m.form,
+                            s),
             "build: msd pack");
   }
   mark(rec, s);

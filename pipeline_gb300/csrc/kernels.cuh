@@ -170,18 +170,21 @@ cudaError_t launch_sort_passes_split(uint32_t* keys, uint32_t* alt, const SortPl
 // set runs the MSD kernels, flags[1] set the LSD passes and unique.
 int msd_min_n();
 size_t msd_scratch_bytes();
+size_t msd_run_slack();  // words that the buffer of the runs has beyond the keys'
 bool msd_plan_ok(const SortPlan& p);  // 10-bit digits, 3 passes, reduce-then-scan
-cudaError_t launch_msd_gate(const uint32_t* top_hist, int n, uint32_t* flags, cudaStream_t s);
-// The sorted unique keys of every top-digit bucket over the front of its
-// range; the counts go to the scratch.
-cudaError_t launch_msd_buckets(uint32_t* keys, const uint32_t* top_base, const uint32_t* top_hist,
-                               void* scratch, const uint32_t* gate, uint32_t* status,
-                               cudaStream_t s);
-// Packs the bucket runs: codes, U to *d_unique, the adjacent deltas and tile
+// Chooses the form and cuts the top-digit buckets into items.
+cudaError_t launch_msd_gate(const uint32_t* top_hist, int n, uint32_t* flags, void* scratch,
+                            cudaStream_t s);
+// The sorted unique keys of every item, one run each in `runs`; counters: two
+// zeroed words.
+cudaError_t launch_msd_buckets(const uint32_t* keys, uint32_t* runs, const uint32_t* top_base,
+                               const uint32_t* top_hist, void* scratch, uint32_t* counters,
+                               const uint32_t* gate, uint32_t* status, cudaStream_t s);
+// Packs the runs: codes, U to *d_unique, the adjacent deltas and tile
 // minima into the tree scratch (as launch_unique_deltas leaves them).
-cudaError_t launch_msd_pack(const uint32_t* keys, const uint32_t* top_base, int n,
-                            uint32_t* codes_out, int* d_unique, void* scratch,
-                            void* tree_scratch, const uint32_t* gate, cudaStream_t s);
+cudaError_t launch_msd_pack(const uint32_t* runs, int n, uint32_t* codes_out, int* d_unique,
+                            void* scratch, void* tree_scratch, const uint32_t* gate,
+                            cudaStream_t s);
 
 // ---- unique --------------------------------------------------------------
 struct ScanPlan {

@@ -147,7 +147,7 @@ int oct_morton_encode(const oct_vec4* points, uint32_t* keys, int64_t n, float m
 // ---------------------------------------------------------------- stage 2 --
 size_t oct_sort_workspace_bytes(int n, int key_bits) {
   if (n < 0 || key_bits < 1 || key_bits > 32) return 0;
-  return sort_plan(n, key_bits).bytes;
+  return sort_keys_bytes(n, key_bits);
 }
 
 int oct_sort_keys(uint32_t* keys, uint32_t* keys_alt, int n, int key_bits, void* workspace,
@@ -155,17 +155,9 @@ int oct_sort_keys(uint32_t* keys, uint32_t* keys_alt, int n, int key_bits, void*
   if (n < 0 || n > OCT_MAX_N || key_bits < 1 || key_bits > 32) return OCT_ERR_INVALID_ARG;
   if (n <= 1) return OCT_OK;
   if (!keys || !keys_alt || !workspace || !aligned(workspace, 256)) return OCT_ERR_INVALID_ARG;
-  const SortPlan p = sort_plan(n, key_bits);
-  if (workspace_bytes < p.bytes) return OCT_ERR_WORKSPACE;
-  cudaStream_t s = S(stream);
-  OCT_TRY(cudaMemsetAsync(workspace, 0, p.zero_bytes, s), "oct_sort_keys: clear");
-  OCT_TRY(launch_histogram(keys, &p, workspace, s), "oct_sort_keys: histogram");
-  uint32_t* result = keys;
-  OCT_TRY(launch_sort_passes(keys, keys_alt, &p, workspace, d_status, s, &result),
-          "oct_sort_keys: passes");
-  if (result != keys)
-    OCT_TRY(cudaMemcpyAsync(keys, result, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToDevice, s),
-            "oct_sort_keys: copy back");
+  if (workspace_bytes < sort_keys_bytes(n, key_bits)) return OCT_ERR_WORKSPACE;
+  OCT_TRY(launch_sort_keys(keys, keys_alt, n, key_bits, workspace, d_status, S(stream)),
+          "oct_sort_keys");
   return OCT_OK;
 }
 

@@ -298,6 +298,32 @@ __device__ __forceinline__ float4 decode_corner(uint32_t code, float min_coord, 
   return c;
 }
 
+// Barrier number `phase` (1, 2, ...) of a grid whose CTAs are all resident (a
+// cooperative launch; bar: zeroed arrivals) or, CLUSTER, one cluster with its
+// hardware barrier: all CTAs have passed every earlier phase, and what they
+// wrote is visible to plain loads. False (in every thread) when the wait ran
+// out.
+template <bool CLUSTER>
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t phase, int* s_ok) {
+  if (CLUSTER) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return true;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    red_release_add_u32(bar, 1u);  // after the barrier above: the whole CTA's writes
+    const uint32_t want = phase * gridDim.x;
+    WaitBound wait(kWaitLimitNs);
+    int ok = 1;
+    while (ok && ld_acquire_u32(bar) < want)
+      if (wait.expired()) ok = 0;
+    *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
 // Block-wide exclusive sum of one value per thread (THREADS a multiple of 32).
 template <int THREADS, typename T>
 __device__ __forceinline__ T block_exclusive_sum(T v, T* warp_tot /* THREADS/32 */, T* total) {

@@ -53,8 +53,6 @@ constexpr int kFuBucketBits = 12;
 constexpr int kFuBuckets = 1 << kFuBucketBits;
 constexpr int kFuSpanBits = 30 - kFuBucketBits;    // values of a bucket: a 32 KiB bitmap
 constexpr int kFuTile = 1024;                      // tree and prefix tiles: multiples of this
-constexpr uint32_t kFuBinMost = 48;  // codes in a bin before the radix sort takes over
-constexpr uint32_t kFuBinFew = 12;   // codes in a bin up to which neighbours are compared blindly
 constexpr int kFuMaxGrid = 256;
 constexpr int kFuMaxCluster = 8;                   // the portable cluster size
 constexpr int kFuMinPer = 1024;                    // points per CTA at least
@@ -107,7 +105,8 @@ struct FusedArgs {
 };
 
 struct FusedSort {
-  uint32_t a[kFuCap], b[kFuCap];
+  __align__(16) uint32_t a[kFuCap + kBinPad];
+  __align__(16) uint32_t b[kFuCap + kBinPad];
   uint32_t base[kFuBuckets];       // counts, then the CTA's place in each bucket
   uint32_t start[kFuBuckets + 1];  // first position of each bucket
   RadixSmem<kFuWarps> radix;
@@ -120,34 +119,15 @@ union FusedSmem {
   uint32_t spread[1024];
 };
 
-// All CTAs have passed every earlier phase, and what they wrote is visible.
-// False (in every thread) when the wait ran out. A grid of one cluster uses
-// the cluster's hardware barrier.
+// grid_barrier whose CTAs report a wait that ran out.
 template <bool CLUSTER>
-__device__ __forceinline__ bool grid_barrier(const FusedArgs& A, uint32_t phase, int* s_ok) {
-  if (CLUSTER) {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    return true;
+__device__ __forceinline__ bool fused_barrier(const FusedArgs& A, uint32_t phase, int* s_ok) {
+  const bool ok = grid_barrier<CLUSTER>(A.bar, phase, s_ok);
+  if (!ok && threadIdx.x == 0) {
+    raise_status(A.status, kStatusSpinTimeout);
+    atomicOr(reinterpret_cast<uint32_t*>(A.d_counts) + 3, kStatusSpinTimeout);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    red_release_add_u32(A.bar, 1u);  // after the barrier above: the whole CTA's writes
-    const uint32_t want = phase * gridDim.x;
-    WaitBound wait(kWaitLimitNs);
-    int ok = 1;
-    while (ld_acquire_u32(A.bar) < want) {
-      if (wait.expired()) {
-        raise_status(A.status, kStatusSpinTimeout);
-        atomicOr(reinterpret_cast<uint32_t*>(A.d_counts) + 3, kStatusSpinTimeout);
-        ok = 0;
-        break;
-      }
-    }
-    *s_ok = ok;
-  }
-  __syncthreads();
-  return *s_ok != 0;
+  return ok;
 }
 
 // Heads of the sorted keys a[0, cnt) (first of each run of equal keys) to
@@ -203,136 +183,6 @@ __device__ uint32_t fused_bitmap_bucket(uint32_t* keys, uint32_t cnt, uint32_t* 
   }
   __syncthreads();
   return *total;
-}
-
-// The codes keys[0, cnt) of whole buckets (cnt <= kFuCap; global positions
-// from lo on) sorted in M.a or M.b. Every bucket has as many bins as codes,
-// spread evenly over its values, so the bins follow the cloud's density and
-// hold about one code each: one count, one scan and one scatter bring a code
-// to its bin, where it finds its place by comparing with the others. (At 7,000
-// codes a CTA 18 us by three 8-bit radix passes, 12 us so.) Codes too
-// concentrated for that, more than kFuBinMost in a bin, take the radix sort.
-__device__ __forceinline__ uint32_t* fused_sort(const uint32_t* keys, int cnt, uint32_t lo,
-                                                FusedSort& M, uint32_t* warp_tot, uint32_t* total,
-                                                uint32_t* s_span) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int items = (cnt + kFuThreads - 1) / kFuThreads;
-  auto bin_of = [&](uint32_t k) {
-    const uint32_t b = k >> kFuSpanBits, s = M.start[b], c = M.start[b + 1] - s;
-    return s - lo + (((k & ((1u << kFuSpanBits) - 1u)) * c) >> kFuSpanBits);
-  };
-  uint32_t key[kFuItems], rank2[kFuItems / 2];
-  for (int j = tid; j < items * kFuThreads; j += kFuThreads) M.a[j] = 0u;
-#pragma unroll
-  for (int it = 0; it < kFuItems; ++it) {
-    if (it >= items) break;
-    const int j = it * kFuThreads + tid;
-    key[it] = j < cnt ? keys[j] : 0u;
-  }
-  __syncthreads();
-  uint32_t most = 0;
-#pragma unroll
-  for (int it = 0; it < kFuItems; ++it) {
-    if (it >= items) break;
-    uint32_t r = 0;
-    if (it * kFuThreads + tid < cnt) r = atomicAdd(&M.a[bin_of(key[it])], 1u);
-    most = max(most, r);
-    if (it & 1) rank2[it / 2] |= r << 16;
-    else rank2[it / 2] = r;
-  }
-  most = __reduce_max_sync(kFull, most);
-  if (lane == 0) M.radix.warp_tot[tid >> 5] = most;
-  __syncthreads();
-  most = __reduce_max_sync(kFull, M.radix.warp_tot[lane]);
-  if (most >= kFuBinMost) {
-    uint32_t kmin = 0xffffffffu, kmax = 0;
-#pragma unroll
-    for (int it = 0; it < kFuItems; ++it) {
-      if (it >= items) break;
-      const int j = it * kFuThreads + tid;
-      if (j < cnt) {
-        M.a[j] = key[it];
-        kmin = min(kmin, key[it]);
-        kmax = max(kmax, key[it]);
-      }
-    }
-    if (tid == 0) {
-      s_span[0] = 0xffffffffu;
-      s_span[1] = 0u;
-    }
-    __syncthreads();
-    kmin = __reduce_min_sync(kFull, kmin);
-    kmax = __reduce_max_sync(kFull, kmax);
-    if (lane == 0) {
-      atomicMin(&s_span[0], kmin);
-      atomicMax(&s_span[1], kmax);
-    }
-    __syncthreads();
-    kmin = s_span[0];
-    return smem_radix_sort<kFuWarps, kFuItems>(M.a, M.b, cnt, kmin, 32 - __clz(s_span[1] - kmin),
-                                               M.radix);
-  }
-  // bin counts to bin starts
-  uint32_t sum = 0;
-  for (int k = 0; k < items; ++k) sum += M.a[tid * items + k];
-  uint32_t ex = block_exclusive_sum<kFuThreads>(sum, warp_tot, total);
-  for (int k = 0; k < items; ++k) {
-    const uint32_t c = M.a[tid * items + k];
-    M.a[tid * items + k] = ex;
-    ex += c;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < kFuItems; ++it) {
-    if (it >= items) break;
-    if (it * kFuThreads + tid < cnt)
-      M.b[M.a[bin_of(key[it])] + ((rank2[it / 2] >> (16 * (it & 1))) & 0xffffu)] = key[it];
-  }
-  __syncthreads();
-  // place among the bin's codes (equal ones in the order they lie)
-#pragma unroll
-  for (int it = 0; it < kFuItems; ++it) {
-    if (it >= items) break;
-    const int j = it * kFuThreads + tid;
-    uint32_t place = 0;
-    if (j < cnt && most < kFuBinFew) {
-      // codes of other bins compare the right way round, so the neighbours
-      // within the largest bin's reach are all there is to look at
-      const uint32_t* at = M.b + j;
-      const uint32_t x = at[0];
-      // (reads past either end stay inside M and don't count)
-      const int after = cnt - 1 - j;
-      int p = j;
-#pragma unroll 4
-      for (int d = 1; d <= (int)most; ++d) {
-        p += (int)(at[d] < x) & (int)(d <= after);
-        p -= (int)(at[-d] > x) & (int)(d <= j);
-      }
-      place = (uint32_t)p;
-      key[it] = x;
-    } else if (j < cnt) {
-      const uint32_t x = M.b[j];
-      const uint32_t bin = bin_of(x);
-      const int s = (int)M.a[bin];
-      const int e = (int)bin + 1 < cnt ? (int)M.a[bin + 1] : cnt;
-      place = (uint32_t)s;
-      for (int q = s; q < e; ++q) {
-        const uint32_t y = M.b[q];
-        place += y < x || (y == x && q < j) ? 1u : 0u;
-      }
-      key[it] = x;
-    }
-    if (it & 1) rank2[it / 2] |= place << 16;
-    else rank2[it / 2] = place;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < kFuItems; ++it) {
-    if (it >= items) break;
-    if (it * kFuThreads + tid < cnt) M.a[(rank2[it / 2] >> (16 * (it & 1))) & 0xffffu] = key[it];
-  }
-  __syncthreads();
-  return M.a;
 }
 
 template <bool CLUSTER>
@@ -402,7 +252,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
       }
     }
     const bool any_bad = __syncthreads_or(bad);
-    if (CLUSTER) grid_barrier<CLUSTER>(A, 0, &s_ok);  // the counts are cleared
+    if (CLUSTER) fused_barrier<CLUSTER>(A, 0, &s_ok);  // the counts are cleared
     if (any_bad && tid == 0) raise_status(A.status, kStatusRange);
     // the CTA's place in each bucket
 #pragma unroll
@@ -412,7 +262,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
       if (c) cnt[b] = atomicAdd(A.hist + b, c);
     }
   }
-  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+  if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
 
   // ---- scatter into buckets; this CTA's share of them
   uint32_t lo, hi, cut, share;
@@ -455,7 +305,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
       if (r != 0xffffu) A.keys[M.s.base[code[it] >> kFuSpanBits] + r] = code[it];
     }
   }
-  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+  if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
 
   // ---- sort and unique: [lo, cut) with the straddling bucket [cut, hi), which
   // goes alone by bitmap (a few us whatever it holds) when it is large beside
@@ -466,7 +316,15 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
     const bool big = hi - lo > (uint32_t)kFuCap ||
                      (hi - cut > 2u * (uint32_t)kFuThreads && hi - cut > 2u * share);
     const int cnt = (int)min((big ? cut : hi) - lo, (uint32_t)kFuCap);
-    uint32_t* sorted = fused_sort(A.keys + lo, cnt, lo, M.s, s_warp, &s_total, s_cut);
+    // every bucket has as many bins as codes, spread evenly over its values
+    auto place_of = [&](uint32_t k, uint32_t& into) {
+      const uint32_t b = k >> kFuSpanBits, s = M.s.start[b], c = M.s.start[b + 1] - s;
+      const uint32_t part = k << (32 - kFuSpanBits);
+      into = part * c;
+      return s - lo + __umulhi(part, c);
+    };
+    uint32_t* sorted = smem_bin_sort<kFuWarps, kFuItems>(A.keys + lo, cnt, M.s.a, M.s.b, M.s.radix,
+                                                         s_warp, &s_total, s_cut, place_of);
     uint32_t* other = sorted == M.s.a ? M.s.b : M.s.a;
     u_small = fused_unique(sorted, cnt, other, s_warp, &s_total);
     run = other;
@@ -477,7 +335,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
       A.cta_first[cta] = u_small ? run[0] : u_big ? A.keys[cut] : 0u;
     }
   }
-  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+  if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
 
   // ---- unique codes and deltas to their places
   int n_unique, tile;
@@ -526,7 +384,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
     for (uint32_t k = tid; k < touched; k += kFuThreads)
       if (tmin[k] < kTtAbsent) atomic_min_u8(A.S.tile_min + t_first + k, tmin[k]);
   }
-  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+  if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
 
   // ---- radix tree and edge counts
   const int n_brt = max(n_unique - 1, 0);
@@ -535,7 +393,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
     const TileInfo I{(int)cta, 0, tiles - 1, n_brt, (int)cta * tile, 0};
     tree_nodes_tile(M.tree, SizedTile{tile}, I, A.codes, A.S, A.tree);
   }
-  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+  if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
 
   // ---- prefix sums, octree tags
   if ((int)cta < tiles) {
@@ -547,7 +405,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
                       A.max_slot, tile / kFuThreads);
     if (tid == 0) bulk_wait_all();
   }
-  if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+  if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
 
   // ---- octree
   const int n_oct = n_brt >= 1 ? *A.max_slot + 1 : 0;
@@ -560,7 +418,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
       for (int i = (int)cta * kFuThreads + tid; i < n_brt; i += (int)G * kFuThreads)
         emit_slots(i, A.oct, A.tags, n_brt, n_oct);
     }
-    if (!grid_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+    if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
   }
   if (cta == 0 && tid == kFuThreads - 1) {  // every status bit is up
     A.d_counts[0] = n_unique;

@@ -100,6 +100,7 @@ struct SortConfig {
   int items;       // keys per thread (16 or 24)
   int scan;        // 0: decoupled look-back (OneSweep); 1: tile histograms + tile scan
 };
+constexpr SortConfig kSortConfigDefault = {10, 16, 16, 1};
 
 struct SortPlan {
   int n;
@@ -139,6 +140,13 @@ cudaError_t launch_tile_hist(int radix_bits, const uint32_t* keys, int n, int sh
                              const uint32_t* gate = nullptr);
 void set_sort_config(const SortConfig& c);
 SortConfig get_sort_config();
+
+// The whole sort of n > 1 keys on their key_bits low bits, in place (sort_once.cu;
+// the digit passes for other sort configurations and very large arrays).
+// workspace: sort_keys_bytes(n, key_bits), 256-byte aligned; alt: n words.
+size_t sort_keys_bytes(int n, int key_bits);
+cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits, void* workspace,
+                             uint32_t* status, cudaStream_t s);
 
 // Morton encode; with plan != nullptr also accumulates the plan's digit
 // histograms into the zeroed control block ctrl.

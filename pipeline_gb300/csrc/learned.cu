@@ -719,7 +719,7 @@ OCT_API int oct_lcdf_layout(int max_segments, size_t offsets[12]) {
 OCT_API size_t oct_lcdf_fit_workspace_bytes(int n_sample) {
   using namespace octgb;
   if (n_sample < 1) return 0;
-  return align_up(sort_plan(n_sample, 30).bytes, 256) + 2 * align_up(4 * (size_t)n_sample, 256) +
+  return align_up(sort_keys_bytes(n_sample, 30), 256) + 2 * align_up(4 * (size_t)n_sample, 256) +
          lcdf_moments_bytes();
 }
 
@@ -733,18 +733,15 @@ OCT_API int oct_lcdf_fit(const uint32_t* sample_keys, int n_sample, int n_segmen
     return OCT_ERR_INVALID_ARG;
   if (workspace_bytes < oct_lcdf_fit_workspace_bytes(n_sample)) return OCT_ERR_WORKSPACE;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const SortPlan p = sort_plan(n_sample, 30);
   char* w = static_cast<char*>(workspace);
-  uint32_t* keys = reinterpret_cast<uint32_t*>(w + align_up(p.bytes, 256));
+  uint32_t* keys = reinterpret_cast<uint32_t*>(w + align_up(sort_keys_bytes(n_sample, 30), 256));
   uint32_t* alt = keys + align_up(4 * (size_t)n_sample, 256) / 4;
   cudaError_t e = cudaMemcpyAsync(keys, sample_keys, 4 * (size_t)n_sample, cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(w, 0, p.zero_bytes, s);
-  if (e == cudaSuccess) e = launch_histogram(keys, &p, w, s);
-  uint32_t* sorted = keys;
-  if (e == cudaSuccess) e = launch_sort_passes(keys, alt, &p, w, nullptr, s, &sorted);
+  if (e == cudaSuccess && n_sample > 1)
+    e = launch_sort_keys(keys, alt, n_sample, 30, w, nullptr, s);
   const LcdfLayout L = lcdf_layout(max_segments);
   if (e == cudaSuccess)
-    e = launch_lcdf_fit(sorted, n_sample, n_segments, steps, lr, static_cast<char*>(model), L,
+    e = launch_lcdf_fit(keys, n_sample, n_segments, steps, lr, static_cast<char*>(model), L,
                         n_buckets, alt + align_up(4 * (size_t)n_sample, 256) / 4, s);
   if (e != cudaSuccess) {
     set_last_error(cudaGetErrorString(e));

@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(1024)
 // --------------------------------------------------------------------------
 // Host-side planning and launch.
 // --------------------------------------------------------------------------
-static SortConfig g_default_cfg = {10, 16, 16, 1};
+static SortConfig g_default_cfg = kSortConfigDefault;
 
 void set_sort_config(const SortConfig& c) { g_default_cfg = c; }
 SortConfig get_sort_config() { return g_default_cfg; }
@@ -546,7 +546,7 @@ static bool valid_config(const SortConfig& c) {
 }
 
 SortPlan sort_plan_cfg(int n, int key_bits, SortConfig cfg) {
-  if (!valid_config(cfg)) cfg = SortConfig{10, 16, 16, 1};
+  if (!valid_config(cfg)) cfg = kSortConfigDefault;
   SortPlan p{};
   p.n = n;
   p.cfg = cfg;

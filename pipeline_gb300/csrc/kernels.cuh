@@ -147,6 +147,14 @@ SortConfig get_sort_config();
 size_t sort_keys_bytes(int n, int key_bits);
 cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits, void* workspace,
                              uint32_t* status, cudaStream_t s);
+// The sort of 30-bit keys that runs only where the device flag gate is set;
+// workspace: sort_keys_gated_bytes(n), its first sort_keys_gated_zero_bytes(n)
+// zeroed; *result: keys or alt.
+size_t sort_keys_gated_bytes(int n);
+size_t sort_keys_gated_zero_bytes(int n);
+cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* workspace,
+                                   uint32_t* status, const uint32_t* gate, cudaStream_t s,
+                                   uint32_t** result);
 
 // Morton encode; with plan != nullptr also accumulates the plan's digit
 // histograms into the zeroed control block ctrl.

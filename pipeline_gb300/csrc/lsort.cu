@@ -783,7 +783,6 @@ LsortPlan lsort_plan(int n, int nb, int max_segments) {
   p.n = n;
   p.nb = nb;
   p.L = lcdf_layout(max_segments);
-  p.fallback_sort = sort_plan(n, 30);
   p.fallback_unique = unique_plan(n);
   size_t o = 0;
   auto take = [&](size_t bytes) {
@@ -796,8 +795,8 @@ LsortPlan lsort_plan(int n, int nb, int max_segments) {
   p.stats_off = take(sizeof(LsortStats));
   p.cursor_off = take(4 * (size_t)nb);
   p.uniq_ctrl_off = take(p.fallback_unique.bytes);
-  p.sort_ctrl_off = take(p.fallback_sort.bytes);
-  p.zero_bytes = p.sort_ctrl_off + p.fallback_sort.zero_bytes;
+  p.sort_ctrl_off = take(sort_keys_gated_bytes(n));
+  p.zero_bytes = p.sort_ctrl_off + sort_keys_gated_zero_bytes(n);
   // not zeroed:
   p.starts_off = take(4 * (size_t)(nb + 1));
   p.ucount_off = take(4 * (size_t)nb);
@@ -875,12 +874,9 @@ cudaError_t launch_lsort(const float4* pts, uint32_t* keys, int n, float min_coo
   mark(rec, s);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  // Fallback: OneSweep + unique on the original keys, gated on the flag.
-  char* sc = ws + p.sort_ctrl_off;
-  e = launch_histogram_gated(keys, &p.fallback_sort, sc, gate, s);
-  if (e != cudaSuccess) return e;
+  // Fallback: sort + unique on the original keys, gated on the flag.
   uint32_t* sorted = keys;
-  e = launch_sort_passes_gated(keys, alt, &p.fallback_sort, sc, status, gate, s, &sorted);
+  e = launch_sort_keys_gated(keys, alt, n, ws + p.sort_ctrl_off, status, gate, s, &sorted);
   if (e != cudaSuccess) return e;
   e = launch_unique_gated(sorted, out, n, d_unique, &p.fallback_unique, ws + p.uniq_ctrl_off,
                           status, gate, s);

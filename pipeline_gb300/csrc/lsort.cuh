@@ -24,7 +24,6 @@ static_assert(sizeof(LsortStats) == 48, "LsortStats is 12 words");
 struct LsortPlan {
   int n, nb;
   LcdfLayout L;
-  SortPlan fallback_sort;
   ScanPlan fallback_unique;
   size_t stats_off, sort_ctrl_off, uniq_ctrl_off, zero_bytes;
   size_t cursor_off, starts_off, counts_off, ucount_off, uoff_off, bkeys_off, alt_off, bytes;

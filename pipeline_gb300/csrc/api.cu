@@ -387,38 +387,63 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
   uint32_t* keys_a = reinterpret_cast<uint32_t*>(w + L.keys_a_off);
   uint32_t* keys_b = reinterpret_cast<uint32_t*>(w + L.keys_b_off);
 
-  mark(rec, s);
-  OCT_TRY(cudaMemsetAsync(w, 0, L.ctrl_bytes, s), "build: clear");
-  mark(rec, s);
-  OCT_TRY(launch_morton(reinterpret_cast<const float4*>(points), keys_a, n, min_coord, range,
-                        &L.sort, w + L.sort_off, m.status, s),
-          "build: morton");
-  mark(rec, s);
-  // Stages 2-3: LSD passes + run-head unique, or for large even clouds the
-  // MSD form (top-digit scatter, per-bucket bitmaps, pack), chosen on the
-  // device from the top-digit histogram; both write the sorted unique codes,
-  // U and the deltas of adjacent codes, from which the tree (with the edge
-  // counts) is built.
+  // Stages 2-3: a sort + run-head unique, or for large clouds the MSD form
+  // (top-digit scatter, per-bucket bitmaps, pack), chosen on the device from
+  // the top-digit histogram; both write the sorted unique codes, U and the
+  // deltas of adjacent codes, from which the tree (with the edge counts) is
+  // built. The sort is the one-launch sort where that takes the cloud: without
+  // the digit passes' histograms and, in the MSD form, without eight of their
+  // launches that only return (10M clustered points 612 -> 575 us,
+  // 16.7M uniform 802 -> 785; in place of the passes 2.3M clustered
+  // from a graph 202 -> 200). Timed stage by stage a build keeps the passes.
   const bool msd = n >= msd_min_n() && msd_plan_ok(L.sort);
   char* sort_ctrl = w + L.sort_off;
-  const uint32_t* top_hist = reinterpret_cast<const uint32_t*>(sort_ctrl + L.sort.hist_off) +
-                             (size_t)(L.sort.passes - 1) * L.sort.bins;
-  const uint32_t* top_base = reinterpret_cast<const uint32_t*>(sort_ctrl + L.sort.base_off) +
-                             (size_t)(L.sort.passes - 1) * L.sort.bins;
-  if (msd) OCT_TRY(launch_msd_gate(top_hist, n, m.form, w + L.msd_off, s), "build: sort form");
+  const size_t top_row = (size_t)(L.sort.passes - 1) * L.sort.bins;
+  const uint32_t* top_hist = reinterpret_cast<const uint32_t*>(sort_ctrl + L.sort.hist_off) + top_row;
+  uint32_t* top_base = reinterpret_cast<uint32_t*>(sort_ctrl + L.sort.base_off) + top_row;
+  const uint32_t* lsd_flag = msd ? m.form + 1 : nullptr;
   uint32_t* sorted = keys_a;
-  OCT_TRY(launch_sort_passes_split(keys_a, keys_b, &L.sort, sort_ctrl, m.status,
-                                   msd ? m.form : nullptr, msd ? m.form + 1 : nullptr, s, &sorted,
-                                   rec),
-          "build: sort");
+  bool once = !rec && sort_once_in_plan(L.sort);
+  if (once) {
+    OCT_TRY(cudaMemsetAsync(w, 0, L.ctrl_bytes, s), "build: clear");
+    OCT_TRY(launch_morton(reinterpret_cast<const float4*>(points), keys_a, n, min_coord, range,
+                          msd ? &L.sort : nullptr, sort_ctrl, m.status, s, true),
+            "build: morton");
+    if (msd) {
+      OCT_TRY(launch_msd_gate(top_hist, n, m.form, w + L.msd_off, top_base, s), "build: sort form");
+      OCT_TRY(launch_msd_scatter(keys_a, keys_b, &L.sort, sort_ctrl, m.status, m.form, s),
+              "build: scatter");
+    }
+    const cudaError_t e =
+        launch_sort_once_in_plan(keys_a, keys_b, L.sort, sort_ctrl, m.status, lsd_flag, s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      (void)cudaGetLastError();  // a context with fewer SMs: again with the passes
+      once = false;
+    } else {
+      OCT_TRY(e, "build: sort");
+    }
+  }
+  if (!once) {
+    mark(rec, s);
+    OCT_TRY(cudaMemsetAsync(w, 0, L.ctrl_bytes, s), "build: clear");
+    mark(rec, s);
+    OCT_TRY(launch_morton(reinterpret_cast<const float4*>(points), keys_a, n, min_coord, range,
+                          &L.sort, sort_ctrl, m.status, s),
+            "build: morton");
+    mark(rec, s);
+    if (msd)
+      OCT_TRY(launch_msd_gate(top_hist, n, m.form, w + L.msd_off, nullptr, s), "build: sort form");
+    OCT_TRY(launch_sort_passes_split(keys_a, keys_b, &L.sort, sort_ctrl, m.status,
+                                     msd ? m.form : nullptr, lsd_flag, s, &sorted, rec),
+            "build: sort");
+  }
   if (msd) {
     OCT_TRY(launch_msd_buckets(keys_b, keys_a, top_base, top_hist, w + L.msd_off, m.msd, m.form,
                                m.status, s),
             "build: msd buckets");
   }
   mark(rec, s);
-  OCT_TRY(launch_unique_deltas(sorted, n, out->codes, m.unique, w + L.tree_off, s,
-                               msd ? m.form + 1 : nullptr),
+  OCT_TRY(launch_unique_deltas(sorted, n, out->codes, m.unique, w + L.tree_off, s, lsd_flag),
           "build: unique");
   if (msd) {
     OCT_TRY(launch_msd_pack(keys_a, n, out->codes, m.unique, w + L.msd_off, w + L.tree_off, m.form,

@@ -156,11 +156,19 @@ cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* w
                                    uint32_t* status, const uint32_t* gate, cudaStream_t s,
                                    uint32_t** result);
 
+// Whether build stages 2-3 of this plan run without digit passes: the one-launch
+// sort, whose scratch lies in parts of the plan's that the passes would use.
+bool sort_once_in_plan(const SortPlan& p);
+// That sort: keys in place; gate: nullptr, or a device flag whose 0 returns at
+// once. ctrl: the plan's control block, its zeroed part cleared.
+cudaError_t launch_sort_once_in_plan(uint32_t* keys, uint32_t* alt, const SortPlan& p, void* ctrl,
+                                     uint32_t* status, const uint32_t* gate, cudaStream_t s);
+
 // Morton encode; with plan != nullptr also accumulates the plan's digit
-// histograms into the zeroed control block ctrl.
+// histograms (top_only: its last digit's) into the zeroed control block ctrl.
 cudaError_t launch_morton(const float4* pts, uint32_t* keys, long long n, float min_coord,
                           float range, const SortPlan* plan, void* ctrl, uint32_t* status,
-                          cudaStream_t s);
+                          cudaStream_t s, bool top_only = false);
 cudaError_t launch_histogram(const uint32_t* keys, const SortPlan* plan, void* ctrl,
                              cudaStream_t s);
 cudaError_t launch_sort_passes(uint32_t* keys, uint32_t* alt, const SortPlan* plan, void* ctrl,
@@ -189,8 +197,13 @@ size_t msd_scratch_bytes();
 size_t msd_run_slack();  // words that the buffer of the runs has beyond the keys'
 bool msd_plan_ok(const SortPlan& p);  // 10-bit digits, 3 passes, reduce-then-scan
 // Chooses the form and cuts the top-digit buckets into items.
+// top_base: nullptr, or the buckets' first positions, to be written.
 cudaError_t launch_msd_gate(const uint32_t* top_hist, int n, uint32_t* flags, void* scratch,
-                            cudaStream_t s);
+                            uint32_t* top_base, cudaStream_t s);
+// The top-digit scatter keys -> alt alone (base: written by the gate kernel).
+cudaError_t launch_msd_scatter(const uint32_t* keys, uint32_t* alt, const SortPlan* plan,
+                               void* ctrl, uint32_t* status, const uint32_t* msd_flag,
+                               cudaStream_t s);
 // The sorted unique keys of every item, one run each in `runs`; counters: two
 // zeroed words.
 cudaError_t launch_msd_buckets(const uint32_t* keys, uint32_t* runs, const uint32_t* top_base,

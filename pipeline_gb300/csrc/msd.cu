@@ -97,7 +97,7 @@ static MsdScratch msd_scratch(void* base) {
 
 __global__ void __launch_bounds__(kMsdBuckets)
     msd_gate_kernel(const uint32_t* __restrict__ top_hist, int n, uint32_t* __restrict__ flags,
-                    MsdScratch M) {
+                    MsdScratch M, uint32_t* __restrict__ top_base) {
   chain_enter();
   __shared__ uint32_t s_max[32], warp_tot[32], total;
   __shared__ unsigned long long s_reads[32];
@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(kMsdBuckets)
   const bool is_long = cnt > 2 * mean;
   const uint32_t of_long = block_exclusive_sum<kMsdBuckets>(is_long ? parts : 0u, warp_tot, &total);
   const uint32_t place = is_long ? of_long : total + (id - of_long);
+  if (top_base) top_base[b] = block_exclusive_sum<kMsdBuckets>(cnt, warp_tot, &total);
   if (items <= (uint32_t)kMsdMaxItems)
     for (uint32_t k = 0; k < parts; ++k) {
       M.item[id + k] = (uint32_t)b | k << 10 | (uint32_t)ls << 16;
@@ -482,9 +483,9 @@ __global__ void __launch_bounds__(kPackThreads)
 }
 
 cudaError_t launch_msd_gate(const uint32_t* top_hist, int n, uint32_t* flags, void* scratch,
-                            cudaStream_t s) {
+                            uint32_t* top_base, cudaStream_t s) {
   return launch_chained(msd_gate_kernel, dim3(1), dim3(kMsdBuckets), 0, s, top_hist, n, flags,
-                        msd_scratch(scratch));
+                        msd_scratch(scratch), top_base);
 }
 
 cudaError_t launch_msd_buckets(const uint32_t* keys, uint32_t* runs, const uint32_t* top_base,

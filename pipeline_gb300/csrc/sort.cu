@@ -27,21 +27,20 @@ namespace octgb {
 // --------------------------------------------------------------------------
 // Morton encode, optionally fused with the per-pass digit histograms.
 // --------------------------------------------------------------------------
-template <int RB, bool HIST>
+// HISTS: the plan's passes, or its top digits only (0: none).
+template <int RB, int HISTS>
 __global__ void __launch_bounds__(256)
     morton_kernel(const float4* __restrict__ pts, uint32_t* __restrict__ keys, long long n,
-                  float min_coord, float range, uint32_t* __restrict__ ghist, int passes,
+                  float min_coord, float range, uint32_t* __restrict__ ghist,
                   uint32_t* __restrict__ status) {
   chain_enter();
   constexpr int BINS = 1 << RB;
   constexpr int PASSES = (30 + RB - 1) / RB;  // the plan's passes over 30-bit codes
-  extern __shared__ uint32_t s_hist[];  // [PASSES * BINS] histograms, then the spread table
-  uint32_t* lut = s_hist + (HIST ? PASSES * BINS : 0);
-  if (HIST)
-    for (int i = threadIdx.x; i < PASSES * BINS; i += blockDim.x) s_hist[i] = 0;
+  extern __shared__ uint32_t s_hist[];  // [HISTS * BINS] histograms, then the spread table
+  uint32_t* lut = s_hist + HISTS * BINS;
+  for (int i = threadIdx.x; i < HISTS * BINS; i += blockDim.x) s_hist[i] = 0;
   fill_spread_lut(lut);
   __syncthreads();
-  (void)passes;
   const float scale = __fdiv_rn(1024.0f, range);
   bool bad = false;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -57,11 +56,9 @@ __global__ void __launch_bounds__(256)
       const uint32_t c = morton_code_lut(p[u].x, p[u].y, p[u].z, min_coord, range, scale, lut, ok);
       bad |= !ok;
       keys[i + u * stride] = c;
-      if (HIST) {
 #pragma unroll
-        for (int ps = 0; ps < PASSES; ++ps)
-          atomicAdd(&s_hist[ps * BINS + ((c >> (ps * RB)) & (BINS - 1))], 1u);
-      }
+      for (int h = 0; h < HISTS; ++h)
+        atomicAdd(&s_hist[h * BINS + ((c >> ((PASSES - HISTS + h) * RB)) & (BINS - 1))], 1u);
     }
   }
   for (; i < n; i += stride) {
@@ -70,17 +67,13 @@ __global__ void __launch_bounds__(256)
     const uint32_t c = morton_code_lut(p.x, p.y, p.z, min_coord, range, scale, lut, ok);
     bad |= !ok;
     keys[i] = c;
-    if (HIST) {
 #pragma unroll
-      for (int ps = 0; ps < PASSES; ++ps)
-        atomicAdd(&s_hist[ps * BINS + ((c >> (ps * RB)) & (BINS - 1))], 1u);
-    }
+    for (int h = 0; h < HISTS; ++h)
+      atomicAdd(&s_hist[h * BINS + ((c >> ((PASSES - HISTS + h) * RB)) & (BINS - 1))], 1u);
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) raise_status(status, kStatusRange);
-  if (HIST) {
-    for (int b = threadIdx.x; b < PASSES * BINS; b += blockDim.x)
-      if (s_hist[b]) atomicAdd(&ghist[b], s_hist[b]);
-  }
+  for (int b = threadIdx.x; b < HISTS * BINS; b += blockDim.x)
+    if (s_hist[b]) atomicAdd(&ghist[b], s_hist[b]);
 }
 
 // --------------------------------------------------------------------------
@@ -695,7 +688,7 @@ cudaError_t launch_pass(const SortPlan& p, bool stable, const uint32_t* src, uin
 
 cudaError_t launch_morton(const float4* pts, uint32_t* keys, long long n, float min_coord,
                           float range, const SortPlan* plan, void* ctrl, uint32_t* status,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool top_only) {
   if (n <= 0) return cudaSuccess;
   const int blocks = device_sm_count() * 6;
   long long need = (n + 255) / 256;
@@ -703,15 +696,16 @@ cudaError_t launch_morton(const float4* pts, uint32_t* keys, long long n, float 
   if (plan) {
     if (plan->passes != (30 + plan->radix_bits - 1) / plan->radix_bits) return cudaErrorInvalidValue;
     uint32_t* hist = reinterpret_cast<uint32_t*>(static_cast<char*>(ctrl) + plan->hist_off);
-    const size_t sm = sizeof(uint32_t) * (plan->passes * plan->bins + 1024);
-    if (plan->radix_bits == 10)
-      return launch_chained(morton_kernel<10, true>, dim3(grid), dim3(256), sm, s, pts, keys, n,
-                            min_coord, range, hist, plan->passes, status);
-    return launch_chained(morton_kernel<8, true>, dim3(grid), dim3(256), sm, s, pts, keys, n,
-                          min_coord, range, hist, plan->passes, status);
+    const int hists = top_only ? 1 : plan->passes;
+    hist += (size_t)(plan->passes - hists) * plan->bins;
+    const size_t sm = sizeof(uint32_t) * (hists * plan->bins + 1024);
+    auto kernel = plan->radix_bits == 10 ? (top_only ? morton_kernel<10, 1> : morton_kernel<10, 3>)
+                                         : (top_only ? morton_kernel<8, 1> : morton_kernel<8, 4>);
+    return launch_chained(kernel, dim3(grid), dim3(256), sm, s, pts, keys, n, min_coord, range,
+                          hist, status);
   }
-  return launch_chained(morton_kernel<10, false>, dim3(grid), dim3(256), sizeof(uint32_t) * 1024, s,
-                        pts, keys, n, min_coord, range, nullptr, 0, status);
+  return launch_chained(morton_kernel<10, 0>, dim3(grid), dim3(256), sizeof(uint32_t) * 1024, s,
+                        pts, keys, n, min_coord, range, static_cast<uint32_t*>(nullptr), status);
 }
 
 cudaError_t launch_histogram_gated(const uint32_t* keys, const SortPlan* plan, void* ctrl,
@@ -822,6 +816,23 @@ cudaError_t launch_sort_passes_split(uint32_t* keys, uint32_t* alt, const SortPl
                                      Recorder* rec) {
   return sort_passes_impl(keys, alt, plan, ctrl, status, nullptr, s, result, rec, msd_flag,
                           lsd_flag);
+}
+
+cudaError_t launch_msd_scatter(const uint32_t* keys, uint32_t* alt, const SortPlan* plan,
+                               void* ctrl, uint32_t* status, const uint32_t* msd_flag,
+                               cudaStream_t s) {
+  char* c = static_cast<char*>(ctrl);
+  const int top = plan->passes - 1;
+  DigitAlt alt0;
+  alt0.flag = msd_flag;
+  alt0.shift = top * plan->radix_bits;
+  alt0.base = reinterpret_cast<uint32_t*>(c + plan->base_off) + (size_t)top * plan->bins;
+  alt0.part = reinterpret_cast<uint32_t*>(c + plan->tile_part_off) +
+              (size_t)top * kScanSplits * plan->bins;
+  return launch_pass(*plan, false, keys, alt, alt0.shift, alt0.base, nullptr,
+                     reinterpret_cast<uint32_t*>(c + plan->counter_off),
+                     reinterpret_cast<uint32_t*>(c + plan->tile_hist_off), status, msd_flag, s,
+                     nullptr, 0, alt0);
 }
 
 bool msd_plan_ok(const SortPlan& p) {

@@ -448,12 +448,15 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
     for (uint32_t i = t0 + tid; i < t1; i += kSoThreads) A.keys[i] = src[i];
 }
 
+// zeroed: the first zero_bytes of the layout (cleared here unless `cleared`),
+// rest: what follows them.
 static cudaError_t launch_sort_once(uint32_t* keys, uint32_t* alt, int n, int key_bits,
-                                    int low_bits, void* workspace, uint32_t* status,
+                                    int low_bits, void* zeroed, void* rest, uint32_t* status,
                                     cudaStream_t s, const uint32_t* gate = nullptr,
                                     bool cleared = false) {
   const SoLayout L = so_layout(n);
-  char* w = static_cast<char*>(workspace);
+  char* w = static_cast<char*>(zeroed);
+  char* r = static_cast<char*>(rest) - L.zero_bytes;
   SoArgs A{};
   A.keys = keys;
   A.alt = alt;
@@ -464,8 +467,8 @@ static cudaError_t launch_sort_once(uint32_t* keys, uint32_t* alt, int n, int ke
   A.high = A.bar + 1;
   A.next = A.bar + 2;
   A.hist = reinterpret_cast<uint32_t*>(w + L.hist_off);
-  A.ids = reinterpret_cast<uint32_t*>(w + L.ids_off);
-  A.mat = reinterpret_cast<uint32_t*>(w + L.mat_off);
+  A.ids = reinterpret_cast<uint32_t*>(r + L.ids_off);
+  A.mat = reinterpret_cast<uint32_t*>(r + L.mat_off);
   A.status = status;
   A.gate = gate;
   const int smem = (int)sizeof(SoSmem);
@@ -507,9 +510,9 @@ cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits,
                              uint32_t* status, cudaStream_t s) {
   const SortPlan p = sort_plan(n, key_bits);
   if (sort_once_takes(n, kSoMaxN)) {
-    const cudaError_t e = launch_sort_once(keys, alt, n, key_bits,
-                                           std::min(32, p.passes * p.radix_bits), workspace,
-                                           status, s);
+    const cudaError_t e =
+        launch_sort_once(keys, alt, n, key_bits, std::min(32, p.passes * p.radix_bits), workspace,
+                         static_cast<char*>(workspace) + so_layout(n).zero_bytes, status, s);
     if (e != cudaErrorCooperativeLaunchTooLarge) return e;
     (void)cudaGetLastError();  // a context with fewer SMs: the passes
   }
@@ -528,6 +531,22 @@ cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits,
 // 157).
 constexpr int kSoMaxGated = 1 << 24;
 
+bool sort_once_in_plan(const SortPlan& p) {
+  const SoLayout L = so_layout(p.n);
+  return sort_once_takes(p.n, kSoMaxGated) && msd_plan_ok(p) &&
+         p.zero_bytes - p.tile_part_off >= 2 * align_up(L.zero_bytes, 256) &&
+         p.bytes - p.tile_hist_off >= L.total - L.zero_bytes;
+}
+
+cudaError_t launch_sort_once_in_plan(uint32_t* keys, uint32_t* alt, const SortPlan& p, void* ctrl,
+                                     uint32_t* status, const uint32_t* gate, cudaStream_t s) {
+  // the first digit's split sums (the MSD form's cursors are the last's) and
+  // the tile histograms
+  char* c = static_cast<char*>(ctrl);
+  return launch_sort_once(keys, alt, p.n, 30, 30, c + p.tile_part_off, c + p.tile_hist_off, status,
+                          s, gate, true);
+}
+
 size_t sort_keys_gated_zero_bytes(int n) {
   return std::max(sort_plan(n, 30).zero_bytes, (size_t)256 + 4 * kSoTop);
 }
@@ -542,8 +561,9 @@ cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* w
                                    uint32_t** result) {
   *result = keys;
   if (sort_once_takes(n, kSoMaxGated)) {
-    const cudaError_t e =
-        launch_sort_once(keys, alt, n, 30, 30, workspace, status, s, gate, true);
+    const cudaError_t e = launch_sort_once(
+        keys, alt, n, 30, 30, workspace, static_cast<char*>(workspace) + so_layout(n).zero_bytes,
+        status, s, gate, true);
     if (e != cudaErrorCooperativeLaunchTooLarge) return e;
     (void)cudaGetLastError();
   }

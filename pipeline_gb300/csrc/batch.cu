@@ -69,21 +69,23 @@ struct BatchDev {
   int T4;
   const int4* slot_tiles; // [Tn] {first slot, end slot, cloud, 0}: 256 OctNode slots
   int Tn;
+  const int4* units;      // [Tu] {first, end, cloud, 0}: the bucket sort's
+  int Tu;
 };
 
 // ------------------------------------------------------------------ morton --
-template <int RB>
+// HISTS: digit histograms, the plan's passes or the top digit's only.
+template <int RB, int HISTS>
 __global__ void __launch_bounds__(256)
     batch_morton_kernel(const float4* __restrict__ pts, uint32_t* __restrict__ keys, BatchDev B,
-                        uint32_t* __restrict__ ghist, int passes, uint32_t* __restrict__ status) {
+                        uint32_t* __restrict__ ghist, uint32_t* __restrict__ status) {
   constexpr int BINS = 1 << RB;
   constexpr int PASSES = (30 + RB - 1) / RB;  // the plan's passes over 30-bit codes
-  extern __shared__ uint32_t s_hist[];  // [PASSES * BINS] histograms, then the spread table
-  uint32_t* lut = s_hist + PASSES * BINS;
-  (void)passes;
+  extern __shared__ uint32_t s_hist[];  // [HISTS * BINS] histograms, then the spread table
+  uint32_t* lut = s_hist + HISTS * BINS;
   const int t0 = (int)((long long)B.Ts * blockIdx.x / gridDim.x);
   const int t1 = (int)((long long)B.Ts * (blockIdx.x + 1) / gridDim.x);
-  for (int i = threadIdx.x; i < PASSES * BINS; i += blockDim.x) s_hist[i] = 0;
+  for (int i = threadIdx.x; i < HISTS * BINS; i += blockDim.x) s_hist[i] = 0;
   fill_spread_lut(lut);
   __syncthreads();
   bool bad = false;
@@ -92,8 +94,8 @@ __global__ void __launch_bounds__(256)
     const int4 d = B.sort_tiles[t];
     if (d.z != cur) {  // flush the previous cloud's histograms
       __syncthreads();
-      uint32_t* g = ghist + (size_t)cur * PASSES * BINS;
-      for (int i = threadIdx.x; i < PASSES * BINS; i += blockDim.x) {
+      uint32_t* g = ghist + (size_t)cur * HISTS * BINS;
+      for (int i = threadIdx.x; i < HISTS * BINS; i += blockDim.x) {
         if (s_hist[i]) atomicAdd(&g[i], s_hist[i]);
         s_hist[i] = 0;
       }
@@ -116,8 +118,8 @@ __global__ void __launch_bounds__(256)
         bad |= !ok;
         keys[i + u * blockDim.x] = c;
 #pragma unroll
-        for (int ps = 0; ps < PASSES; ++ps)
-          atomicAdd(&s_hist[ps * BINS + ((c >> (ps * RB)) & (BINS - 1))], 1u);
+        for (int h = 0; h < HISTS; ++h)
+          atomicAdd(&s_hist[h * BINS + ((c >> ((PASSES - HISTS + h) * RB)) & (BINS - 1))], 1u);
       }
     }
     for (; i < d.y; i += blockDim.x) {
@@ -127,14 +129,14 @@ __global__ void __launch_bounds__(256)
       bad |= !ok;
       keys[i] = c;
 #pragma unroll
-      for (int ps = 0; ps < PASSES; ++ps)
-        atomicAdd(&s_hist[ps * BINS + ((c >> (ps * RB)) & (BINS - 1))], 1u);
+      for (int h = 0; h < HISTS; ++h)
+        atomicAdd(&s_hist[h * BINS + ((c >> ((PASSES - HISTS + h) * RB)) & (BINS - 1))], 1u);
     }
   }
   __syncthreads();
   if (cur >= 0) {
-    uint32_t* g = ghist + (size_t)cur * passes * BINS;
-    for (int i = threadIdx.x; i < passes * BINS; i += blockDim.x)
+    uint32_t* g = ghist + (size_t)cur * HISTS * BINS;
+    for (int i = threadIdx.x; i < HISTS * BINS; i += blockDim.x)
       if (s_hist[i]) atomicAdd(&g[i], s_hist[i]);
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) raise_status(status, kStatusRange);
@@ -568,10 +570,12 @@ struct oct_batch_plan {
   bool slots = true;  // slot tags: no cloud above kSlotTagMaxPoints
   octgb::SortPlan sp{};
   std::vector<int> start, node_start, cloud_tile0;
-  std::vector<int4> sort_tiles, tiles4k, slot_tiles;
+  bool buckets = false;  // the bucket sort can stand in for digit passes
+  int largest = 0;       // points of the largest cloud
+  std::vector<int4> sort_tiles, tiles4k, slot_tiles, units;
   // device tables (caller buffer) offsets
   size_t t_start = 0, t_node_start = 0, t_tile0 = 0, t_sort = 0, t_4k = 0, t_slots = 0,
-         tables_bytes = 0;
+         t_units = 0, tables_bytes = 0;
   // workspace offsets
   size_t w_status = 0, w_queue = 0, w_unique = 0, w_maxslot = 0, w_hist = 0,
          zero_bytes = 0, w_tree = 0, w_base = 0, w_th = 0, w_blocks = 0, w_keys_a = 0, w_keys_b = 0,
@@ -623,6 +627,8 @@ octgb::BatchDev dev_view(const oct_batch_plan* P, const void* tables, const floa
   B.T4 = (int)P->tiles4k.size();
   B.slot_tiles = reinterpret_cast<const int4*>(t + P->t_slots);
   B.Tn = (int)P->slot_tiles.size();
+  B.units = reinterpret_cast<const int4*>(t + P->t_units);
+  B.Tu = (int)P->units.size();
   return B;
 }
 
@@ -647,6 +653,7 @@ OCT_API oct_batch_plan* oct_batch_plan_create(int n_clouds, const int32_t* h_siz
       return nullptr;
     }
     P->start[c] = (int)N;
+    P->largest = std::max(P->largest, h_sizes[c]);
     P->node_start[c] = (int)cap;
     P->slots = P->slots && h_sizes[c] <= kSlotTagMaxPoints;
     N += h_sizes[c];
@@ -663,11 +670,17 @@ OCT_API oct_batch_plan* oct_batch_plan_create(int n_clouds, const int32_t* h_siz
   SortConfig cfg = get_sort_config();
   cfg.scan = 1;  // batched passes use per-cloud tile prefixes
   P->sp = sort_plan_cfg(P->N, 30, cfg);
+  const SortConfig d = kSortConfigDefault;
+  P->buckets = cfg.radix_bits == d.radix_bits && cfg.warps == d.warps && cfg.items == d.items;
   const int tile = P->sp.tile;
   P->cloud_tile0.resize(n_clouds + 1);
   for (int c = 0; c < n_clouds; ++c) {
     P->cloud_tile0[c] = (int)P->sort_tiles.size();
     const int f4 = (int)P->tiles4k.size();
+    const int n = h_sizes[c], units = P->buckets ? (n + kBatchUnit - 1) / kBatchUnit : 0;
+    for (int u = 0; u < units; ++u)  // even stretches
+      P->units.push_back(make_int4(P->start[c] + (int)((long long)n * u / units),
+                                   P->start[c] + (int)((long long)n * (u + 1) / units), c, 0));
     for (int lo = P->start[c]; lo < P->start[c + 1]; lo += tile)
       P->sort_tiles.push_back(make_int4(lo, std::min(lo + tile, P->start[c + 1]), c, P->cloud_tile0[c]));
     for (int lo = P->start[c]; lo < P->start[c + 1]; lo += kBatchTile4k)
@@ -676,6 +689,10 @@ OCT_API oct_batch_plan* oct_batch_plan_create(int n_clouds, const int32_t* h_siz
       P->slot_tiles.push_back(make_int4(lo, std::min(lo + kFinThreads, P->node_start[c + 1]), c, 0));
   }
   P->cloud_tile0[n_clouds] = (int)P->sort_tiles.size();
+  // largest clouds first: their large buckets, which take longest, start early
+  std::stable_sort(P->units.begin(), P->units.end(), [&](const int4& x, const int4& y) {
+    return h_sizes[x.z] > h_sizes[y.z];
+  });
   size_t o = 0;
   auto take = [&](size_t b) {
     const size_t at = o;
@@ -688,11 +705,12 @@ OCT_API oct_batch_plan* oct_batch_plan_create(int n_clouds, const int32_t* h_siz
   P->t_sort = take(16 * (P->sort_tiles.size() + 1));
   P->t_4k = take(16 * (P->tiles4k.size() + 1));
   P->t_slots = take(16 * (P->slot_tiles.size() + 1));
+  P->t_units = take(16 * (P->units.size() + 1));
   P->tables_bytes = o;
   const int passes = P->sp.passes, bins = P->sp.bins;
   o = 0;
   P->w_status = take(4);
-  P->w_queue = take(64);  // work-queue counters: prefix sum, emit, finalize
+  P->w_queue = take(64);  // work-queue counters: prefix sum, emit, finalize, bucket sort
   P->w_unique = take(4 * (size_t)n_clouds);
   P->w_maxslot = take(4 * (size_t)n_clouds);
   P->w_hist = take(4 * (size_t)n_clouds * passes * bins);
@@ -741,6 +759,9 @@ OCT_API int oct_batch_upload_tables(const oct_batch_plan* P, void* d_tables, oct
                         cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && !P->slot_tiles.empty())
     e = cudaMemcpyAsync(t + P->t_slots, P->slot_tiles.data(), 16 * P->slot_tiles.size(),
+                        cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && !P->units.empty())
+    e = cudaMemcpyAsync(t + P->t_units, P->units.data(), 16 * P->units.size(),
                         cudaMemcpyHostToDevice, s);
   // the host vectors live in the plan: wait so the copies have read them
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -800,19 +821,33 @@ int batch_build(const oct_batch_plan* P, const void* d_tables, const oct_vec4* p
   }
   if (P->N > 0) {
     const int mgrid = std::max(1, std::min(B.Ts, sms * 16));
-    const size_t msm = 4 * ((size_t)passes * bins + 1024);  // histograms + spread table
+    // Sort: the top digit's scatter and the bucket sort, or stable digit passes
+    // (which count every digit): for other sort configurations, and for large
+    // clouds, whose uneven ones have buckets that a CTA sorts by itself for
+    // long. Whole builds, us, by passes and by buckets: 128 clouds of 3,000
+    // points, even 168 and 130, around 8 centres 173 and 139; 32 of 30,000, 195
+    // and 169, 213 and 196; 256 of 65,536, 1,049 and 985, 1,082 and 1,095; 16 of
+    // a million, 976 and 925, 923 and 1,172. A learned build, which runs this
+    // only when the model does not fit, takes whichever returns sooner (224
+    // frames 982 and 940).
+    constexpr int kBucketMost = 49152;
+    const bool buckets = P->buckets && (lb || P->largest <= kBucketMost);
+    const int hists = buckets ? 1 : passes;
+    const size_t msm = 4 * ((size_t)hists * bins + 1024);  // histograms + spread table
     if (passes != (30 + rb - 1) / rb) return OCT_ERR_INVALID_ARG;
-    if (rb == 10) {
-      batch_morton_kernel<10><<<mgrid, 256, msm, s>>>(reinterpret_cast<const float4*>(points), ka,
-                                                      B, hist, passes, status);
-      batch_hist_scan_kernel<10><<<P->C * passes, 1024, 0, s>>>(hist, base, B, passes);
-    } else {
-      batch_morton_kernel<8><<<mgrid, 256, msm, s>>>(reinterpret_cast<const float4*>(points), ka,
-                                                     B, hist, passes, status);
-      batch_hist_scan_kernel<8><<<P->C * passes, 256, 0, s>>>(hist, base, B, passes);
-    }
-    // the sorted keys land in the buffer the LSD passes end in
-    uint32_t* sorted = (passes & 1) ? kb : ka;
+    const float4* pts4 = reinterpret_cast<const float4*>(points);
+    if (buckets)
+      batch_morton_kernel<10, 1><<<mgrid, 256, msm, s>>>(pts4, ka, B, hist, status);
+    else if (rb == 10)
+      batch_morton_kernel<10, 3><<<mgrid, 256, msm, s>>>(pts4, ka, B, hist, status);
+    else
+      batch_morton_kernel<8, 4><<<mgrid, 256, msm, s>>>(pts4, ka, B, hist, status);
+    if (rb == 10)
+      batch_hist_scan_kernel<10><<<P->C * hists, 1024, 0, s>>>(hist, base, B, hists);
+    else
+      batch_hist_scan_kernel<8><<<P->C * hists, 256, 0, s>>>(hist, base, B, hists);
+    // the sorted keys land in the buffer the passes end in
+    uint32_t* sorted = !buckets && (passes & 1) ? kb : ka;
     if (lb) {
       LbatchArgs la{};
       la.keys = ka;
@@ -830,24 +865,27 @@ int batch_build(const oct_batch_plan* P, const void* d_tables, const oct_vec4* p
       la.stats = reinterpret_cast<LsortStats*>(lb->ws);
       e = launch_lbatch_sort(la, s);
       if (e != cudaSuccess) return batch_fail(e, "batch: learned sort");
-      // The learned result must not land in the passes' input (ka): with an
-      // even pass count `sorted` is ka, so the learned path is offered for
-      // odd pass counts only (host check).
+      // The learned sort reads ka before it writes its result, which it leaves
+      // out when the flag sends the keys in ka through the fallback; an even
+      // number of passes is not offered (host check).
     }
     uint32_t* a = ka;
     uint32_t* b = kb;
-    for (int p = 0; p < passes && e == cudaSuccess; ++p) {
-      const int shift = p * rb;
+    for (int p = 0; p < hists && e == cudaSuccess; ++p) {
+      const int shift = buckets ? (passes - 1) * rb : p * rb;
       e = launch_tile_hist(rb, a, P->N, shift, B.sort_tiles, B.Ts, th, s, fallback);
       if (e != cudaSuccess) break;
       batch_tile_scan_kernel<<<dim3(P->C, (bins + 31) / 32), 32 * kTsGroups, 0, s>>>(
-          th, bins, base, passes, p, B, fallback);
+          th, bins, base, hists, p, B, fallback);
       e = launch_pass(sp, p > 0, a, b, shift, nullptr, nullptr, nullptr, th, status, fallback, s,
                       B.sort_tiles, B.Ts);
       uint32_t* t = a;
       a = b;
       b = t;
     }
+    if (e == cudaSuccess && buckets)
+      e = launch_batch_bucket_sort(kb, ka, B.units, B.Tu, base, B.start,
+                                   reinterpret_cast<uint32_t*>(w + P->w_queue) + 12, fallback, s);
     if (e != cudaSuccess) return batch_fail(e, "batch: sort");
     a = sorted;
     void* tree_ws = w + P->w_tree;

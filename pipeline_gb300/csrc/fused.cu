@@ -109,7 +109,7 @@ struct FusedSort {
   __align__(16) uint32_t b[kFuCap + kBinPad];
   uint32_t base[kFuBuckets];       // counts, then the CTA's place in each bucket
   uint32_t start[kFuBuckets + 1];  // first position of each bucket
-  RadixSmem<kFuWarps> radix;
+  uint32_t aux[kBinAux];
 };
 union FusedSmem {
   FusedSort s;
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
       into = part * c;
       return s - lo + __umulhi(part, c);
     };
-    uint32_t* sorted = smem_bin_sort<kFuWarps, kFuItems>(A.keys + lo, cnt, M.s.a, M.s.b, M.s.radix,
+    uint32_t* sorted = smem_bin_sort<kFuWarps, kFuItems>(A.keys + lo, cnt, M.s.a, M.s.b, M.s.aux,
                                                          s_warp, &s_total, s_cut, place_of);
     uint32_t* other = sorted == M.s.a ? M.s.b : M.s.a;
     u_small = fused_unique(sorted, cnt, other, s_warp, &s_total);

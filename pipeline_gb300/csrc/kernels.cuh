@@ -164,6 +164,13 @@ bool sort_once_in_plan(const SortPlan& p);
 cudaError_t launch_sort_once_in_plan(uint32_t* keys, uint32_t* alt, const SortPlan& p, void* ctrl,
                                      uint32_t* status, const uint32_t* gate, cudaStream_t s);
 
+// The keys of a batch's clouds from their top-digit buckets in src to sorted
+// order in dst (batch_sort.cu).
+constexpr int kBatchUnit = 7168;  // positions of a unit at most
+cudaError_t launch_batch_bucket_sort(const uint32_t* src, uint32_t* dst, const int4* units,
+                                     int n_units, const uint32_t* base, const int* start,
+                                     uint32_t* next, const uint32_t* gate, cudaStream_t s);
+
 // Morton encode; with plan != nullptr also accumulates the plan's digit
 // histograms (top_only: its last digit's) into the zeroed control block ctrl.
 cudaError_t launch_morton(const float4* pts, uint32_t* keys, long long n, float min_coord,

@@ -134,11 +134,22 @@ __device__ uint32_t* smem_radix_sort(uint32_t* a, uint32_t* b, int cnt, uint32_t
   return a;
 }
 
+// First i in [lo, hi) with start[i] >= x, or hi.
+__device__ __forceinline__ int first_at_least(const uint32_t* start, int lo, int hi, uint32_t x) {
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (start[mid] < x) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
 constexpr uint32_t kBinNet = 8;     // keys in a bin up to which the networks of 16 place them
 constexpr uint32_t kBinCut = 32;    // keys in a bin up to which the bins stay as they are
 constexpr uint32_t kBinWarp = 512;  // keys in a bin that a warp sorts
 constexpr uint32_t kBinList = 2048;    // larger bins' list, words
 constexpr uint32_t kBinValues = 2048;  // values counted
+constexpr uint32_t kBinAux = kBinList + kBinValues + 1;  // words of smem_bin_sort's scratch
 constexpr int kBinPad = 16;         // words behind smem_bin_sort's b
 
 // Word j of the binned keys lives at bin_swz(j): threads that read 16
@@ -296,7 +307,7 @@ __device__ __forceinline__ void smem_count_bin(uint32_t* b, uint32_t from, uint3
 // kBinWarp keys by the CTA (then the bin has at most kBinValues values).
 template <int WARPS, int ITEMS>
 __device__ __forceinline__ void smem_sort_bins(uint32_t* k, const uint32_t* start, int cnt,
-                                               bool more, RadixSmem<WARPS>& R, uint32_t* warp_tot,
+                                               bool more, uint32_t* aux, uint32_t* warp_tot,
                                                uint32_t* total, uint32_t* s_span) {
   constexpr int kThreads = WARPS * 32;
   const int tid = threadIdx.x, wid = tid >> 5;
@@ -330,10 +341,9 @@ __device__ __forceinline__ void smem_sort_bins(uint32_t* k, const uint32_t* star
   __syncthreads();
   if (!more) return;
   // the larger bins, listed first: they lie side by side, in few warps' rows
-  uint32_t* list = reinterpret_cast<uint32_t*>(R.whist);  // start | keys << 16
+  uint32_t* list = aux;  // start | keys << 16
   uint32_t* values = list + kBinList;
   static_assert(kThreads * ITEMS / kBinNet <= kBinList, "every larger bin fits");
-  static_assert(sizeof(R.whist) / 4 >= kBinList + kBinValues, "list and values");
   for (int j = tid; j < cnt; j += kThreads) {
     const uint32_t s = start[j], e = j + 1 < cnt ? start[j + 1] : (uint32_t)cnt, m = e - s;
     if (m > kBinWarp) list[kBinList - 1u - atomicAdd(&s_span[1], 1u)] = s | m << 16;
@@ -354,7 +364,7 @@ __device__ __forceinline__ void smem_sort_bins(uint32_t* k, const uint32_t* star
     bool same = true;
     for (uint32_t j = tid; j < m; j += kThreads) same &= k[bin_swz(from + j)] == k[bin_swz(from)];
     if (!__syncthreads_and(same))
-      smem_count_bin<WARPS>(k, from, m, values, R.dstart, warp_tot, total);
+      smem_count_bin<WARPS>(k, from, m, values, values + kBinValues, warp_tot, total);
   }
   __syncthreads();
 }
@@ -366,12 +376,13 @@ __device__ __forceinline__ void smem_sort_bins(uint32_t* k, const uint32_t* star
 // density hold about one each: one count, one scan and one scatter then bring a
 // key to within its bin's size of its place. Where a bin has more than kBinCut
 // keys, every bin is cut into as many as it has keys, and the keys are counted
-// once more: what is large after that is mostly one value. s_span: two words.
+// once more: what is large after that is mostly one value. aux: kBinAux words,
+// s_span: two; the keys may lie in b.
 // (By 1,024 threads 16,384 even keys take 13 us; 22 us with comparisons within
 // the bins and a scan of 16 bins per thread.)
 template <int WARPS, int ITEMS, class PlaceOf>
 __device__ __forceinline__ uint32_t* smem_bin_sort(const uint32_t* keys, int cnt, uint32_t* a,
-                                                   uint32_t* b, RadixSmem<WARPS>& R,
+                                                   uint32_t* b, uint32_t* aux,
                                                    uint32_t* warp_tot, uint32_t* total,
                                                    uint32_t* s_span, PlaceOf place_of) {
   constexpr int kThreads = WARPS * 32;
@@ -431,10 +442,38 @@ __device__ __forceinline__ uint32_t* smem_bin_sort(const uint32_t* keys, int cnt
       dst[bin_swz(at)] = key[it];
     }
   }
-  smem_sort_bins<WARPS, ITEMS>(dst, start, cnt, more, R, warp_tot, total, s_span);
+  smem_sort_bins<WARPS, ITEMS>(dst, start, cnt, more, aux, warp_tot, total, s_span);
   for (int j = tid; j < cnt; j += kThreads) start[j] = dst[bin_swz((uint32_t)j)];
   __syncthreads();
   return start;
+}
+
+// cnt keys written in order from how often each of their values occurs:
+// bins[v], v < values (room a multiple of WARPS * 32, values or more; zero from
+// values on), counts top | v. A warp writes consecutive positions; a position's
+// value is the last that starts at or before it, searched by doubled steps from
+// the lane's last one. All threads call it, behind a barrier.
+template <int WARPS>
+__device__ __forceinline__ void smem_emit_counts(uint32_t* bins, uint32_t values, uint32_t room,
+                                                 uint32_t cnt, uint32_t top, uint32_t* dst,
+                                                 uint32_t* warp_tot, uint32_t* total) {
+  constexpr uint32_t kThreads = WARPS * 32;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  smem_exclusive_rows<WARPS>(bins, (int)(room / kThreads), warp_tot, total);
+  const uint32_t span = ((cnt + kThreads - 1u) / kThreads) * 32u;
+  const uint32_t p0 = (tid >> 5) * span, p1 = min(p0 + span, cnt);
+  uint32_t v = 0;
+  for (uint32_t p = p0 + lane; p < p1; p += 32u) {
+    uint32_t step = 1;
+    while (v + step < values && bins[v + step] <= p) {
+      v += step;
+      step <<= 1;
+    }
+    while (step >>= 1)
+      if (v + step < values && bins[v + step] <= p) v += step;
+    dst[p] = top | v;
+  }
+  __syncthreads();
 }
 
 // Bitmap words [seg0, seg1) of this warp: lanes take consecutive words.

@@ -96,21 +96,11 @@ struct SoSmem {
   uint32_t tab[kSoTop];         // a top bucket's first bucket | log2(buckets) << 16
   RadixSmem<kSoWarps> radix;
 };
+static_assert(sizeof(RadixSmem<kSoWarps>) >= 4 * kBinAux, "the bin sort's scratch");
 static_assert(kSoIds <= 2 * kSoCap && (1 << kSoCountBits) <= 2 * kSoCap, "aliases of ab");
 
-// First i in [lo, hi) with start[i] >= x, or hi.
-__device__ __forceinline__ int so_first(const uint32_t* start, int lo, int hi, uint32_t x) {
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (start[mid] < x) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
 // src[0, cnt), keys of one bucket whose values differ in their low `bits` bits
-// only (bits <= kSoCountBits), sorted to dst: the values counted in bins, the
-// counts scanned, every position's value found by search.
+// only (bits <= kSoCountBits), sorted to dst by counting the values in bins.
 __device__ __forceinline__ void so_count_sort(const uint32_t* src, uint32_t cnt, uint32_t* dst,
                                               int bits, uint32_t* bins, uint32_t* warp_tot,
                                               uint32_t* total) {
@@ -131,23 +121,7 @@ __device__ __forceinline__ void so_count_sort(const uint32_t* src, uint32_t cnt,
     for (int q = 0; q < 4; ++q) warp_count(bins, k[q]);
   }
   __syncthreads();
-  smem_exclusive_rows<kSoWarps>(bins, (int)(room / kSoThreads), warp_tot, total);
-  // a warp writes consecutive positions; a position's value is the last bin
-  // that starts at or before it
-  const uint32_t span = ((cnt + kSoThreads - 1u) / kSoThreads) * 32u;
-  const uint32_t p0 = (uint32_t)(tid >> 5) * span, p1 = min(p0 + span, cnt);
-  uint32_t v = 0;
-  for (uint32_t p = p0 + lane; p < p1; p += 32u) {
-    uint32_t step = 1;  // doubled while the values it passes start at or before p
-    while (v + step < values && bins[v + step] <= p) {
-      v += step;
-      step <<= 1;
-    }
-    while (step >>= 1)
-      if (v + step < values && bins[v + step] <= p) v += step;
-    dst[p] = top | v;
-  }
-  __syncthreads();
+  smem_emit_counts<kSoWarps>(bins, values, room, cnt, top, dst, warp_tot, total);
 }
 
 template <bool CLUSTER>
@@ -334,12 +308,12 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
     for (int turn = 0; (unsigned long long)k * stretch < n; turn ^= 1) {
       if (!one && tid == 0) s_next[turn] = G + atomicAdd(A.next, 1u);
       const uint32_t w0 = k * stretch, w1 = min(w0 + stretch, n);
-      int i = so_first(M.start, 0, ids, w0);
-      const int end = so_first(M.start, i, ids, w1);
+      int i = first_at_least(M.start, 0, ids, w0);
+      const int end = first_at_least(M.start, i, ids, w1);
       while (i < end) {
         const uint32_t lo = M.start[i];
         // as many buckets as fit: all up to the first that starts past the end
-        int e = so_first(M.start, i + 1, end + 1, lo + (uint32_t)kSoCap + 1u) - 1;
+        int e = first_at_least(M.start, i + 1, end + 1, lo + (uint32_t)kSoCap + 1u) - 1;
         e = min(max(e, i + 1), end);
         const uint32_t cnt = M.start[e] - lo;
         if (cnt > (uint32_t)kSoCap) {
@@ -357,7 +331,8 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
           };
           const uint32_t* sorted =
               smem_bin_sort<kSoWarps, kSoItems>(A.alt + lo, (int)cnt, M.ab, M.ab + kSoCap + kBinPad,
-                                                M.radix, s_warp, &s_total, s_span, place_of);
+                                                reinterpret_cast<uint32_t*>(&M.radix), s_warp,
+                                                &s_total, s_span, place_of);
           for (uint32_t j = tid; j < cnt; j += kSoThreads) A.keys[lo + j] = sorted[j];
           __syncthreads();
         }

@@ -242,8 +242,15 @@ __device__ __forceinline__ uint32_t compact3(uint32_t m) {
 // exact), so t = RN(a * scale), scale = RN(1024 / range), stands in for it
 // whenever no integer lies within t * 2^-20 of t: t and RN(a / range) * 1024
 // are each within a relative 2^-23 of a * 1024 / range, so they are within
-// t * 2^-22.3 of each other and have the same floor. Otherwise (near a cell
-// boundary, t < 0, huge, NaN) the division itself decides.
+// t * 2^-22.3 of each other and have the same floor. Near a boundary K the
+// question is whether RN(a / range) reaches b = K / 1024, that is, whether
+// a / range reaches the middle of b and the float below it (h away from b, in
+// units of a; a quotient is never such a middle): the remainder a - b * range,
+// which is exact that close, tells. Otherwise (t < 0, at or past the last cell's
+// end, odd ranges, NaN) the division itself decides. Clouds clamped to their box
+// have every clamped coordinate on a boundary, where the division cost a third
+// to a half of the Morton kernel: 16.7M points around 64 centres 97 -> 70 us,
+// 16.7M even ones 60 -> 60.
 __device__ __forceinline__ uint32_t quantise(float v, float min_coord, float range, float scale,
                                              bool& ok) {
   const float a = __fsub_rn(v, min_coord);
@@ -254,6 +261,15 @@ __device__ __forceinline__ uint32_t quantise(float v, float min_coord, float ran
   if (t >= 0.0f && t < 0x1p22f && f > m && __fsub_rn(1.0f, f) > m) {
     ok = ok && k < 1024.0f;
     return (uint32_t)k;
+  }
+  if (a == 0.0f && t == 0.0f) return 0u;
+  const float near = rintf(t);
+  if (near >= 1.0f && near <= 1024.0f && range >= 0x1p-60f && range <= 0x1p60f) {
+    const float b = __fmul_rn(near, 0x1p-10f);
+    const float below = __uint_as_float(__float_as_uint(b) - 1u);
+    const float h = __fmul_rn(__fmul_rn(__fsub_rn(b, below), 0.5f), range);
+    const float in = __fmaf_rn(-b, range, a) >= -h ? near : near - 1.0f;
+    if (in < 1024.0f) return (uint32_t)in;
   }
   const float q = __fmul_rn(__fdiv_rn(a, range), 1024.0f);
   ok = ok && q >= 0.0f && q <= 1024.0f;

@@ -494,21 +494,27 @@ def host_link_bound(dev, pinned_in, pinned_out, in_bytes: int, out_bytes: int) -
 
 
 def build_launches(n: int = 0) -> int:
-    """Kernel launches of one plain build under the active sort shape:
-    Morton, digit-base scan, per pass (tile histogram + tile scan +) pass,
-    unique (run-head count, their scan, compaction with the deltas), tree
-    nodes, tile-sum scan + prefix sum (which clears the octree tags), octree
-    emit/finalize, counts."""
+    """Kernel launches of one plain build under the active sort shape. Up to
+    12,288 points per SM: one. Otherwise stages 2-3, then tree nodes, tile-sum
+    scan + prefix sum (which clears the octree tags), octree emit/finalize and
+    counts. Stages 2-3: Morton, the one-launch sort and unique (run-head count,
+    their scan, compaction with the deltas), from 2^22 points on with the MSD
+    form beside them (form gate, top-digit scatter, bucket bitmaps, pack scan +
+    pack); for other sort shapes and more than 2^24 points digit passes (base
+    scan, per pass a tile histogram + tile scan and the pass; the first doubles
+    as the top-digit scatter)."""
+    import torch
+
     from pipeline_gb300 import autotune
 
-    rb, _, _, scan = autotune.get_config()
+    rb, warps, items, scan = autotune.get_config()
+    if n and n <= 12288 * torch.cuda.get_device_properties(0).multi_processor_count:
+        return 1
     passes = (30 + rb - 1) // rb
-    lsd = 2 + passes * (3 if scan == 1 else 1) + 3 + 1 + 2 + 2 + 1
-    # MSD form (launched beside the LSD passes for clouds of 2^22+ points; pass
-    # 0's launches double as its top-digit scatter): form gate, bucket
-    # bitmaps, pack scan + pack
-    msd = 4 if (n >= (1 << 22) and rb == 10 and passes == 3 and scan == 1) else 0
-    return lsd + msd
+    once = (rb, warps, items, scan) == (10, 16, 16, 1) and n <= (1 << 24)
+    sort = 1 if once else 1 + passes * (3 if scan == 1 else 1)
+    msd = n >= (1 << 22) and rb == 10 and passes == 3 and scan == 1
+    return 1 + sort + 3 + (4 + once if msd else 0) + 1 + 2 + 2 + 1
 
 
 def profile_only(args):
@@ -550,8 +556,7 @@ def profile_only(args):
         model = LearnedCDF(max_segments=4096).fit(sk, n_segments=4096, steps=0, n_buckets=4096)
         b = LearnedOctreeBuilder(n, model)
     elif args.profile_only == "clustered":
-        # plain build of the clustered cloud of n points (uneven top digits:
-        # stages 2-3 take the LSD form)
+        # plain build of the clustered cloud of n points (uneven top digits)
         from pipeline_gb300 import datasets
 
         pts = torch.from_numpy(datasets.clustered(n, seed=7)).cuda()
@@ -1004,9 +1009,9 @@ TRAFFIC_POINTS = 16777216
 TRAFFIC_KERNELS = {"morton+histogram": ["morton_kernel<10, 1>"],
                    "unique": ["unique_count_kernel", "unique_deltas_kernel"],
                    "radix tree+edge count": ["tree_nodes_kernel"],
-                   "prefix sum": ["tile_sums_scan_kernel", "edge_scan_kernel"],
-                   "octree emit": ["oct_emit_kernel"],
-                   "octree finalize": ["oct_finalize_kernel"]}
+                   "prefix sum": ["tile_sums_scan_kernel", "prefix_slots_kernel"],
+                   "octree emit": ["slot_emit_kernel"],
+                   "octree finalize": ["slot_finalize_kernel"]}
 
 
 def read_traffic(kernel_step: str, n: int):

@@ -280,11 +280,11 @@ OCT_API int oct_build_octree(const oct_vec4* points, int n, float min_coord, flo
                      oct_stream_t stream);
 
 /* Which form stages 2-3 took in the last whole build of n points with this
- * workspace (read back after that build has finished): 0 the LSD radix passes
- * and run-head unique (clouds below 2^22 points; also reported for clouds
- * built by one launch, which sorts its own way), 1 the MSD form (top-digit
- * scatter, per-bucket bitmaps, pack), 2 the LSD form chosen by the device
- * because the top-digit buckets were too uneven. Both give the same bytes. */
+ * workspace (read back after that build has finished): 0 a sort and run-head
+ * unique (clouds below 2^22 points; also reported for clouds built by one
+ * launch, which sorts its own way), 1 the MSD form (top-digit scatter,
+ * per-bucket bitmaps, pack), 2 the form of 0 chosen by the device because the
+ * top-digit buckets were too uneven. Both give the same bytes. */
 #define OCT_SORT_FORM_LSD 0
 #define OCT_SORT_FORM_MSD 1
 #define OCT_SORT_FORM_LSD_FALLBACK 2
@@ -364,7 +364,8 @@ OCT_API int oct_build_octree_learned(const oct_vec4* points, int n, float min_co
                                      void* d_stats, void* workspace, size_t workspace_bytes,
                                      oct_stream_t stream);
 /* Radix sort shape used by sort plans made after the call (the autotuner's
- * knob): radix_bits 10 or 8, warps 16, items 16 or 24, scan 0 (decoupled
+ * knob; shapes other than the default 10, 16, 16, 1 also keep digit passes
+ * where the default takes one-launch and bucket sorts): radix_bits 10 or 8, warps 16, items 16 or 24, scan 0 (decoupled
  * look-back) or 1 (per-tile histograms + tile scan). */
 OCT_API int oct_set_sort_config(int radix_bits, int warps, int items, int scan);
 OCT_API int oct_get_sort_config(int out[4]);

@@ -165,7 +165,7 @@ class BatchOctreeBuilder:
         return True
 
     def learned_stats(self) -> dict:
-        """Learned stage of the last build: fallback (1 if the LSD passes
+        """Learned stage of the last build: fallback (1 if the plain sort
         sorted the batch), the largest bucket, buckets per bucket form."""
         v = self.stats.cpu().tolist()
         return {"fallback": int(v[0]), "max_bucket": int(v[3]), "bitmap_buckets": int(v[7]),

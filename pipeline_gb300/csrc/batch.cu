@@ -827,11 +827,9 @@ int batch_build(const oct_batch_plan* P, const void* d_tables, const oct_vec4* p
     // long. Whole builds, us, by passes and by buckets: 128 clouds of 3,000
     // points, even 168 and 130, around 8 centres 173 and 139; 32 of 30,000, 195
     // and 169, 213 and 196; 256 of 65,536, 1,049 and 985, 1,082 and 1,095; 16 of
-    // a million, 976 and 925, 923 and 1,172. A learned build, which runs this
-    // only when the model does not fit, takes whichever returns sooner (224
-    // frames 982 and 940).
+    // a million, 976 and 925, 923 and 1,172.
     constexpr int kBucketMost = 49152;
-    const bool buckets = P->buckets && (lb || P->largest <= kBucketMost);
+    const bool buckets = P->buckets && P->largest <= kBucketMost;
     const int hists = buckets ? 1 : passes;
     const size_t msm = 4 * ((size_t)hists * bins + 1024);  // histograms + spread table
     if (passes != (30 + rb - 1) / rb) return OCT_ERR_INVALID_ARG;

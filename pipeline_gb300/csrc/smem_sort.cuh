@@ -146,6 +146,8 @@ __device__ __forceinline__ int first_at_least(const uint32_t* start, int lo, int
 
 constexpr uint32_t kBinNet = 8;     // keys in a bin up to which the networks of 16 place them
 constexpr uint32_t kBinCut = 32;    // keys in a bin up to which the bins stay as they are
+constexpr int kBinFewItems = 2;        // keys per thread that compare within their bins
+constexpr uint32_t kBinCompare = 128;  // of at most as many keys
 constexpr uint32_t kBinWarp = 512;  // keys in a bin that a warp sorts
 constexpr uint32_t kBinList = 2048;    // larger bins' list, words
 constexpr uint32_t kBinValues = 2048;  // values counted
@@ -413,6 +415,39 @@ __device__ __forceinline__ uint32_t* smem_bin_sort(const uint32_t* keys, int cnt
   __syncthreads();
   const bool more = s_span[0] != 0u, cut = s_span[0] >= kBinCut;
   smem_exclusive_rows<WARPS>(a, items, warp_tot, total);  // bin counts to bin starts
+  if (items <= kBinFewItems && s_span[0] < kBinCompare) {
+    // few keys: each finds its place by comparing with its bin's others, in
+    // fewer steps than the forms below need whatever the keys
+#pragma unroll
+    for (int it = 0; it < kBinFewItems; ++it)
+      if (it * kThreads + tid < cnt) {
+        uint32_t into;
+        b[a[place_of(key[it], into)] + rank[it]] = key[it];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < kBinFewItems; ++it) {
+      const int j = it * kThreads + tid;
+      if (j >= cnt) break;
+      uint32_t into;
+      const uint32_t x = b[j], bin = place_of(x, into);
+      const int s = (int)a[bin], e = (int)bin + 1 < cnt ? (int)a[bin + 1] : cnt;
+      uint32_t place = (uint32_t)s;
+#pragma unroll 4
+      for (int q = s; q < e; ++q) {
+        const uint32_t y = b[q];
+        place += y < x || (y == x && q < j) ? 1u : 0u;
+      }
+      key[it] = x;
+      rank[it] = place;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < kBinFewItems; ++it)
+      if (it * kThreads + tid < cnt) a[rank[it]] = key[it];
+    __syncthreads();
+    return a;
+  }
   if (cut) {
     for (int j = tid; j < items * kThreads; j += kThreads) b[j] = 0u;
     __syncthreads();

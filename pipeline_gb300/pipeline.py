@@ -87,8 +87,8 @@ class OctreeBuilder:
         self._last_n = n
 
     def sort_form(self) -> int:
-        """Form of stages 2-3 in the last build (synchronises): 0 LSD passes,
-        1 MSD form, 2 LSD chosen by the device for an uneven cloud."""
+        """Form of stages 2-3 in the last build (synchronises): 0 sort and unique,
+        1 MSD form, 2 sort and unique chosen by the device for an uneven cloud."""
         torch.cuda.synchronize(self.device)
         f = C.c_int(-1)
         _lib.check(self.lib.oct_build_sort_form(C.c_void_p(self.workspace.data_ptr()),

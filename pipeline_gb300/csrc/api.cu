@@ -80,7 +80,7 @@ Misc misc_at(char* base) {
   return m;
 }
 
-__global__ void node_count_init_kernel(const int* ps, int n, int* out) { *out = ps[n - 1]; }
+__global__ void node_count_init_kernel(const int* ps, int n, int* out) { *out = ps[n - 1] + 1; }
 
 __global__ void node_count_kernel(const int* __restrict__ ec, const int* __restrict__ ps, int n,
                                   int* out) {
@@ -88,10 +88,8 @@ __global__ void node_count_kernel(const int* __restrict__ ec, const int* __restr
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     if (i > 0 && ec[i] > 0) mx = max(mx, ps[i] + ec[i] - 1);
   for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0 && mx > 0) atomicMax(out, mx);
+  if ((threadIdx.x & 31) == 0 && mx > 0) atomicMax(out, mx + 1);
 }
-
-__global__ void plus_one_kernel(int* v) { *v += 1; }
 
 __global__ void root_init_kernel(oct_node* nodes, const uint32_t* codes, const uint8_t* prefix_n,
                                  float min_coord, float range) {
@@ -260,7 +258,6 @@ int oct_octree_node_count(const int32_t* edge_count, const int32_t* prefix_sum, 
   int grid = (n_nodes + 255) / 256;
   if (grid > device_sm_count() * 8) grid = device_sm_count() * 8;
   node_count_kernel<<<grid, 256, 0, s>>>(edge_count, prefix_sum, n_nodes, d_n_oct_nodes);
-  plus_one_kernel<<<1, 1, 0, s>>>(d_n_oct_nodes);
   OCT_TRY(cudaGetLastError(), "oct_octree_node_count");
   return OCT_OK;
 }

@@ -51,7 +51,9 @@ constexpr int kSoStretch = 14336; // positions whose buckets are sorted together
 constexpr int kSoMinPer = 1024;   // keys per CTA at least
 // Larger arrays take the launched passes: uneven keys would lose (codes around
 // 64 centres 16.7M: 388 us by passes, 445 here) although even ones would not
-// (412 and 310). The line also bounds the loss of the digit passes in here where
+// (412 and 310). At the line codes break even (231 and 224 to 230; passed as
+// 32-bit keys, which leaves three quarters of the buckets empty, 228 and 236)
+// and even keys gain a third. The line also bounds the loss of the digit passes in here where
 // most of a large array is a few values: nine tenths one value 167 and 165 us at
 // 4.2M, 237 and 283 at 8.4M.
 constexpr int kSoMaxN = 1 << 23;

@@ -696,11 +696,13 @@ cudaError_t launch_morton(const float4* pts, uint32_t* keys, long long n, float 
   if (plan) {
     if (plan->passes != (30 + plan->radix_bits - 1) / plan->radix_bits) return cudaErrorInvalidValue;
     uint32_t* hist = reinterpret_cast<uint32_t*>(static_cast<char*>(ctrl) + plan->hist_off);
+    if (top_only && plan->radix_bits != 10) return cudaErrorInvalidValue;
     const int hists = top_only ? 1 : plan->passes;
     hist += (size_t)(plan->passes - hists) * plan->bins;
     const size_t sm = sizeof(uint32_t) * (hists * plan->bins + 1024);
-    auto kernel = plan->radix_bits == 10 ? (top_only ? morton_kernel<10, 1> : morton_kernel<10, 3>)
-                                         : (top_only ? morton_kernel<8, 1> : morton_kernel<8, 4>);
+    auto kernel = plan->radix_bits != 10 ? morton_kernel<8, 4>
+                  : top_only             ? morton_kernel<10, 1>
+                                         : morton_kernel<10, 3>;
     return launch_chained(kernel, dim3(grid), dim3(256), sm, s, pts, keys, n, min_coord, range,
                           hist, status);
   }

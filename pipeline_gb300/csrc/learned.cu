@@ -356,7 +356,7 @@ constexpr int kTrThreads = 512;
 constexpr int kTrWarps = kTrThreads / 32;
 constexpr int kTrCtas = kLcdfMaxSegments / kTrThreads;
 // The fixed point covers heights from 2^-32 to 2^16, i.e. theta above -22;
-// theta moves by about lr a step, so fits with steps * |lr| above this take
+// theta moves by about lr a step, so fits with steps * lr above this take
 // three launches a step instead.
 constexpr float kTrMost = 16.f;
 static_assert(kTrCtas <= 8, "a portable cluster");
@@ -644,7 +644,8 @@ cudaError_t launch_lcdf_fit(const uint32_t* sorted_sample, int S, int k_req, int
   if (grid > device_sm_count() * 4) grid = device_sm_count() * 4;
   if (grid < 1) grid = 1;
   set_smem_limit(lcdf_fwd_bwd_kernel, 12 * (kLcdfMaxSegments + 1));
-  if (steps > 0 && (float)steps * fabsf(lr) <= kTrMost) {
+  // (a rate that is not positive moves nothing, as in the stepwise kernels)
+  if (steps > 0 && lr > 0.f && (float)steps * lr <= kTrMost) {
     const LcdfMoments M = lcdf_moments_carve(moments);
     lcdf_moments_kernel<<<(k_req + 7) / 8, 256, 0, s>>>(sorted_sample, S, blob, L, M);
     cudaLaunchConfig_t c = {};
@@ -658,7 +659,7 @@ cudaError_t launch_lcdf_fit(const uint32_t* sorted_sample, int S, int k_req, int
     c.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&c, lcdf_train_kernel, blob, L, M, S, steps, lr);
     if (e != cudaSuccess) return e;
-  } else {  // heights could leave the fixed point's range
+  } else {  // heights could leave the fixed point's range, or nothing moves
     const cudaError_t e = launch_lcdf_train(sorted_sample, S, steps, lr, blob, L, s);
     if (e != cudaSuccess) return e;
   }

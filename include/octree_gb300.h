@@ -462,15 +462,25 @@ OCT_API int oct_check_tree(const oct_node* nodes, int n_nodes, const uint32_t* c
 /* publishes (the workspace is cleared first), with the bound limit_ns (at   */
 /* most 1 s), so a caller can check that it returns within that time with   */
 /* the bit set. which: OCT_DIAG_WAIT_SORT (the sort's per-digit look-back)   */
-/* or OCT_DIAG_WAIT_SCAN (the warp look-back of unique and prefix sum).      */
+/* or OCT_DIAG_WAIT_SCAN (the warp look-back of unique and prefix sum), or   */
+/* OCT_DIAG_WAIT_GRID: the grid barrier of the one-launch sort, which waits   */
+/* for a block that does not exist.                                           */
 /* workspace: DEVICE, 256-byte aligned, oct_diag_wait_workspace_bytes().     */
 /* ----------------------------------------------------------------------- */
 #define OCT_DIAG_WAIT_SORT 0
 #define OCT_DIAG_WAIT_SCAN 1
+#define OCT_DIAG_WAIT_GRID 2
 OCT_API size_t oct_diag_wait_workspace_bytes(void);
 OCT_API int oct_diag_lookback_timeout(int which, unsigned long long limit_ns, void* workspace,
                                       size_t workspace_bytes, uint32_t* d_status,
                                       oct_stream_t stream);
+/* The same for the one-launch build (oct_build_octree, same arguments): its
+ * barriers wait for a block that does not exist, so d_counts reads 0, 0, 0 and
+ * OCT_STATUS_SPIN_TIMEOUT afterwards. OCT_ERR_INVALID_ARG for a cloud that is not
+ * built in one launch, or by at most eight blocks (whose barrier is hardware). */
+OCT_API int oct_diag_build_timeout(const oct_vec4* points, int n, float min_coord, float range,
+                                   const oct_build_outputs* out, unsigned long long limit_ns,
+                                   void* workspace, size_t workspace_bytes, oct_stream_t stream);
 
 #ifdef __cplusplus
 } /* extern "C" */

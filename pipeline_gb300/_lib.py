@@ -30,6 +30,7 @@ OCT_MAX_N = (1 << 30) - 1
 
 OCT_DIAG_WAIT_SORT = 0
 OCT_DIAG_WAIT_SCAN = 1
+OCT_DIAG_WAIT_GRID = 2
 
 _STATUS_NAMES = {
     OCT_ERR_INVALID_ARG: "invalid argument",
@@ -132,6 +133,7 @@ SIGNATURES = {
     "oct_build_step_name": (C.c_char_p, [I]),
     "oct_build_octree_timed": (I, [P, I, F, F, C.POINTER(OctBuildOutputs), P, Z, P, I, P]),
     "oct_diag_wait_workspace_bytes": (Z, []),
+    "oct_diag_build_timeout": (I, [P, I, F, F, C.POINTER(OctBuildOutputs), C.c_ulonglong, P, Z, P]),
     "oct_diag_lookback_timeout": (I, [I, C.c_ulonglong, P, Z, P, P]),
 }
 

@@ -339,7 +339,7 @@ size_t oct_build_workspace_bytes(int n, int nodes_capacity) {
 
 static int build_impl(const oct_vec4* points, int n, float min_coord, float range,
                       const oct_build_outputs* out, void* workspace, size_t workspace_bytes,
-                      oct_stream_t stream, Recorder* rec) {
+                      oct_stream_t stream, Recorder* rec, const GridBarrier* bar = nullptr) {
   if (n < 0 || n > OCT_MAX_N || !out || !out->d_counts) return OCT_ERR_INVALID_ARG;
   if (out->nodes_capacity > 0 && n > OCT_MAX_OCTREE_NODES + 1) return OCT_ERR_TOO_LARGE;
   cudaStream_t s = S(stream);
@@ -373,7 +373,7 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
   if (!rec && n <= fused_max_points()) {
     const cudaError_t e = launch_fused_build(reinterpret_cast<const float4*>(points), n, min_coord,
                                              range, out->codes, a, out->edge_count,
-                                             out->prefix_sum, out->d_counts, w, s);
+                                             out->prefix_sum, out->d_counts, w, s, bar);
     if (e != cudaErrorCooperativeLaunchTooLarge) {
       OCT_TRY(e, "build: fused");
       return OCT_OK;
@@ -525,19 +525,35 @@ int oct_build_octree_timed(const oct_vec4* points, int n, float min_coord, float
   return rc;
 }
 
+static const size_t kDiagWords = 2 * 1024 * sizeof(uint32_t);  // of the look-back waits
+size_t oct_diag_wait_workspace_bytes(void) { return std::max(kDiagWords, diag_grid_wait_bytes()); }
 
-
-size_t oct_diag_wait_workspace_bytes(void) { return 2 * 1024 * sizeof(uint32_t); }
+int oct_diag_build_timeout(const oct_vec4* points, int n, float min_coord, float range,
+                           const oct_build_outputs* out, unsigned long long limit_ns,
+                           void* workspace, size_t workspace_bytes, oct_stream_t stream) {
+  if (limit_ns == 0 || limit_ns > kWaitLimitNs || n < 1 || n > fused_max_points() ||
+      fused_is_cluster(n))
+    return OCT_ERR_INVALID_ARG;
+  const GridBarrier bar{nullptr, 1u, limit_ns};
+  return build_impl(points, n, min_coord, range, out, workspace, workspace_bytes, stream, nullptr,
+                    &bar);
+}
 
 int oct_diag_lookback_timeout(int which, unsigned long long limit_ns, void* workspace,
                               size_t workspace_bytes, uint32_t* d_status, oct_stream_t stream) {
-  if ((which != OCT_DIAG_WAIT_SORT && which != OCT_DIAG_WAIT_SCAN) || limit_ns == 0 ||
+  if ((which != OCT_DIAG_WAIT_SORT && which != OCT_DIAG_WAIT_SCAN && which != OCT_DIAG_WAIT_GRID) ||
+      limit_ns == 0 ||
       limit_ns > kWaitLimitNs || !workspace || !aligned(workspace, 256) || !d_status)
     return OCT_ERR_INVALID_ARG;
-  if (workspace_bytes < oct_diag_wait_workspace_bytes()) return OCT_ERR_WORKSPACE;
+  if (workspace_bytes < (which == OCT_DIAG_WAIT_GRID ? diag_grid_wait_bytes() : kDiagWords))
+    return OCT_ERR_WORKSPACE;
   cudaStream_t s = S(stream);
+  if (which == OCT_DIAG_WAIT_GRID) {
+    OCT_TRY(launch_diag_grid_wait(workspace, d_status, limit_ns, s), "oct_diag_lookback_timeout");
+    return OCT_OK;
+  }
   // Every look-back word starts unpublished; nothing publishes tile 0.
-  OCT_TRY(cudaMemsetAsync(workspace, 0, oct_diag_wait_workspace_bytes(), s), "oct_diag: clear");
+  OCT_TRY(cudaMemsetAsync(workspace, 0, kDiagWords, s), "oct_diag: clear");
   if (which == OCT_DIAG_WAIT_SORT)
     OCT_TRY(launch_diag_sort_wait(static_cast<uint32_t*>(workspace), d_status, limit_ns, s),
             "oct_diag_lookback_timeout");

@@ -315,12 +315,16 @@ __device__ __forceinline__ float4 decode_corner(uint32_t code, float min_coord, 
 }
 
 // Barrier number `phase` (1, 2, ...) of a grid whose CTAs are all resident (a
-// cooperative launch; bar: zeroed arrivals) or, CLUSTER, one cluster with its
-// hardware barrier: all CTAs have passed every earlier phase, and what they
-// wrote is visible to plain loads. False (in every thread) when the wait ran
-// out.
+// cooperative launch) or, CLUSTER, one cluster with its hardware barrier: all
+// CTAs have passed every earlier phase, and what they wrote is visible to plain
+// loads. False (in every thread) when the wait ran out.
+struct GridBarrier {
+  uint32_t* arrivals;  // zeroed
+  uint32_t absent;     // arrivals waited for beyond the grid's: 0, or 1 for a wait that runs out
+  unsigned long long limit_ns;
+};
 template <bool CLUSTER>
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t phase, int* s_ok) {
+__device__ __forceinline__ bool grid_barrier(const GridBarrier& b, uint32_t phase, int* s_ok) {
   if (CLUSTER) {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -328,11 +332,11 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t phase, int*
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    red_release_add_u32(bar, 1u);  // after the barrier above: the whole CTA's writes
-    const uint32_t want = phase * gridDim.x;
-    WaitBound wait(kWaitLimitNs);
+    red_release_add_u32(b.arrivals, 1u);  // after the barrier above: the whole CTA's writes
+    const uint32_t want = phase * gridDim.x + b.absent;
+    WaitBound wait(b.limit_ns);
     int ok = 1;
-    while (ok && ld_acquire_u32(bar) < want)
+    while (ok && ld_acquire_u32(b.arrivals) < want)
       if (wait.expired()) ok = 0;
     *s_ok = ok;
   }

@@ -88,7 +88,7 @@ struct FusedArgs {
   const float4* pts;
   int n;
   float min_coord, range;
-  uint32_t* bar;     // grid barrier arrivals
+  GridBarrier bar;
   uint32_t* hist;    // [kFuBuckets] zeroed
   uint32_t* status;
   int* max_slot;
@@ -119,7 +119,9 @@ union FusedSmem {
   uint32_t spread[1024];
 };
 
-// grid_barrier whose CTAs report a wait that ran out.
+// grid_barrier whose CTAs report a wait that ran out, in counts that CTA 0
+// cleared when it started. (Should it get there only after others gave up at the
+// first barrier, it waits for them in vain at the second and reports it itself.)
 template <bool CLUSTER>
 __device__ __forceinline__ bool fused_barrier(const FusedArgs& A, uint32_t phase, int* s_ok) {
   const bool ok = grid_barrier<CLUSTER>(A.bar, phase, s_ok);
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
   uint32_t phase = 0;
 
   // ---- codes and bucket counts
+  if (cta == 0 && tid < 4) A.d_counts[tid] = 0;
   const int per = (int)(((uint32_t)A.n + G - 1u) / G);
   const int t0 = (int)min((long long)cta * per, (long long)A.n), t1 = min(t0 + per, A.n);
   uint32_t code[kFuItems];
@@ -424,7 +427,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
     A.d_counts[0] = n_unique;
     A.d_counts[1] = n_brt;
     A.d_counts[2] = n_oct;
-    A.d_counts[3] = (int)*reinterpret_cast<volatile uint32_t*>(A.status);
+    atomicOr(A.d_counts + 3, (int)*reinterpret_cast<volatile uint32_t*>(A.status));
   }
   if (octree) {
     if (fits && n_brt >= 1) {
@@ -442,22 +445,29 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
 
 size_t fused_workspace_bytes(int n, int cap) { return fused_layout(n, cap).total; }
 
+static int fused_grid(int n) {
+  return std::max(1, std::min((n + kFuMinPer - 1) / kFuMinPer,
+                              std::min(device_sm_count(), kFuMaxGrid)));
+}
+bool fused_is_cluster(int n) { return fused_grid(n) <= kFuMaxCluster; }
+
 int fused_max_points() { return device_sm_count() * kFuShare; }
 
 cudaError_t launch_fused_build(const float4* pts, int n, float min_coord, float range,
                                uint32_t* codes, const OctArgs& oct, int* ec, int* ps,
-                               int* d_counts, void* workspace, cudaStream_t s) {
+                               int* d_counts, void* workspace, cudaStream_t s,
+                               const GridBarrier* bar) {
   const FusedLayout L = fused_layout(n, oct.cap);
   char* w = static_cast<char*>(workspace);
-  const int grid = std::max(1, std::min((n + kFuMinPer - 1) / kFuMinPer,
-                                        std::min(device_sm_count(), kFuMaxGrid)));
+  const int grid = fused_grid(n);
   FusedArgs A{};
   A.pts = pts;
   A.n = n;
   A.min_coord = min_coord;
   A.range = range;
   A.status = reinterpret_cast<uint32_t*>(w + L.misc_off);
-  A.bar = A.status + 1;
+  A.bar = bar ? *bar : GridBarrier{nullptr, 0u, kWaitLimitNs};
+  A.bar.arrivals = A.status + 1;
   A.max_slot = reinterpret_cast<int*>(A.status + 2);
   A.hist = reinterpret_cast<uint32_t*>(w + L.hist_off);
   A.cta_count = reinterpret_cast<uint32_t*>(w + L.cta_off);
@@ -476,7 +486,7 @@ cudaError_t launch_fused_build(const float4* pts, int n, float min_coord, float 
   A.tags = slot_tags(oct_tags_carve(w + L.tags_off, oct.cap), 0, oct.cap);
   A.d_counts = d_counts;
   const int smem = (int)sizeof(FusedSmem);
-  const bool cluster = grid <= kFuMaxCluster;
+  const bool cluster = fused_is_cluster(n);
   auto kernel = cluster ? fused_build_kernel<true> : fused_build_kernel<false>;
   cudaError_t e = set_smem_limit(kernel, smem);
   if (e != cudaSuccess) return e;

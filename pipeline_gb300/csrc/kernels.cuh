@@ -89,6 +89,10 @@ void set_last_error(const char* msg);
 // look-back over 2 words), bounded by limit_ns.
 cudaError_t launch_diag_sort_wait(uint32_t* lookback, uint32_t* status,
                                   unsigned long long limit_ns, cudaStream_t s);
+// One sort_once launch whose grid barrier waits for a CTA that does not exist.
+size_t diag_grid_wait_bytes();
+cudaError_t launch_diag_grid_wait(void* workspace, uint32_t* status, unsigned long long limit_ns,
+                                  cudaStream_t s);
 cudaError_t launch_diag_scan_wait(unsigned long long* lb, uint32_t* status,
                                   unsigned long long limit_ns, cudaStream_t s);
 
@@ -420,11 +424,15 @@ cudaError_t launch_prefix_sum_clear_tags(int n_host, const int* d_unique, int* e
 // The whole build of a cloud of at most fused_max_points() points in one
 // cooperative launch (fused.cu). oct holds the tree's output arrays as well.
 // cudaErrorCooperativeLaunchTooLarge: the grid does not fit this context.
+// bar: nullptr, or another bound and number of arrivals (a diagnosis; it has
+// nothing to act on in a build of one cluster).
 int fused_max_points();
+bool fused_is_cluster(int n);
 size_t fused_workspace_bytes(int n, int cap);
 cudaError_t launch_fused_build(const float4* pts, int n, float min_coord, float range,
                                uint32_t* codes, const OctArgs& oct, int* ec, int* ps,
-                               int* d_counts, void* workspace, cudaStream_t s);
+                               int* d_counts, void* workspace, cudaStream_t s,
+                               const GridBarrier* bar = nullptr);
 
 // Copies U, B, M, status into out[4] (device).
 cudaError_t launch_publish_counts(const int* d_unique, const int* d_max_slot,

@@ -81,7 +81,7 @@ struct SoArgs {
   int n;
   int key_bits;  // the keys' significant bits
   int low_bits;  // bits that order the keys, should some have more
-  uint32_t* bar;   // grid barrier arrivals
+  GridBarrier bar;
   uint32_t* high;  // keys have bits above key_bits
   uint32_t* next;  // stretches taken, beyond one per CTA
   uint32_t* hist;  // [kSoTop] zeroed
@@ -430,7 +430,8 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
 static cudaError_t launch_sort_once(uint32_t* keys, uint32_t* alt, int n, int key_bits,
                                     int low_bits, void* zeroed, void* rest, uint32_t* status,
                                     cudaStream_t s, const uint32_t* gate = nullptr,
-                                    bool cleared = false) {
+                                    bool cleared = false, uint32_t absent = 0,
+                                    unsigned long long limit_ns = kWaitLimitNs) {
   const SoLayout L = so_layout(n);
   char* w = static_cast<char*>(zeroed);
   char* r = static_cast<char*>(rest) - L.zero_bytes;
@@ -440,9 +441,9 @@ static cudaError_t launch_sort_once(uint32_t* keys, uint32_t* alt, int n, int ke
   A.n = n;
   A.key_bits = key_bits;
   A.low_bits = low_bits;
-  A.bar = reinterpret_cast<uint32_t*>(w);
-  A.high = A.bar + 1;
-  A.next = A.bar + 2;
+  A.bar = GridBarrier{reinterpret_cast<uint32_t*>(w), absent, limit_ns};
+  A.high = A.bar.arrivals + 1;
+  A.next = A.bar.arrivals + 2;
   A.hist = reinterpret_cast<uint32_t*>(w + L.hist_off);
   A.ids = reinterpret_cast<uint32_t*>(r + L.ids_off);
   A.mat = reinterpret_cast<uint32_t*>(r + L.mat_off);
@@ -500,6 +501,23 @@ cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits,
   if (e == cudaSuccess && result != keys)
     e = cudaMemcpyAsync(keys, result, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToDevice, s);
   return e;
+}
+
+constexpr int kSoDiagKeys = (kSoMaxCluster + 1) * kSoMinPer;  // the fewest of a cooperative grid
+size_t diag_grid_wait_bytes() {
+  return 2 * sizeof(uint32_t) * (size_t)kSoDiagKeys + so_layout(kSoDiagKeys).total;
+}
+cudaError_t launch_diag_grid_wait(void* workspace, uint32_t* status, unsigned long long limit_ns,
+                                  cudaStream_t s) {
+  uint32_t* keys = static_cast<uint32_t*>(workspace);
+  uint32_t* alt = keys + kSoDiagKeys;
+  char* w = reinterpret_cast<char*>(alt + kSoDiagKeys);
+  const cudaError_t e = cudaMemsetAsync(keys, 0, sizeof(uint32_t) * (size_t)kSoDiagKeys, s);
+  return e == cudaSuccess
+             ? launch_sort_once(keys, alt, kSoDiagKeys, 30, 30, w,
+                                w + so_layout(kSoDiagKeys).zero_bytes, status, s, nullptr, false,
+                                1u, limit_ns)
+             : e;
 }
 
 // A sort that mostly does not run (gate 0) is chosen by what its return costs:

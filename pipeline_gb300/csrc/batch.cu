@@ -233,6 +233,7 @@ __global__ void __launch_bounds__(kPfThreads, 5)
     prefix_slots_tile(S, ec + cs, ps_out + cs, n, lo, tile_prefix[t] - tile_prefix[d.w],
                       slot_tags(tags, ns, B.node_start[c + 1] - ns), max_slot_c + c);
   }
+  if (threadIdx.x == 0) bulk_wait_all();
 }
 
 // Inclusive prefix sum of each cloud's edge counts (written by the tree

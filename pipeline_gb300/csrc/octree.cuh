@@ -232,7 +232,9 @@ __device__ __forceinline__ int pf_pad(int j) { return j + (j >> 5); }
 
 // ec, ps: the cloud's arrays; the tile's nodes are [lo, min(lo + kTile, n)), its
 // exclusive prefix ex. max_slot: raised to the largest slot stages 7-8 write.
-// All threads call it; ends with a barrier.
+// All threads call it; ends with a barrier. The zeroing copies may still be on
+// their way then: thread 0 waits for them (bulk_wait_all) before its kernel
+// ends, or before a barrier after which the tags are written.
 template <int THREADS, int ITEMS>
 __device__ __forceinline__ void prefix_slots_tile(PrefixSmem<THREADS, ITEMS>& S, const int* ec,
                                                   int* ps, int n, int lo, uint32_t ex,
@@ -720,7 +722,8 @@ __device__ __forceinline__ void finalize_slot(bool fresh, int p, const OctArgs& 
 // The block's staged nodes to dst[0, count): one bulk copy (the TMA engine
 // writes it) when dst is 16-byte aligned and the block a whole number of
 // 16-byte words, else vector and word stores. The block's threads call it
-// after staging; the stage is free again when it returns.
+// after staging; the stage is free again when it returns, the copy done when
+// thread 0 has waited for it (bulk_wait_all), as it does before its kernel ends.
 __device__ __forceinline__ void store_node_block(const int* s_nodes, oct_node* nodes, int count) {
   bulk_fence_writes();
   __syncthreads();

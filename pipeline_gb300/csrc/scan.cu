@@ -405,6 +405,7 @@ __global__ void __launch_bounds__(kPfThreads, 5)
   const int lo = blockIdx.x * kPfTile;
   if (lo >= n) return;
   prefix_slots_tile(S, ec, ps, n, lo, tile_prefix[blockIdx.x], t, d_max_slot);
+  if (threadIdx.x == 0) bulk_wait_all();
 }
 
 cudaError_t launch_prefix_sum_clear_tags(int n_host, const int* d_unique, int* ec, int* ps,

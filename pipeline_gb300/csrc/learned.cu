@@ -282,6 +282,8 @@ struct LcdfMoments {
   float* B;
   float* C;
   uint32_t* mid;  // first + one past last sample rank: twice the mean t times S
+  // (of a segment of more than kMomChunk keys A and B hold the first and the one
+  // past the last rank, as integers; its sums are those of its parts)
 };
 static size_t lcdf_moments_bytes() { return 5 * 4 * (size_t)kLcdfMaxSegments; }
 static LcdfMoments lcdf_moments_carve(void* base) {
@@ -314,17 +316,126 @@ __device__ __forceinline__ int warp_lower_rank(const uint32_t* __restrict__ samp
   return (int)lo;
 }
 
-// One warp per segment.
-__global__ void __launch_bounds__(256)
+// A segment of more than kMomChunk keys is summed by chunks of as many ranks
+// first, one warp each, so that no warp walks a segment that holds most of the
+// sample (one value, or few segments: 2.5 ms for 262,144 keys by one warp, 41 ms
+// for 4M, where a stepwise step took 0.04 and 0.34).
+constexpr int kMomChunk = 512;
+constexpr int kMomRows = kMomChunk / 32;
+// The sums of a chunk's first segment and of its last one where that is another,
+// ranks counted from the chunk's middle. A segment longer than a chunk is one of
+// these in every chunk that it meets.
+struct LcdfPart {
+  double a, b, c;
+};
+static size_t lcdf_chunks(int S) { return ((size_t)S + kMomChunk - 1) / kMomChunk; }
+
+template <class T>
+__device__ __forceinline__ T warp_sum(T v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Segment of key v (whole warp).
+__device__ __forceinline__ int warp_segment(const uint32_t* __restrict__ x, int K, uint32_t v) {
+  return min(max(warp_lower_rank(x, K, v + 1u) - 1, 0), K - 1);
+}
+
+// By the calling warp, in whole numbers (exact, and the 64-bit floating-point pipe
+// would bound 4M keys at 0.2 ms); parts of segments that are not longer than a
+// chunk are mostly left out (nobody reads them).
+__device__ __forceinline__ void lcdf_chunk_parts(const uint32_t* __restrict__ sample, int S,
+                                                 const uint32_t* __restrict__ x, int K,
+                                                 long long chunk, LcdfPart* __restrict__ parts) {
+  const int lane = threadIdx.x & 31;
+  const long long r0 = chunk * kMomChunk, r1 = min(r0 + kMomChunk, (long long)S);
+  if (r0 >= S) return;
+  uint32_t key[kMomRows];
+#pragma unroll
+  for (int j = 0; j < kMomRows; ++j) {
+    const long long i = r0 + j * 32 + lane;
+    key[j] = i < r1 ? sample[i] : 0u;
+  }
+  const uint32_t end = sample[r1 - 1];
+  const int s0 = warp_segment(x, K, __shfl_sync(0xffffffffu, key[0], 0));
+  const int s1 = s0 == K - 1 || end < x[s0 + 1] ? s0 : warp_segment(x, K, end);
+#pragma unroll 1
+  for (int slot = 0; slot < 2; ++slot) {
+    const int k = slot ? s1 : s0;
+    const uint32_t x0 = x[k], x1 = x[k + 1];
+    const uint32_t from = k == 0 ? 0u : x0, to = k == K - 1 ? 0xffffffffu : x1;
+    int own = 0;  // the segment's keys in this chunk
+#pragma unroll
+    for (int j = 0; j < kMomRows; ++j)
+      own += r0 + j * 32 + lane < r1 && key[j] >= from && (key[j] < to || k == K - 1);
+    own = __reduce_add_sync(0xffffffffu, own);
+    if (s0 != s1) {  // one end is here: does it reach a chunk's length beyond?
+      const long long far = slot ? r1 - own + kMomChunk : r0 + own - kMomChunk - 1;
+      if (far < 0 || far >= S) continue;
+      const uint32_t v = sample[far];
+      if (v < from || (v >= to && k != K - 1)) continue;
+    }
+    // sums of d, d^2 (its halves apart) and d times twice the rank from the middle
+    long long sd = 0, lo = 0, hi = 0, sr = 0;
+#pragma unroll
+    for (int j = 0; j < kMomRows; ++j) {
+      const uint32_t v = key[j];
+      if (r0 + j * 32 + lane < r1 && v >= max(from, x0) && (v < to || k == K - 1)) {
+        const uint32_t d = v - x0;
+        const unsigned long long dd = (unsigned long long)d * d;
+        sd += d;
+        lo += (uint32_t)dd;
+        hi += (uint32_t)(dd >> 32);
+        sr += (long long)d * (2 * (j * 32 + lane) + 1 - kMomChunk);
+      }
+    }
+    sd = warp_sum(sd);
+    lo = warp_sum(lo);
+    hi = warp_sum(hi);
+    sr = warp_sum(sr);
+    const double inv = 1.0 / (double)(x1 - x0);
+    if (lane == 0)
+      parts[chunk * 2 + slot] =
+          LcdfPart{(double)sd * inv, ((double)hi * 0x1p32 + (double)lo) * inv * inv,
+                   (double)sr * inv * (0.5 / (double)S)};
+    if (s0 == s1) break;
+  }
+}
+
+// One warp per segment in the first seg_blocks CTAs, per chunk in the others.
+constexpr int kMomWarps = 8;
+__global__ void __launch_bounds__(32 * kMomWarps)
     lcdf_moments_kernel(const uint32_t* __restrict__ sample, int S, const char* __restrict__ blob,
-                        LcdfLayout L, LcdfMoments M) {
+                        LcdfLayout L, LcdfMoments M, int k_req, int seg_blocks,
+                        LcdfPart* __restrict__ parts) {
   const int K = reinterpret_cast<const LcdfHeader*>(blob)->n_knots;
   const uint32_t* x = reinterpret_cast<const uint32_t*>(blob + L.x);
-  const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5);
+  if ((int)blockIdx.x >= seg_blocks) {
+    // Knots that are all different lie close: no segment is as long as two
+    // steps from one knot's rank to the next.
+    if (K == k_req && 2 * (((long long)S + k_req - 1) / k_req) <= kMomChunk) return;
+    lcdf_chunk_parts(sample, S, x, K,
+                     (long long)((int)blockIdx.x - seg_blocks) * kMomWarps + warp, parts);
+    return;
+  }
+  const int k = (int)blockIdx.x * kMomWarps + warp;
   if (k >= K) return;
   const uint32_t x0 = x[k], x1 = x[k + 1];
   const int a = k == 0 ? 0 : warp_lower_rank(sample, S, x0);
   const int b = k == K - 1 ? S : warp_lower_rank(sample, S, x1);
+  if (lane == 0) {
+    M.c[k] = (float)(b - a);
+    M.mid[k] = (uint32_t)a + (uint32_t)b;
+  }
+  if (b - a > kMomChunk) {
+    if (lane == 0) {
+      M.A[k] = __int_as_float(a);
+      M.B[k] = __int_as_float(b);
+    }
+    return;
+  }
   const double inv = 1.0 / (double)(x1 - x0), invS = 1.0 / (double)S;
   const double mean = 0.5 * ((double)a + (double)b);
   double sa = 0.0, sb = 0.0, sc = 0.0;
@@ -335,19 +446,32 @@ __global__ void __launch_bounds__(256)
     sb += f * f;
     sc += f * (((double)i + 0.5 - mean) * invS);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    sa += __shfl_xor_sync(0xffffffffu, sa, o);
-    sb += __shfl_xor_sync(0xffffffffu, sb, o);
-    sc += __shfl_xor_sync(0xffffffffu, sc, o);
-  }
+  sa = warp_sum(sa);
+  sb = warp_sum(sb);
+  sc = warp_sum(sc);
   if (lane == 0) {
-    M.c[k] = (float)(b - a);
     M.A[k] = (float)sa;
     M.B[k] = (float)sb;
     M.C[k] = (float)sc;
-    M.mid[k] = (uint32_t)a + (uint32_t)b;
   }
+}
+
+// The sums of a segment of ranks [a, b), b - a > kMomChunk, from its parts
+// (whole warp).
+__device__ __forceinline__ LcdfPart lcdf_long_segment(const LcdfPart* __restrict__ parts, int a,
+                                                      int b, int S) {
+  const int lane = threadIdx.x & 31;
+  const double invS = 1.0 / (double)S, mean = 0.5 * ((double)a + (double)b);
+  const int first = a / kMomChunk, last = (b - 1) / kMomChunk;
+  LcdfPart s = {0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int q = first + lane; q <= last; q += 32) {
+    const LcdfPart p = parts[2 * (size_t)q + (q == first && a % kMomChunk != 0 ? 1 : 0)];
+    s.a += p.a;
+    s.b += p.b;
+    s.c += p.c + p.a * (((double)q * kMomChunk + kMomChunk / 2 - mean) * invS);
+  }
+  return LcdfPart{warp_sum(s.a), warp_sum(s.b), warp_sum(s.c)};
 }
 
 // The steps run on one cluster of up to eight CTAs, a segment per thread: one
@@ -371,12 +495,6 @@ __device__ __forceinline__ void st_cluster(long long* p, uint32_t rank, long lon
   uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
   asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(a) : "r"(rank));
   asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
-}
-
-__device__ __forceinline__ long long warp_sum64(long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
 }
 
 // Warp totals of a cluster-wide scan, in every CTA: one slot per warp.
@@ -410,12 +528,13 @@ __device__ __forceinline__ long long cluster_scan_read(const ClusterTotals& T, l
     all += t;
     before += i < me ? t : 0;
   }
-  total = warp_sum64(all);
-  return warp_sum64(before);
+  total = warp_sum(all);
+  return warp_sum(before);
 }
 
 __global__ void __launch_bounds__(kTrThreads)
-    lcdf_train_kernel(char* blob, LcdfLayout L, LcdfMoments M, int S, int steps, float lr) {
+    lcdf_train_kernel(char* blob, LcdfLayout L, LcdfMoments M, const LcdfPart* parts, int S,
+                      int steps, float lr) {
   // three tables a step; each is written again only after a barrier that
   // follows its last read
   __shared__ ClusterTotals s_height, s_grad, s_gy;
@@ -426,8 +545,18 @@ __global__ void __launch_bounds__(kTrThreads)
   float* g_theta = reinterpret_cast<float*>(blob + L.theta);
   float* g_m = reinterpret_cast<float*>(blob + L.adam_m);
   float* g_v = reinterpret_cast<float*>(blob + L.adam_v);
-  const float c = in ? M.c[k] : 0.f, A = in ? M.A[k] : 0.f, B = in ? M.B[k] : 0.f;
-  const float C = in ? M.C[k] : 0.f;
+  const float c = in ? M.c[k] : 0.f;
+  float A = in ? M.A[k] : 0.f, B = in ? M.B[k] : 0.f, C = in ? M.C[k] : 0.f;
+  for (uint32_t todo = __ballot_sync(0xffffffffu, c > (float)kMomChunk); todo; todo &= todo - 1u) {
+    const int src = __ffs(todo) - 1;  // a lane's segment is long: the warp adds its parts
+    const LcdfPart p = lcdf_long_segment(parts, __shfl_sync(0xffffffffu, __float_as_int(A), src),
+                                         __shfl_sync(0xffffffffu, __float_as_int(B), src), S);
+    if (lane == src) {
+      A = (float)p.a;
+      B = (float)p.b;
+      C = (float)p.c;
+    }
+  }
   const unsigned long long mid = in ? M.mid[k] : 0u;
   float th = in ? g_theta[k] : 0.f, m = in ? g_m[k] : 0.f, v = in ? g_v[k] : 0.f;
   const unsigned long long two_s = 2ull * (unsigned)S;
@@ -458,7 +587,7 @@ __global__ void __launch_bounds__(kTrThreads)
     const long long gy_own =
         __float2ll_rn(a0 * y0 * 0x1p60f) + __float2ll_rn(a1 * y1 * 0x1p60f);
     const long long ginc = cluster_scan_send(g0 + g1, s_grad);
-    const long long gy_warp = warp_sum64(gy_own);
+    const long long gy_warp = warp_sum(gy_own);
     if (lane < (int)gridDim.x)
       st_cluster(&s_gy.t[blockIdx.x * kTrWarps + (threadIdx.x >> 5)], (uint32_t)lane, gy_warp);
     const int step = step0 + it + 1;
@@ -636,7 +765,7 @@ cudaError_t launch_lcdf_train(const uint32_t* sorted_sample, int S, int steps, f
 }
 
 cudaError_t launch_lcdf_fit(const uint32_t* sorted_sample, int S, int k_req, int steps, float lr,
-                            char* blob, const LcdfLayout& L, int nb, void* moments,
+                            char* blob, const LcdfLayout& L, int nb, void* moments, void* scratch,
                             cudaStream_t s) {
   lcdf_knots_kernel<<<1, 1024, 0, s>>>(sorted_sample, S, k_req, blob, L);
   const size_t fb_smem = 12 * (size_t)(L.max_knots + 1);
@@ -647,7 +776,12 @@ cudaError_t launch_lcdf_fit(const uint32_t* sorted_sample, int S, int k_req, int
   // (a rate that is not positive moves nothing, as in the stepwise kernels)
   if (steps > 0 && lr > 0.f && (float)steps * lr <= kTrMost) {
     const LcdfMoments M = lcdf_moments_carve(moments);
-    lcdf_moments_kernel<<<(k_req + 7) / 8, 256, 0, s>>>(sorted_sample, S, blob, L, M);
+    LcdfPart* parts = static_cast<LcdfPart*>(scratch);
+    const int seg_blocks = (k_req + kMomWarps - 1) / kMomWarps;
+    const size_t chunks = S > kMomChunk ? lcdf_chunks(S) : 0;  // (fewer keys: no long segment)
+    const unsigned blocks = seg_blocks + (unsigned)((chunks + kMomWarps - 1) / kMomWarps);
+    lcdf_moments_kernel<<<blocks, 32 * kMomWarps, 0, s>>>(sorted_sample, S, blob, L, M, k_req,
+                                                          seg_blocks, parts);
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3((k_req + kTrThreads - 1) / kTrThreads);
     c.blockDim = dim3(kTrThreads);
@@ -657,7 +791,7 @@ cudaError_t launch_lcdf_fit(const uint32_t* sorted_sample, int S, int k_req, int
     at[0].val.clusterDim = {c.gridDim.x, 1u, 1u};
     c.attrs = at;
     c.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&c, lcdf_train_kernel, blob, L, M, S, steps, lr);
+    const cudaError_t e = cudaLaunchKernelEx(&c, lcdf_train_kernel, blob, L, M, parts, S, steps, lr);
     if (e != cudaSuccess) return e;
   } else {  // heights could leave the fixed point's range, or nothing moves
     const cudaError_t e = launch_lcdf_train(sorted_sample, S, steps, lr, blob, L, s);
@@ -743,7 +877,7 @@ OCT_API int oct_lcdf_fit(const uint32_t* sample_keys, int n_sample, int n_segmen
   const LcdfLayout L = lcdf_layout(max_segments);
   if (e == cudaSuccess)
     e = launch_lcdf_fit(keys, n_sample, n_segments, steps, lr, static_cast<char*>(model), L,
-                        n_buckets, alt + align_up(4 * (size_t)n_sample, 256) / 4, s);
+                        n_buckets, alt + align_up(4 * (size_t)n_sample, 256) / 4, alt, s);
   if (e != cudaSuccess) {
     set_last_error(cudaGetErrorString(e));
     return OCT_ERR_CUDA;

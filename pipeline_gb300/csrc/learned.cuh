@@ -112,8 +112,9 @@ __device__ __forceinline__ uint32_t lcdf_bucket(const LcdfTables& t, uint32_t v)
   return min(fx >> kLcdfFix, (uint32_t)(t.nb - 1));
 }
 
+// scratch: S words, 8-byte aligned.
 cudaError_t launch_lcdf_fit(const uint32_t* sorted_sample, int S, int k_req, int steps, float lr,
-                            char* blob, const LcdfLayout& L, int nb, void* moments,
+                            char* blob, const LcdfLayout& L, int nb, void* moments, void* scratch,
                             cudaStream_t s);
 cudaError_t launch_lcdf_train(const uint32_t* sorted_sample, int S, int steps, float lr, char* blob,
                               const LcdfLayout& L, cudaStream_t s);

@@ -19,10 +19,12 @@
 //            taken from the global count's atomic add
 //   scatter  bucket bases (every CTA scans the 4,096 counts), the codes to
 //            their buckets
+//   cut      only when a bucket holds far more codes than a CTA's share (a cloud
+//            in a small part of its box): such buckets are cut by further bits,
+//            and the codes counted again before they are scattered
 //   sort     a CTA takes the buckets that start in its share of the codes:
 //            sorted in shared memory and made unique; a bucket too large for
-//            that by a bitmap over its 2^18 values, which takes any number of
-//            codes, so a cloud that falls into few buckets costs time only
+//            that (few values then) by a bitmap, which takes any number of codes
 //   codes    every run to its place (a scan of the CTAs' counts), the deltas
 //            of adjacent codes and the tiles' smallest
 //   tree     tree_nodes_tile, one tile per CTA (1,024 positions at least)
@@ -52,13 +54,24 @@ constexpr int kFuShare = 12288;                    // codes per CTA at most (the
 constexpr int kFuBucketBits = 12;
 constexpr int kFuBuckets = 1 << kFuBucketBits;
 constexpr int kFuSpanBits = 30 - kFuBucketBits;    // values of a bucket: a 32 KiB bitmap
+// Codes from which a bucket is cut. A bucket that is not costs its CTA 1.5 ns for
+// each of its unique codes (their stores, and later their places) and up to 47 us
+// here; the cut costs a build that takes it 6 (a frame's size) to 12 us (1.9M). With
+// it clouds in one such bucket take 49 us (122,880 points), 59 (400,000), 72 (1M) and
+// 90 (1.86M) where one CTA took 162, 310, 413 and 537, and the stage-by-stage build
+// 150, 154, 164 and 188.
+constexpr uint32_t kFuCut = 32768;
+constexpr uint32_t kFuUnit = 2048;                 // codes of the parts that even ones give
+constexpr int kFuIds = 7168;                       // buckets after the cut, at most
 constexpr int kFuTile = 1024;                      // tree and prefix tiles: multiples of this
 constexpr int kFuMaxGrid = 256;
 constexpr int kFuMaxCluster = 8;                   // the portable cluster size
 constexpr int kFuMinPer = 1024;                    // points per CTA at least
+static_assert(kFuBuckets + 2 * (kFuMaxGrid * kFuShare / (int)kFuUnit) <= kFuIds,
+              "a bucket of c codes has fewer than 2 c / kFuUnit parts");
 
 struct FusedLayout {
-  size_t misc_off, hist_off, zero_bytes, cta_off, keys_off, min_off, sum_off, d_off, tags_off,
+  size_t misc_off, hist_off, zero_bytes, ids_off, cta_off, keys_off, min_off, sum_off, d_off, tags_off,
       total;
 };
 
@@ -74,6 +87,7 @@ static FusedLayout fused_layout(int n, int cap) {
   L.misc_off = take(256);
   L.hist_off = take(4 * (size_t)kFuBuckets);
   L.zero_bytes = o;
+  L.ids_off = take(4 * (size_t)kFuIds);
   L.cta_off = take(8 * (size_t)kFuMaxGrid);
   L.keys_off = take(4 * (size_t)n);
   L.min_off = take(align_up(tiles, kTtMinBlock));
@@ -90,6 +104,7 @@ struct FusedArgs {
   float min_coord, range;
   GridBarrier bar;
   uint32_t* hist;    // [kFuBuckets] zeroed
+  uint32_t* ids;     // [kFuIds] counts after the cut
   uint32_t* status;
   int* max_slot;
   uint32_t* cta_count;  // [grid] unique codes of a CTA's run
@@ -107,10 +122,16 @@ struct FusedArgs {
 struct FusedSort {
   __align__(16) uint32_t a[kFuCap + kBinPad];
   __align__(16) uint32_t b[kFuCap + kBinPad];
-  uint32_t base[kFuBuckets];       // counts, then the CTA's place in each bucket
-  uint32_t start[kFuBuckets + 1];  // first position of each bucket
-  uint32_t aux[kBinAux];
+  uint32_t start[kFuIds + 1];  // first position of each bucket
+  uint16_t tab[kFuBuckets + 2];  // after a cut: a bucket's first part
+  union {
+    uint32_t base[kFuIds];  // counts, then the CTA's place in each bucket
+    uint32_t aux[kBinAux];
+  };
 };
+// 196 KiB of an SM's 256: the rest is the L1 cache of the tree and octree phases
+// (with 228 KiB taken a build of 1M points took 4 us more).
+static_assert(sizeof(FusedSort) <= 196 * 1024 - 3072, "leaves the next L1 size");
 union FusedSmem {
   FusedSort s;
   TreeSmem<kFuShare, kFuThreads> tree;
@@ -147,40 +168,82 @@ __device__ __forceinline__ uint32_t fused_unique(const uint32_t* a, int cnt, uin
   return *total;
 }
 
-// Sorted unique codes of a bucket of any size by bitmap (bm: 2^18 bits of
-// shared memory), over the front of its own range keys[0, cnt).
-__device__ uint32_t fused_bitmap_bucket(uint32_t* keys, uint32_t cnt, uint32_t* bm,
-                                        uint32_t* warp_tot, uint32_t* total) {
-  constexpr int kWords = 1 << (kFuSpanBits - 5);
-  constexpr int kPer = kWords / kFuThreads;
-  constexpr uint32_t kMask = (1u << kFuSpanBits) - 1u;
+// First positions of the buckets of counts c (EACH per thread, in order; ex: codes
+// before the thread's), added to the CTA's places; in s_cut the CTA's share
+// [w0, w1) of the `kept` codes as whole buckets: lo, hi, start of the last.
+template <int EACH>
+__device__ __forceinline__ void fused_starts(FusedSort& M, const uint32_t (&c)[EACH], uint32_t ex,
+                                             uint32_t w0, uint32_t w1, uint32_t kept,
+                                             uint32_t* s_cut) {
   const int tid = threadIdx.x;
-  for (int w = tid; w < kWords; w += kFuThreads) bm[w] = 0u;
-  const uint32_t top = keys[0] & ~kMask;
+  if (tid == 0) {
+    s_cut[0] = w0 == 0 ? 0u : kept;
+    s_cut[1] = kept;
+    s_cut[2] = kept;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < EACH; ++k) {
+    // a boundary inside or at the end of this bucket moves to its end
+    if (ex < w0 && w0 <= ex + c[k]) s_cut[0] = ex + c[k];
+    if (ex < w1 && w1 <= ex + c[k]) {
+      s_cut[1] = ex + c[k];
+      s_cut[2] = ex;
+    }
+    M.start[EACH * tid + k] = ex;
+    M.base[EACH * tid + k] += ex;
+    ex += c[k];
+  }
+  if (tid == kFuThreads - 1) M.start[EACH * kFuThreads] = ex;
+  __syncthreads();
+}
+
+// Bucket of code k after a cut, and the bits of its values.
+__device__ __forceinline__ uint32_t fused_part(const FusedSort& M, uint32_t k, int& bits) {
+  const uint32_t b = k >> kFuSpanBits, t = M.tab[b], n = M.tab[b + 1u] - t;  // a power of two
+  bits = kFuSpanBits - (31 - __clz(n));
+  return t + ((k >> bits) & (n - 1u));
+}
+
+// Sorted unique codes of a bucket of any size by bitmap (bm: 2^bits bits of
+// shared memory, bits >= 5), over the front of its own range keys[0, cnt).
+__device__ uint32_t fused_bitmap_bucket(uint32_t* keys, uint32_t cnt, int bits, uint32_t* bm,
+                                        uint32_t* warp_tot, uint32_t* total) {
+  const int words = 1 << (bits - 5);
+  const int per = (words + kFuThreads - 1) / kFuThreads;
+  const uint32_t mask = (1u << bits) - 1u;
+  const int tid = threadIdx.x;
+  for (int w = tid; w < words; w += kFuThreads) bm[w] = 0u;
+  const uint32_t top = keys[0] & ~mask;
   __syncthreads();
   for (uint32_t i0 = tid; i0 < cnt; i0 += 4 * kFuThreads) {
     uint32_t k[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const uint32_t i = i0 + (uint32_t)q * kFuThreads;
-      k[q] = i < cnt ? keys[i] & kMask : 0xffffffffu;
+      k[q] = i < cnt ? keys[i] & mask : 0xffffffffu;
     }
+    uint32_t seen[4];  // (a value that comes often would be a chain of atomics)
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      if (k[q] != 0xffffffffu) atomicOr(&bm[k[q] >> 5], 1u << (k[q] & 31u));
+      seen[q] = k[q] != 0xffffffffu ? *(volatile uint32_t*)&bm[k[q] >> 5] : 0xffffffffu;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (!(seen[q] >> (k[q] & 31u) & 1u)) atomicOr(&bm[k[q] >> 5], 1u << (k[q] & 31u));
   }
   __syncthreads();
+  const int w0 = min(tid * per, words), w1 = min(w0 + per, words);
   uint32_t own = 0;
-#pragma unroll
-  for (int q = 0; q < kPer; ++q) own += __popc(bm[tid * kPer + q]);
+#pragma unroll 8
+  for (int w = w0; w < w1; ++w) own += __popc(bm[w]);
   uint32_t pos = block_exclusive_sum<kFuThreads>(own, warp_tot, total);
 #pragma unroll 1
-  for (int q = 0; q < kPer; ++q) {
-    uint32_t bits = bm[tid * kPer + q];
-    while (bits) {
-      const int bit = __ffs(bits) - 1;
-      bits &= bits - 1u;
-      keys[pos++] = top | ((uint32_t)(tid * kPer + q) << 5) | (uint32_t)bit;
+  for (int w = w0; w < w1; ++w) {
+    uint32_t set = bm[w];
+    while (set) {
+      const int bit = __ffs(set) - 1;
+      set &= set - 1u;
+      keys[pos++] = top | ((uint32_t)w << 5) | (uint32_t)bit;
     }
   }
   __syncthreads();
@@ -217,6 +280,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
         *A.max_slot = 0;
       }
     }
+    for (int b = (int)cta * kFuThreads + tid; b < kFuIds; b += (int)G * kFuThreads) A.ids[b] = 0u;
     fill_spread_lut(lut);
     // tile sums and minima start empty (used three barriers later)
     const int pad = (int)align_up((size_t)A.S.tiles, kTtMinBlock);
@@ -269,44 +333,82 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
 
   // ---- scatter into buckets; this CTA's share of them
   uint32_t lo, hi, cut, share;
+  bool parts;  // (the same in every CTA: all read the same counts)
   {
     constexpr int kPer = kFuBuckets / kFuThreads;
     static_assert(kPer == 4, "one 16-byte load of counts per thread");
     const uint4 q = reinterpret_cast<const uint4*>(A.hist)[tid];
     const uint32_t c[kPer] = {q.x, q.y, q.z, q.w};
-    uint32_t ex = block_exclusive_sum<kFuThreads>(c[0] + c[1] + c[2] + c[3], s_warp, &s_total);
+    const uint32_t ex =
+        block_exclusive_sum<kFuThreads>(c[0] + c[1] + c[2] + c[3], s_warp, &s_total);
     const uint32_t kept = s_total;
     share = (kept + G - 1u) / G;
     const uint32_t w0 = min(cta * share, kept), w1 = min(w0 + share, kept);
-    if (tid == 0) {
-      s_cut[0] = w0 == 0 ? 0u : kept;
-      s_cut[1] = kept;
-      s_cut[2] = kept;
-    }
-    __syncthreads();
+    parts = __syncthreads_or(max(max(c[0], c[1]), max(c[2], c[3])) > kFuCut) != 0;
+    if (!parts) {
+      fused_starts(M.s, c, ex, w0, w1, kept, s_cut);
+    } else {
+      uint32_t sub[kPer], mine = 0;
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      // a boundary inside or at the end of this bucket moves to its end
-      if (ex < w0 && w0 <= ex + c[k]) s_cut[0] = ex + c[k];
-      if (ex < w1 && w1 <= ex + c[k]) {
-        s_cut[1] = ex + c[k];
-        s_cut[2] = ex;
+      for (int k = 0; k < kPer; ++k) {
+        sub[k] = 0;
+        if (c[k] > kFuCut)
+          while ((kFuUnit << sub[k]) < c[k]) ++sub[k];
+        mine += 1u << sub[k];
       }
-      M.s.start[kPer * tid + k] = ex;
-      M.s.base[kPer * tid + k] += ex;
-      ex += c[k];
+      uint32_t id = block_exclusive_sum<kFuThreads>(mine, s_warp, &s_total);
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        M.s.tab[kPer * tid + k] = (uint16_t)id;
+        id += 1u << sub[k];
+      }
+      if (tid == kFuThreads - 1) M.s.tab[kFuBuckets] = (uint16_t)id;
+      for (int b = tid; b < kFuIds; b += kFuThreads) M.s.base[b] = 0u;
+      __syncthreads();
+#pragma unroll
+      for (int it = 0; it < kFuItems; ++it) {
+        if (it * kFuThreads >= per) break;
+        const int sh = 16 * (it & 1);
+        if (((rank2[it / 2] >> sh) & 0xffffu) != 0xffffu) {
+          int bits;
+          const uint32_t r = atomicAdd(&M.s.base[fused_part(M.s, code[it], bits)], 1u);
+          rank2[it / 2] = (rank2[it / 2] & ~(0xffffu << sh)) | r << sh;
+        }
+      }
+      __syncthreads();
+      for (int b = tid; b < kFuIds; b += kFuThreads) {
+        const uint32_t n = M.s.base[b];
+        if (n) M.s.base[b] = atomicAdd(A.ids + b, n);
+      }
+      if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
+      constexpr int kEach = kFuIds / kFuThreads;
+      uint32_t p[kEach], sum = 0;
+#pragma unroll
+      for (int k = 0; k < kEach; ++k) {
+        p[k] = A.ids[kEach * tid + k];
+        sum += p[k];
+      }
+      fused_starts(M.s, p, block_exclusive_sum<kFuThreads>(sum, s_warp, &s_total), w0, w1, kept,
+                   s_cut);
     }
-    if (tid == kFuThreads - 1) M.s.start[kFuBuckets] = ex;
-    __syncthreads();
     lo = s_cut[0];
     hi = max(s_cut[1], lo);
     cut = max(s_cut[2], lo);
+    auto scatter = [&](auto bucket_of) {
 #pragma unroll
-    for (int it = 0; it < kFuItems; ++it) {
-      if (it * kFuThreads >= per) break;
-      const uint32_t r = (rank2[it / 2] >> (16 * (it & 1))) & 0xffffu;
-      if (r != 0xffffu) A.keys[M.s.base[code[it] >> kFuSpanBits] + r] = code[it];
-    }
+      for (int it = 0; it < kFuItems; ++it) {
+        if (it * kFuThreads >= per) break;
+        const uint32_t r = (rank2[it / 2] >> (16 * (it & 1))) & 0xffffu;
+        if (r != 0xffffu) A.keys[M.s.base[bucket_of(code[it])] + r] = code[it];
+      }
+    };
+    if (parts)
+      scatter([&](uint32_t k) {
+        int bits;
+        return fused_part(M.s, k, bits);
+      });
+    else
+      scatter([](uint32_t k) { return k >> kFuSpanBits; });
   }
   if (!fused_barrier<CLUSTER>(A, ++phase, &s_ok)) return;
 
@@ -320,19 +422,34 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
                      (hi - cut > 2u * (uint32_t)kFuThreads && hi - cut > 2u * share);
     const int cnt = (int)min((big ? cut : hi) - lo, (uint32_t)kFuCap);
     // every bucket has as many bins as codes, spread evenly over its values
-    auto place_of = [&](uint32_t k, uint32_t& into) {
-      const uint32_t b = k >> kFuSpanBits, s = M.s.start[b], c = M.s.start[b + 1] - s;
-      const uint32_t part = k << (32 - kFuSpanBits);
+    auto place_in = [&](uint32_t b, uint32_t part, uint32_t& into) {
+      const uint32_t s = M.s.start[b], c = M.s.start[b + 1] - s;
       into = part * c;
       return s - lo + __umulhi(part, c);
     };
-    uint32_t* sorted = smem_bin_sort<kFuWarps, kFuItems>(A.keys + lo, cnt, M.s.a, M.s.b, M.s.aux,
-                                                         s_warp, &s_total, s_cut, place_of);
+    auto sort = [&](auto place_of) {
+      return smem_bin_sort<kFuWarps, kFuItems>(A.keys + lo, cnt, M.s.a, M.s.b, M.s.aux, s_warp,
+                                               &s_total, s_cut, place_of);
+    };
+    // (two sorts: one that asks for every code costs 5 us of 104 at 1M points)
+    uint32_t* sorted =
+        parts ? sort([&](uint32_t k, uint32_t& into) {
+          int bits;
+          const uint32_t b = fused_part(M.s, k, bits);
+          return place_in(b, k << (32 - bits), into);
+        })
+              : sort([&](uint32_t k, uint32_t& into) {
+                  return place_in(k >> kFuSpanBits, k << (32 - kFuSpanBits), into);
+                });
     uint32_t* other = sorted == M.s.a ? M.s.b : M.s.a;
     u_small = fused_unique(sorted, cnt, other, s_warp, &s_total);
     run = other;
     __syncthreads();
-    if (big) u_big = fused_bitmap_bucket(A.keys + cut, hi - cut, sorted, s_warp, &s_total);
+    if (big) {
+      int bits = kFuSpanBits;
+      if (parts) fused_part(M.s, A.keys[cut], bits);
+      u_big = fused_bitmap_bucket(A.keys + cut, hi - cut, bits, sorted, s_warp, &s_total);
+    }
     if (tid == 0) {
       A.cta_count[cta] = u_small + u_big;
       A.cta_first[cta] = u_small ? run[0] : u_big ? A.keys[cut] : 0u;
@@ -470,6 +587,7 @@ cudaError_t launch_fused_build(const float4* pts, int n, float min_coord, float 
   A.bar.arrivals = A.status + 1;
   A.max_slot = reinterpret_cast<int*>(A.status + 2);
   A.hist = reinterpret_cast<uint32_t*>(w + L.hist_off);
+  A.ids = reinterpret_cast<uint32_t*>(w + L.ids_off);
   A.cta_count = reinterpret_cast<uint32_t*>(w + L.cta_off);
   A.cta_first = A.cta_count + kFuMaxGrid;
   A.keys = reinterpret_cast<uint32_t*>(w + L.keys_off);

@@ -823,13 +823,13 @@ int batch_build(const oct_batch_plan* P, const void* d_tables, const oct_vec4* p
   if (P->N > 0) {
     const int mgrid = std::max(1, std::min(B.Ts, sms * 16));
     // Sort: the top digit's scatter and the bucket sort, or stable digit passes
-    // (which count every digit): for other sort configurations, and for large
-    // clouds, whose uneven ones have buckets that a CTA sorts by itself for
-    // long. Whole builds, us, by passes and by buckets: 128 clouds of 3,000
-    // points, even 168 and 130, around 8 centres 173 and 139; 32 of 30,000, 195
-    // and 169, 213 and 196; 256 of 65,536, 1,049 and 985, 1,082 and 1,095; 16 of
-    // a million, 976 and 925, 923 and 1,172.
-    constexpr int kBucketMost = 49152;
+    // (which count every digit): for other sort configurations, and where a cloud
+    // may have a bucket that a CTA sorts by itself for long, as one in a small part
+    // of its box has. Whole builds, us, by passes and by buckets, even clouds and
+    // clouds in one bucket: 64 of 8,000 points 177 and 132, 174 and 146; 64 of
+    // 12,288, 192 and 155, 191 and 171; 64 of 16,384, 200 and 157, 198 and 203; 64
+    // of 49,152, 317 and 263, 307 and 454.
+    constexpr int kBucketMost = 12288;
     const bool buckets = P->buckets && P->largest <= kBucketMost;
     const int hists = buckets ? 1 : passes;
     const size_t msm = 4 * ((size_t)hists * bins + 1024);  // histograms + spread table

@@ -20,16 +20,15 @@
 //
 // Equal keys are alike, so their order is free: unless a key has bits above
 // key_bits, which the sort passes over. Such keys, and buckets beyond the
-// limits above (a few values that hold most of a large array), take stable
-// 8-bit digit passes inside the same launch.
+// limits above (a few values that hold much of a large array, which a look at
+// 1,024 keys finds first), take stable 8-bit digit passes inside the same launch.
 //
 // Measured against the launched digit passes, us: 20,000 even 32-bit keys 99 ->
-// 20, 130,000 99 -> 22, 1,048,576 102 -> 33, 4.2M 160 -> 75, 8.4M 231 -> 151;
-// Morton codes of points around 64 centres 99 -> 48 at 1M, 231 -> 224 at 8.4M;
-// one value 92 -> 68 at 130,000, 231 -> 89 at 8.4M. Up to some 100,000 keys the
-// phases' latencies are what is left, later the scatter's 4-byte stores (50 us
-// of 151 at 8.4M: an SM stores about one sector a cycle) and the shared-memory
-// work of the sort phase (64 us).
+// 20, 130,000 99 -> 22, 1,048,576 102 -> 33, 4M 157 -> 75; Morton codes of points
+// around 64 centres 99 -> 48 at 1M; one value 92 -> 68 at 130,000, 157 -> 48 at 4M.
+// Up to some 100,000 keys the phases' latencies are what is left, later the
+// scatter's 4-byte stores (a third at 8.4M: an SM stores about one sector a
+// cycle) and the shared-memory work of the sort phase.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -49,14 +48,21 @@ constexpr int kSoMaxGrid = 256;
 constexpr int kSoMaxCluster = 8;
 constexpr int kSoStretch = 14336; // positions whose buckets are sorted together (mostly at once)
 constexpr int kSoMinPer = 1024;   // keys per CTA at least
-// Larger arrays take the launched passes: uneven keys would lose (codes around
-// 64 centres 16.7M: 388 us by passes, 445 here) although even ones would not
-// (412 and 310). At the line codes break even (231 and 224 to 230; passed as
-// 32-bit keys, which leaves three quarters of the buckets empty, 228 and 236)
-// and even keys gain a third. The line also bounds the loss of the digit passes in here where
-// most of a large array is a few values: nine tenths one value 167 and 165 us at
-// 4.2M, 237 and 283 at 8.4M.
-constexpr int kSoMaxN = 1 << 23;
+// Larger arrays take the launched passes, which uneven keys, and keys of a few
+// values above all, are sorted faster by (8.4M Morton codes around 64 centres 235
+// us and 242 here, ten values that hold nine tenths 223 and 292) although even
+// ones are not (232 and 160). Up to the line none of 20 distributions is slower here
+// by more than 3%: 4M keys, even 157 and 75, codes around 64 centres 155 and 132,
+// a cloud a sixteenth of its box thick 155 and 116, a few values 146 to 164 and 141
+// to 144. (Just past it clouds a sixteenth of their box thick lose an eighth: 256
+// buckets about as large as a CTA sorts, some of which are split.)
+constexpr int kSoMaxN = 4000000;
+// Keys of which a few values hold much go through the digit passes in here at
+// once, not after two counts, 20 us of 155 at 4M: 1,024 keys of the array tell, of
+// which more than kSoFew are alike in all but 12 bits (the passes lose nothing to
+// the buckets' form on such keys). Fewer than kSoLook keys lose little.
+constexpr int kSoLook = 1 << 21;
+constexpr uint32_t kSoFew = 16;
 
 struct SoLayout {
   size_t hist_off, zero_bytes, ids_off, mat_off, total;
@@ -188,6 +194,16 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
   };
   auto top_of = [&](uint32_t k) { return (k >> shift) & (uint32_t)(kSoTop - 1); };
 
+  // ---- look
+  bool lsd = false;
+  if (A.n > kSoLook) {  // (every CTA looks at the same keys)
+    const uint32_t k = A.keys[(unsigned long long)tid * n / kSoThreads];
+    for (int b = tid; b < kSoTop; b += kSoThreads) M.tab[b] = 0u;
+    __syncthreads();
+    const uint32_t cell = ((k >> 12) * 0x9e3779b1u) >> (32 - kSoTopBits);
+    lsd = __syncthreads_or(atomicAdd(&M.tab[cell], 1u) >= kSoFew) != 0;
+  }
+
   // ---- count
   for (int b = tid; b < kSoTop; b += kSoThreads) base[b] = 0u;
   for (int b = (int)cta * kSoThreads + tid; b < kSoIds; b += (int)G * kSoThreads) A.ids[b] = 0u;
@@ -197,20 +213,22 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
     grid_barrier<CLUSTER>(A.bar, 0, &s_ok);
   }
   __syncthreads();
-  bool high = false;
-  count(kSoTop, A.hist, [&](uint32_t k) {
-    high |= A.key_bits < 32 && (k >> A.key_bits) != 0u;
-    return top_of(k);
-  });
-  if (__syncthreads_or(high) && tid == 0) *A.high = 1u;
-  if (!barrier()) return;
+  if (!lsd) {
+    bool high = false;
+    count(kSoTop, A.hist, [&](uint32_t k) {
+      high |= A.key_bits < 32 && (k >> A.key_bits) != 0u;
+      return top_of(k);
+    });
+    if (__syncthreads_or(high) && tid == 0) *A.high = 1u;
+    if (!barrier()) return;
+    lsd = *reinterpret_cast<volatile uint32_t*>(A.high) != 0u;
+  }
 
   // ---- bucket bases; buckets that don't fit are split
   constexpr int kPer = kSoTop / kSoThreads;
   static_assert(kPer == 4, "one 16-byte load of counts per thread");
   const uint4 q4 = reinterpret_cast<const uint4*>(A.hist)[tid];
   const uint32_t c4[kPer] = {q4.x, q4.y, q4.z, q4.w};
-  bool lsd = *reinterpret_cast<volatile uint32_t*>(A.high) != 0u;
   const uint32_t c_most = max(max(c4[0], c4[1]), max(c4[2], c4[3]));
   const bool split = __syncthreads_or(c_most > (uint32_t)kSoCap) != 0 && !lsd;
   int ids = kSoTop;

@@ -79,3 +79,41 @@ def test_batched_builds_of_concentrated_clouds(kind, clouds, n):
     with passes():
         want = us()
     assert us() < MARGIN * want
+
+
+def sort_us(src, bits):
+    from pipeline_gb300.kernels import k_SimpleRadixSort
+
+    keys, alt = torch.empty_like(src), torch.empty_like(src)
+
+    def run():
+        keys.copy_(src)
+        k_SimpleRadixSort(keys, alt, src.numel(), key_bits=bits)
+
+    return best_us(run, 10)
+
+
+@pytest.mark.parametrize("kind", ["nine tenths", "ten values", "narrow"])
+@pytest.mark.parametrize("n", [1_000_000, 3_900_000, 8_000_000])
+def test_sorts_of_keys_of_a_few_values(kind, n):
+    src = codes(kind, n).to(torch.int32)
+    for bits in (30, 32):
+        with passes():
+            want = sort_us(src, bits)
+        assert sort_us(src, bits) < MARGIN * want
+
+
+@pytest.mark.parametrize("kind", ["nine tenths", "ten values", "narrow", "one bucket", "one value"])
+@pytest.mark.parametrize("n", [(1 << 21) + 1, 3_999_999, 4_000_000, 4_000_001])
+def test_few_values_sort_like_torch(kind, n):
+    """On both sides of the array sizes from which the keys are looked at first and
+    from which they take launched passes; with bits above key_bits as well."""
+    from pipeline_gb300.kernels import k_SimpleRadixSort
+
+    src = codes(kind, n).to(torch.int32)
+    for bits, above in ((30, 0), (32, 0), (30, 1 << 30)):
+        keys = src + above
+        want = torch.sort(keys).values
+        alt, status = torch.empty_like(keys), torch.zeros(1, dtype=torch.int32, device="cuda")
+        k_SimpleRadixSort(keys, alt, n, key_bits=bits, status=status)
+        assert int(status[0]) == 0 and torch.equal(keys, want)

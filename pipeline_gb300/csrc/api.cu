@@ -388,12 +388,13 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
   // (top-digit scatter, per-bucket bitmaps, pack), chosen on the device from
   // the top-digit histogram; both write the sorted unique codes, U and the
   // deltas of adjacent codes, from which the tree (with the edge counts) is
-  // built. The sort is the one-launch sort where that takes the cloud: without
-  // the digit passes' histograms and, in the MSD form, without eight of their
-  // launches that only return (10M clustered points 612 -> 575 us,
-  // 16.7M uniform 802 -> 785; in place of the passes 2.3M clustered
-  // from a graph 202 -> 200). Timed stage by stage a build keeps the passes.
+  // built. The sort is the one-launch sort where that takes the cloud (2.5M
+  // even points 279 -> 207 us), else digit passes. Beside the MSD form they
+  // mostly do not run: up to 2^24 points they are three launches that return at
+  // once, and the Morton kernel counts the top digit only.
   const bool msd = n >= msd_min_n() && msd_plan_ok(L.sort);
+  const SortConfig cfg = L.sort.cfg, def = kSortConfigDefault;
+  const bool few = msd && n <= 1 << 24 && cfg.warps == def.warps && cfg.items == def.items;
   char* sort_ctrl = w + L.sort_off;
   const size_t top_row = (size_t)(L.sort.passes - 1) * L.sort.bins;
   const uint32_t* top_hist = reinterpret_cast<const uint32_t*>(sort_ctrl + L.sort.hist_off) + top_row;
@@ -404,15 +405,9 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
   if (once) {
     OCT_TRY(cudaMemsetAsync(w, 0, L.ctrl_bytes, s), "build: clear");
     OCT_TRY(launch_morton(reinterpret_cast<const float4*>(points), keys_a, n, min_coord, range,
-                          msd ? &L.sort : nullptr, sort_ctrl, m.status, s, true),
+                          nullptr, nullptr, m.status, s),
             "build: morton");
-    if (msd) {
-      OCT_TRY(launch_msd_gate(top_hist, n, m.form, w + L.msd_off, top_base, s), "build: sort form");
-      OCT_TRY(launch_msd_scatter(keys_a, keys_b, &L.sort, sort_ctrl, m.status, m.form, s),
-              "build: scatter");
-    }
-    const cudaError_t e =
-        launch_sort_once_in_plan(keys_a, keys_b, L.sort, sort_ctrl, m.status, lsd_flag, s);
+    const cudaError_t e = launch_sort_once_in_plan(keys_a, keys_b, L.sort, sort_ctrl, m.status, s);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       (void)cudaGetLastError();  // a context with fewer SMs: again with the passes
       once = false;
@@ -425,14 +420,20 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
     OCT_TRY(cudaMemsetAsync(w, 0, L.ctrl_bytes, s), "build: clear");
     mark(rec, s);
     OCT_TRY(launch_morton(reinterpret_cast<const float4*>(points), keys_a, n, min_coord, range,
-                          &L.sort, sort_ctrl, m.status, s),
+                          &L.sort, sort_ctrl, m.status, s, few),
             "build: morton");
     mark(rec, s);
     if (msd)
-      OCT_TRY(launch_msd_gate(top_hist, n, m.form, w + L.msd_off, nullptr, s), "build: sort form");
-    OCT_TRY(launch_sort_passes_split(keys_a, keys_b, &L.sort, sort_ctrl, m.status,
-                                     msd ? m.form : nullptr, lsd_flag, s, &sorted, rec),
-            "build: sort");
+      OCT_TRY(launch_msd_gate(top_hist, n, m.form, w + L.msd_off, few ? top_base : nullptr, s),
+              "build: sort form");
+    if (few)  // (the look-back words: the tree's scratch is not used yet)
+      OCT_TRY(launch_sort_passes_few(keys_a, keys_b, &L.sort, sort_ctrl, w + L.tree_off, m.status,
+                                     lsd_flag, m.form, s, &sorted, rec),
+              "build: sort");
+    else
+      OCT_TRY(launch_sort_passes_split(keys_a, keys_b, &L.sort, sort_ctrl, m.status,
+                                       msd ? m.form : nullptr, lsd_flag, s, &sorted, rec),
+              "build: sort");
   }
   if (msd) {
     OCT_TRY(launch_msd_buckets(keys_b, keys_a, top_base, top_hist, w + L.msd_off, m.msd, m.form,

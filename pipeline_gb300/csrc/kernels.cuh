@@ -133,6 +133,7 @@ struct DigitAlt {
   int shift = 0;
   const uint32_t* base = nullptr;
   uint32_t* part = nullptr;
+  uint32_t* low = nullptr;  // cursors of the pass's own digit where the flag is not set
 };
 constexpr int kCursorStride = 16;
 cudaError_t launch_pass(const SortPlan& p, bool stable, const uint32_t* src, uint32_t* dst,
@@ -163,10 +164,18 @@ cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* w
 // Whether build stages 2-3 of this plan run without digit passes: the one-launch
 // sort, whose scratch lies in parts of the plan's that the passes would use.
 bool sort_once_in_plan(const SortPlan& p);
-// That sort: keys in place; gate: nullptr, or a device flag whose 0 returns at
-// once. ctrl: the plan's control block, its zeroed part cleared.
+// That sort, keys in place. ctrl: the plan's control block, its zeroed part cleared.
 cudaError_t launch_sort_once_in_plan(uint32_t* keys, uint32_t* alt, const SortPlan& p, void* ctrl,
-                                     uint32_t* status, const uint32_t* gate, cudaStream_t s);
+                                     uint32_t* status, cudaStream_t s);
+// Digit passes of a default 30-bit plan that run where the device flag gate is
+// set, in few launches. msd_flag: nullptr, or the flag that makes the first pass
+// the MSD form's scatter (the plan's top digit is counted). ctrl: as above;
+// lookback: sort_few_lookback_bytes(n), 16-byte aligned, any contents. *result: alt.
+size_t sort_few_lookback_bytes(int n);
+cudaError_t launch_sort_passes_few(uint32_t* keys, uint32_t* alt, const SortPlan* plan, void* ctrl,
+                                   void* lookback, uint32_t* status, const uint32_t* gate,
+                                   const uint32_t* msd_flag, cudaStream_t s, uint32_t** result,
+                                   Recorder* rec = nullptr);
 
 // The keys of a batch's clouds from their top-digit buckets in src to sorted
 // order in dst (batch_sort.cu).
@@ -211,10 +220,6 @@ bool msd_plan_ok(const SortPlan& p);  // 10-bit digits, 3 passes, reduce-then-sc
 // top_base: nullptr, or the buckets' first positions, to be written.
 cudaError_t launch_msd_gate(const uint32_t* top_hist, int n, uint32_t* flags, void* scratch,
                             uint32_t* top_base, cudaStream_t s);
-// The top-digit scatter keys -> alt alone (base: written by the gate kernel).
-cudaError_t launch_msd_scatter(const uint32_t* keys, uint32_t* alt, const SortPlan* plan,
-                               void* ctrl, uint32_t* status, const uint32_t* msd_flag,
-                               cudaStream_t s);
 // The sorted unique keys of every item, one run each in `runs`; counters: two
 // zeroed words.
 cudaError_t launch_msd_buckets(const uint32_t* keys, uint32_t* runs, const uint32_t* top_base,

@@ -546,18 +546,16 @@ constexpr int kSoMaxGated = 1 << 24;
 
 bool sort_once_in_plan(const SortPlan& p) {
   const SoLayout L = so_layout(p.n);
-  return sort_once_takes(p.n, kSoMaxGated) && msd_plan_ok(p) &&
+  return sort_once_takes(p.n, kSoMaxN) && msd_plan_ok(p) &&
          p.zero_bytes - p.tile_part_off >= 2 * align_up(L.zero_bytes, 256) &&
          p.bytes - p.tile_hist_off >= L.total - L.zero_bytes;
 }
 
 cudaError_t launch_sort_once_in_plan(uint32_t* keys, uint32_t* alt, const SortPlan& p, void* ctrl,
-                                     uint32_t* status, const uint32_t* gate, cudaStream_t s) {
-  // the first digit's split sums (the MSD form's cursors are the last's) and
-  // the tile histograms
-  char* c = static_cast<char*>(ctrl);
+                                     uint32_t* status, cudaStream_t s) {
+  char* c = static_cast<char*>(ctrl);  // the split sums and the tile histograms
   return launch_sort_once(keys, alt, p.n, 30, 30, c + p.tile_part_off, c + p.tile_hist_off, status,
-                          s, gate, true);
+                          s, nullptr, true);
 }
 
 size_t sort_keys_gated_zero_bytes(int n) {

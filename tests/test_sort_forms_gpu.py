@@ -117,3 +117,27 @@ def test_few_values_sort_like_torch(kind, n):
         alt, status = torch.empty_like(keys), torch.zeros(1, dtype=torch.int32, device="cuda")
         k_SimpleRadixSort(keys, alt, n, key_bits=bits, status=status)
         assert int(status[0]) == 0 and torch.equal(keys, want)
+
+
+def build_us(pts):
+    from pipeline_gb300.pipeline import OctreeBuilder
+
+    b = OctreeBuilder(pts.shape[0])
+    return best_us(lambda: b.build(pts, 0.0, 1024.0), 10)
+
+
+@pytest.mark.parametrize("kind", ["two values", "one octant"])
+@pytest.mark.parametrize("n", [4_300_000, 8_300_000, 16_700_000])
+def test_builds_of_clouds_that_the_msd_form_refuses(kind, n):
+    g = torch.Generator(device="cuda").manual_seed(2)
+    c = torch.randint(0, 1 << 30, (n,), generator=g, device="cuda")
+    if kind == "two values":
+        share = torch.rand(n, generator=g, device="cuda")
+        c = torch.where(share < 0.45, 123_456_789, torch.where(share < 0.9, 987_654_321, c))
+    else:
+        c = (9 << 18) + c % (1 << 18)
+    pts = points(c)
+    del c
+    with passes():
+        want = build_us(pts)
+    assert build_us(pts) < MARGIN * want

@@ -393,8 +393,7 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
   // mostly do not run: up to 2^24 points they are three launches that return at
   // once, and the Morton kernel counts the top digit only.
   const bool msd = n >= msd_min_n() && msd_plan_ok(L.sort);
-  const SortConfig cfg = L.sort.cfg, def = kSortConfigDefault;
-  const bool few = msd && n <= 1 << 24 && cfg.warps == def.warps && cfg.items == def.items;
+  const bool few = msd && sort_few_ok(L.sort);
   char* sort_ctrl = w + L.sort_off;
   const size_t top_row = (size_t)(L.sort.passes - 1) * L.sort.bins;
   const uint32_t* top_hist = reinterpret_cast<const uint32_t*>(sort_ctrl + L.sort.hist_off) + top_row;

@@ -876,7 +876,8 @@ cudaError_t launch_lsort(const float4* pts, uint32_t* keys, int n, float min_coo
   if (e != cudaSuccess) return e;
   // Fallback: sort + unique on the original keys, gated on the flag.
   uint32_t* sorted = keys;
-  e = launch_sort_keys_gated(keys, alt, n, ws + p.sort_ctrl_off, status, gate, s, &sorted);
+  // (the look-back words: the buckets' keys are not needed any more)
+  e = launch_sort_keys_gated(keys, alt, n, ws + p.sort_ctrl_off, bkeys, status, gate, s, &sorted);
   if (e != cudaSuccess) return e;
   e = launch_unique_gated(sorted, out, n, d_unique, &p.fallback_unique, ws + p.uniq_ctrl_off,
                           status, gate, s);

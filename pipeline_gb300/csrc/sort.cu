@@ -881,6 +881,13 @@ static int few_tiles(int n) {
   const int tile = kFewConfig.warps * 32 * kFewConfig.items;
   return (n + tile - 1) / tile;
 }
+// Larger arrays lose more by the look-back than the launches cost.
+static constexpr int kFewMaxN = 1 << 24;
+bool sort_few_ok(const SortPlan& p) {
+  const SortConfig d = kSortConfigDefault;
+  return msd_plan_ok(p) && p.cfg.warps == d.warps && p.cfg.items == d.items && p.n > 1 &&
+         p.n <= kFewMaxN;
+}
 size_t sort_few_lookback_bytes(int n) { return 2 * sizeof(uint32_t) * 1024 * (size_t)few_tiles(n); }
 
 cudaError_t launch_sort_passes_few(uint32_t* keys, uint32_t* alt, const SortPlan* plan, void* ctrl,

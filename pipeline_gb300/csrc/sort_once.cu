@@ -538,12 +538,6 @@ cudaError_t launch_diag_grid_wait(void* workspace, uint32_t* status, unsigned lo
              : e;
 }
 
-// A sort that mostly does not run (gate 0) is chosen by what its return costs:
-// one launch instead of eleven, 5 us instead of 32 behind a learned sort that
-// fits (whole build of 16.7M points 867 -> 823 us, of 239,010 points 196 ->
-// 157).
-constexpr int kSoMaxGated = 1 << 24;
-
 bool sort_once_in_plan(const SortPlan& p) {
   const SoLayout L = so_layout(p.n);
   return sort_once_takes(p.n, kSoMaxN) && msd_plan_ok(p) &&
@@ -564,14 +558,18 @@ size_t sort_keys_gated_zero_bytes(int n) {
 
 size_t sort_keys_gated_bytes(int n) {
   const size_t least = std::max(sort_plan(n, 30).bytes, sort_keys_gated_zero_bytes(n));
-  return n > 1 && n <= kSoMaxGated ? std::max(least, so_layout(n).total) : least;
+  return n > 1 && n <= kSoMaxN ? std::max(least, so_layout(n).total) : least;
 }
 
+// A sort that mostly does not run (gate 0) should cost little then: one launch,
+// or four where that is the slower sort, instead of eleven (5, 14 and 32 us
+// behind a learned sort that fits; whole build of 239,010 points 196 -> 157, of
+// 16.7M 867 -> 829).
 cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* workspace,
-                                   uint32_t* status, const uint32_t* gate, cudaStream_t s,
-                                   uint32_t** result) {
+                                   void* lookback, uint32_t* status, const uint32_t* gate,
+                                   cudaStream_t s, uint32_t** result) {
   *result = keys;
-  if (sort_once_takes(n, kSoMaxGated)) {
+  if (sort_once_takes(n, kSoMaxN)) {
     const cudaError_t e = launch_sort_once(
         keys, alt, n, 30, 30, workspace, static_cast<char*>(workspace) + so_layout(n).zero_bytes,
         status, s, gate, true);
@@ -579,6 +577,9 @@ cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* w
     (void)cudaGetLastError();
   }
   const SortPlan p = sort_plan(n, 30);
+  if (sort_few_ok(p))
+    return launch_sort_passes_few(keys, alt, &p, workspace, lookback, status, gate, nullptr, s,
+                                  result);
   const cudaError_t e = launch_histogram_gated(keys, &p, workspace, gate, s);
   return e == cudaSuccess
              ? launch_sort_passes_gated(keys, alt, &p, workspace, status, gate, s, result)

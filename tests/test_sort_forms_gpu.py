@@ -141,3 +141,35 @@ def test_builds_of_clouds_that_the_msd_form_refuses(kind, n):
     with passes():
         want = build_us(pts)
     assert build_us(pts) < MARGIN * want
+
+
+@pytest.mark.parametrize("kind", ["nine tenths", "one bucket"])
+@pytest.mark.parametrize("n", [1_000_000, 8_300_000, 16_700_000])
+def test_learned_builds_whose_model_does_not_fit(kind, n):
+    """The fall-back runs, and costs no more than by passes; the tree is the plain build's."""
+    from pipeline_gb300.learned import LearnedCDF
+    from pipeline_gb300.pipeline import LearnedOctreeBuilder, OctreeBuilder
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    other = torch.randint(0, 1 << 30, (100_000,), generator=g, device="cuda").to(torch.int32)
+    model = LearnedCDF(1024).fit(other, n_segments=1024, steps=20, n_buckets=4096)
+    pts = points(codes(kind, n))
+
+    def built():
+        b = LearnedOctreeBuilder(n, model)
+        us = best_us(lambda: b.build(pts, 0.0, 1024.0), 10)
+        return us, b
+
+    with passes():
+        want, _ = built()
+    got, b = built()
+    assert b.lsort_stats()["fallback"] == 1
+    assert got < MARGIN * want
+    result = b.result()
+    del b
+    plain = OctreeBuilder(n)
+    plain.build(pts, 0.0, 1024.0)
+    want = plain.result()
+    assert result["status"] == want["status"] == 0
+    for key in ("sorted_unique", "parent", "prefix_sum", "oct_nodes"):
+        assert result[key].tobytes() == want[key].tobytes(), key

@@ -154,7 +154,7 @@ cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits,
                              uint32_t* status, cudaStream_t s);
 // The sort of 30-bit keys that runs only where the device flag gate is set;
 // workspace: sort_keys_gated_bytes(n), its first sort_keys_gated_zero_bytes(n)
-// zeroed; lookback: sort_few_lookback_bytes(n), any contents; *result: keys or alt.
+// zeroed; lookback: n words, any contents; *result: keys or alt.
 size_t sort_keys_gated_bytes(int n);
 size_t sort_keys_gated_zero_bytes(int n);
 cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* workspace,
@@ -167,12 +167,12 @@ bool sort_once_in_plan(const SortPlan& p);
 // That sort, keys in place. ctrl: the plan's control block, its zeroed part cleared.
 cudaError_t launch_sort_once_in_plan(uint32_t* keys, uint32_t* alt, const SortPlan& p, void* ctrl,
                                      uint32_t* status, cudaStream_t s);
-// Digit passes of a default 30-bit plan (sort_few_ok) that run where the device
-// flag gate is set, in few launches. msd_flag: nullptr, or the flag that makes the first pass
-// the MSD form's scatter (the plan's top digit is counted). ctrl: as above;
-// lookback: sort_few_lookback_bytes(n), 16-byte aligned, any contents. *result: alt.
+// Digit passes of a plan of the default shape (sort_few_ok) that run where the
+// device flag gate is set, in few launches. msd_flag: nullptr, or the flag that
+// makes the first pass the MSD form's scatter (the plan's top digit is counted).
+// ctrl: as above; lookback: 16-byte aligned, any contents. *result: keys or alt.
 bool sort_few_ok(const SortPlan& p);
-size_t sort_few_lookback_bytes(int n);
+size_t sort_few_lookback_bytes(const SortPlan& p);
 cudaError_t launch_sort_passes_few(uint32_t* keys, uint32_t* alt, const SortPlan* plan, void* ctrl,
                                    void* lookback, uint32_t* status, const uint32_t* gate,
                                    const uint32_t* msd_flag, cudaStream_t s, uint32_t** result,

@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(256)
 // The same for passes that mostly do not run (one launch in place of three): the
 // CTA that is done last scans all the plan's digits into their bases, and the
 // look-back words are cleared. ticket: a zeroed word.
+template <int RB>
 __global__ void __launch_bounds__(256)
     histogram_bases_kernel(const uint32_t* __restrict__ keys, int n, uint32_t* ghist, int counted,
                            int passes, uint32_t* __restrict__ base, uint32_t* ticket,
@@ -128,12 +129,12 @@ __global__ void __launch_bounds__(256)
                            const uint32_t* __restrict__ gate) {
   chain_enter();
   if (*gate == 0) return;
-  constexpr int BINS = 1024, PER = BINS / 256;
+  constexpr int BINS = 1 << RB, PER = BINS / 256;
   extern __shared__ uint32_t s_hist[];
   __shared__ uint32_t warp_tot[32], total, s_last;
   for (int i = blockIdx.x * 256 + threadIdx.x; i < lookback4; i += gridDim.x * 256)
     lookback[i] = make_uint4(0u, 0u, 0u, 0u);
-  add_histograms<10>(keys, n, ghist, counted, s_hist);
+  add_histograms<RB>(keys, n, ghist, counted, s_hist);
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1u;
@@ -876,25 +877,25 @@ cudaError_t launch_sort_passes_split(uint32_t* keys, uint32_t* alt, const SortPl
 // cursors, two look-back passes over 12,288-key tiles. Against ten launches of
 // the tile-scan form the sort is as fast at 4.3M keys (154 us) and at 8.4M (249
 // and 246), 7% slower at 16.7M (447 and 417).
-static constexpr SortConfig kFewConfig = {10, 16, 24, 0};
 static int few_tiles(int n) {
-  const int tile = kFewConfig.warps * 32 * kFewConfig.items;
-  return (n + tile - 1) / tile;
+  constexpr int kTile = 16 * 32 * 24;
+  return (n + kTile - 1) / kTile;
 }
 // Larger arrays lose more by the look-back than the launches cost.
 static constexpr int kFewMaxN = 1 << 24;
 bool sort_few_ok(const SortPlan& p) {
   const SortConfig d = kSortConfigDefault;
-  return msd_plan_ok(p) && p.cfg.warps == d.warps && p.cfg.items == d.items && p.n > 1 &&
+  return p.cfg.scan == d.scan && p.cfg.warps == d.warps && p.cfg.items == d.items && p.n > 1 &&
          p.n <= kFewMaxN;
 }
-size_t sort_few_lookback_bytes(int n) { return 2 * sizeof(uint32_t) * 1024 * (size_t)few_tiles(n); }
+size_t sort_few_lookback_bytes(const SortPlan& p) {
+  return align_up(sizeof(uint32_t) * (size_t)(p.passes - 1) * p.bins * few_tiles(p.n), 16);
+}
 
 cudaError_t launch_sort_passes_few(uint32_t* keys, uint32_t* alt, const SortPlan* plan, void* ctrl,
                                    void* lookback, uint32_t* status, const uint32_t* gate,
                                    const uint32_t* msd_flag, cudaStream_t s, uint32_t** result,
                                    Recorder* rec) {
-  *result = alt;
   char* c = static_cast<char*>(ctrl);
   uint32_t* hist = reinterpret_cast<uint32_t*>(c + plan->hist_off);
   uint32_t* base = reinterpret_cast<uint32_t*>(c + plan->base_off);
@@ -905,9 +906,10 @@ cudaError_t launch_sort_passes_few(uint32_t* keys, uint32_t* alt, const SortPlan
   // (with the MSD form beside, the top digit is counted already)
   const int counted = msd_flag ? top : plan->passes;
   cudaError_t e = launch_chained(
-      histogram_bases_kernel, dim3(ctas), dim3(256), sizeof(uint32_t) * 1024 * counted, s, keys,
-      plan->n, hist, counted, plan->passes, base, counters + 32,
-      reinterpret_cast<uint4*>(lookback), (int)(sort_few_lookback_bytes(plan->n) / 16), gate);
+      plan->radix_bits == 10 ? histogram_bases_kernel<10> : histogram_bases_kernel<8>, dim3(ctas),
+      dim3(256), sizeof(uint32_t) * plan->bins * counted, s, keys, plan->n, hist, counted,
+      plan->passes, base, counters + 32, reinterpret_cast<uint4*>(lookback),
+      (int)(sort_few_lookback_bytes(*plan) / 16), gate);
   if (e != cudaSuccess) return e;
   mark(rec, s);
   DigitAlt a0;
@@ -918,21 +920,28 @@ cudaError_t launch_sort_passes_few(uint32_t* keys, uint32_t* alt, const SortPlan
     a0.base = base + (size_t)top * plan->bins;
     a0.part = part + (size_t)top * kScanSplits * plan->bins;
   }
-  e = launch_pass(*plan, false, keys, alt, 0, base, nullptr, counters,
-                  reinterpret_cast<uint32_t*>(c + plan->tile_hist_off), status,
-                  msd_flag ? nullptr : gate, s, nullptr, 0, a0);
-  if (e != cudaSuccess) return e;
-  mark(rec, s);
   SortPlan few = *plan;
-  few.cfg = kFewConfig;
+  few.cfg.items = 24;
+  few.cfg.scan = 0;
   const int grid = std::min(ctas, few_tiles(plan->n));
-  for (int p = 1; p <= 2; ++p) {
-    e = launch_pass(few, true, p == 1 ? alt : keys, p == 1 ? keys : alt, p * plan->radix_bits,
-                    base + p * plan->bins, lb + (size_t)(p - 1) * 1024 * few_tiles(plan->n),
-                    counters + p, nullptr, status, gate, s, nullptr, grid);
+  uint32_t* a = keys;
+  uint32_t* b = alt;
+  for (int p = 0; p < plan->passes; ++p) {
+    if (p == 0)
+      e = launch_pass(*plan, false, a, b, 0, base, nullptr, counters,
+                      reinterpret_cast<uint32_t*>(c + plan->tile_hist_off), status,
+                      msd_flag ? nullptr : gate, s, nullptr, 0, a0);
+    else
+      e = launch_pass(few, true, a, b, p * plan->radix_bits, base + p * plan->bins,
+                      lb + (size_t)(p - 1) * plan->bins * few_tiles(plan->n), counters + p,
+                      nullptr, status, gate, s, nullptr, grid);
     if (e != cudaSuccess) return e;
     mark(rec, s);
+    uint32_t* t = a;
+    a = b;
+    b = t;
   }
+  *result = a;
   return cudaSuccess;
 }
 

@@ -20,8 +20,8 @@
 //
 // Equal keys are alike, so their order is free: unless a key has bits above
 // key_bits, which the sort passes over. Such keys, and buckets beyond the
-// limits above (a few values that hold much of a large array, which a look at
-// 1,024 keys finds first), take stable 8-bit digit passes inside the same launch.
+// limits above (a few values that hold much of a large array), take stable 8-bit
+// digit passes inside the same launch, or are left to passes behind it.
 //
 // Measured against the launched digit passes, us: 20,000 even 32-bit keys 99 ->
 // 20, 130,000 99 -> 22, 1,048,576 102 -> 33, 4M 157 -> 75; Morton codes of points
@@ -48,21 +48,28 @@ constexpr int kSoMaxGrid = 256;
 constexpr int kSoMaxCluster = 8;
 constexpr int kSoStretch = 14336; // positions whose buckets are sorted together (mostly at once)
 constexpr int kSoMinPer = 1024;   // keys per CTA at least
-// Larger arrays take the launched passes, which uneven keys, and keys of a few
-// values above all, are sorted faster by (8.4M Morton codes around 64 centres 235
-// us and 242 here, ten values that hold nine tenths 223 and 292) although even
-// ones are not (232 and 160). Up to the line none of 20 distributions is slower here
-// by more than 3%: 4M keys, even 157 and 75, codes around 64 centres 155 and 132,
-// a cloud a sixteenth of its box thick 155 and 116, a few values 146 to 164 and 141
-// to 144. (Just past it clouds a sixteenth of their box thick lose an eighth: 256
-// buckets about as large as a CTA sorts, some of which are split.)
-constexpr int kSoMaxN = 4000000;
-// Keys of which a few values hold much go through the digit passes in here at
-// once, not after two counts, 20 us of 155 at 4M: 1,024 keys of the array tell, of
-// which more than kSoFew are alike in all but 12 bits (the passes lose nothing to
-// the buckets' form on such keys). Fewer than kSoLook keys lose little.
+// Up to kSoAny keys the launch sorts whatever it is given: none of 20 distributions
+// is slower than by launched passes by more than 3% (4M keys: even 157 us by passes
+// and 75 here, codes around 64 centres 155 and 132, a cloud a sixteenth of its box
+// thick 155 and 116, a few values 146 to 164 and 141 to 144). Beyond, passes are
+// faster for uneven keys (8.4M: codes around 64 centres 235 and 242, ten values
+// that hold nine tenths 223 and 292), but not for even ones (232 and 160): up to
+// kSoEven the launch leaves keys that a look finds uneven to passes behind it, which
+// otherwise are four launches that return at once (even 232 and 190; uneven within
+// 1% of the passes alone). Larger arrays take passes alone (16.7M: even keys would
+// gain an eighth, uneven ones lose 4%).
+constexpr int kSoAny = 4000000;
+constexpr int kSoEven = 1 << 23;
+// The look: 1,024 keys of the array. Few values hold much of it if more than kSoFew
+// are alike in all but 12 bits; such keys take the digit passes in here at once, not
+// after two counts (20 us of 155 at 4M; fewer than kSoLook keys lose little). It is
+// uneven, for kSoEven, if more than kSoTopMost are alike in the top 10 bits or
+// kSoPairs meet another in a cell of 2^12 values (even keys: 32 by the table's size).
 constexpr int kSoLook = 1 << 21;
 constexpr uint32_t kSoFew = 16;
+constexpr uint32_t kSoTopMost = 14;
+constexpr int kSoPairs = 80;
+constexpr int kSoCellBits = 14;
 
 struct SoLayout {
   size_t hist_off, zero_bytes, ids_off, mat_off, total;
@@ -95,6 +102,7 @@ struct SoArgs {
   uint32_t* mat;   // [2][grid][kRsBins]
   uint32_t* status;
   const uint32_t* gate;  // device flag: 0 returns at once
+  uint32_t* defer;  // nullptr, or a zeroed flag: keys left to passes set it
 };
 
 struct SoSmem {
@@ -198,11 +206,24 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
   bool lsd = false;
   if (A.n > kSoLook) {  // (every CTA looks at the same keys)
     const uint32_t k = A.keys[(unsigned long long)tid * n / kSoThreads];
+    const uint32_t hash = (k >> 12) * 0x9e3779b1u;
     for (int b = tid; b < kSoTop; b += kSoThreads) M.tab[b] = 0u;
+    for (int b = tid; A.defer && b < 1 << kSoCellBits; b += kSoThreads) M.ab[b] = 0u;
     __syncthreads();
-    const uint32_t cell = ((k >> 12) * 0x9e3779b1u) >> (32 - kSoTopBits);
-    lsd = __syncthreads_or(atomicAdd(&M.tab[cell], 1u) >= kSoFew) != 0;
+    if (A.defer) {
+      const uint32_t top = (k >> max(A.key_bits - 10, 0)) & 1023u;
+      const bool met = atomicAdd(&M.ab[hash >> (32 - kSoCellBits)], 1u) > 0u;
+      lsd = __syncthreads_or(atomicAdd(&M.tab[top], 1u) >= kSoTopMost) != 0;
+      lsd |= __syncthreads_count(met) >= kSoPairs;
+    } else {
+      lsd = __syncthreads_or(atomicAdd(&M.tab[hash >> (32 - kSoTopBits)], 1u) >= kSoFew) != 0;
+    }
   }
+  auto deferred = [&]() {
+    if (lsd && A.defer && cta == 0 && tid == 0) *A.defer = 1u;
+    return lsd && A.defer;
+  };
+  if (deferred()) return;
 
   // ---- count
   for (int b = tid; b < kSoTop; b += kSoThreads) base[b] = 0u;
@@ -303,6 +324,7 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
     }
   }
   __syncthreads();
+  if (deferred()) return;
 
   if (!lsd) {
     // ---- scatter
@@ -448,7 +470,8 @@ __global__ void __launch_bounds__(kSoThreads, 1) sort_once_kernel(SoArgs A) {
 static cudaError_t launch_sort_once(uint32_t* keys, uint32_t* alt, int n, int key_bits,
                                     int low_bits, void* zeroed, void* rest, uint32_t* status,
                                     cudaStream_t s, const uint32_t* gate = nullptr,
-                                    bool cleared = false, uint32_t absent = 0,
+                                    bool cleared = false, uint32_t* defer = nullptr,
+                                    uint32_t absent = 0,
                                     unsigned long long limit_ns = kWaitLimitNs) {
   const SoLayout L = so_layout(n);
   char* w = static_cast<char*>(zeroed);
@@ -467,6 +490,7 @@ static cudaError_t launch_sort_once(uint32_t* keys, uint32_t* alt, int n, int ke
   A.mat = reinterpret_cast<uint32_t*>(r + L.mat_off);
   A.status = status;
   A.gate = gate;
+  A.defer = defer;
   const int smem = (int)sizeof(SoSmem);
   const bool cluster = L.grid <= kSoMaxCluster;
   auto kernel = cluster ? sort_once_kernel<true> : sort_once_kernel<false>;
@@ -497,25 +521,59 @@ static bool sort_once_takes(int n, int most) {
          c.items == d.items && c.scan == d.scan;
 }
 
+// Past kSoAny: the launch's zeroed scratch and the plan's control block, cleared
+// together, then the rest of the launch's scratch and the look-back words (past
+// kSoEven as much beside the plan as there, so that more keys never need less).
 size_t sort_keys_bytes(int n, int key_bits) {
   const size_t plan = sort_plan(n, key_bits).bytes;
-  return n > 1 && n <= kSoMaxN ? std::max(plan, so_layout(n).total) : plan;
+  if (n <= 1) return plan;
+  const int m = std::min(n, kSoEven);
+  const size_t once = so_layout(m).total;
+  return n <= kSoAny ? std::max(plan, once)
+                     : once + align_up(plan, 256) + sort_few_lookback_bytes(sort_plan(m, key_bits));
+}
+
+__global__ void __launch_bounds__(1024)
+    copy_gated_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int n,
+                      const uint32_t* __restrict__ gate) {
+  chain_enter();
+  if (*gate == 0u) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    dst[i] = src[i];
 }
 
 cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits, void* workspace,
                              uint32_t* status, cudaStream_t s) {
   const SortPlan p = sort_plan(n, key_bits);
-  if (sort_once_takes(n, kSoMaxN)) {
+  const SoLayout L = so_layout(n);
+  const int low_bits = std::min(32, p.passes * p.radix_bits);
+  char* w = static_cast<char*>(workspace);
+  uint32_t* result = keys;
+  if (sort_once_takes(n, kSoAny)) {
     const cudaError_t e =
-        launch_sort_once(keys, alt, n, key_bits, std::min(32, p.passes * p.radix_bits), workspace,
-                         static_cast<char*>(workspace) + so_layout(n).zero_bytes, status, s);
+        launch_sort_once(keys, alt, n, key_bits, low_bits, w, w + L.zero_bytes, status, s);
     if (e != cudaErrorCooperativeLaunchTooLarge) return e;
     (void)cudaGetLastError();  // a context with fewer SMs: the passes
+  } else if (sort_once_takes(n, kSoEven) && sort_few_ok(p)) {
+    char* plan = w + align_up(L.zero_bytes, 256);
+    char* rest = plan + align_up(p.bytes, 256);
+    uint32_t* defer = reinterpret_cast<uint32_t*>(w) + 3;
+    cudaError_t e = cudaMemsetAsync(w, 0, (size_t)(plan - w) + p.zero_bytes, s);
+    if (e == cudaSuccess)
+      e = launch_sort_once(keys, alt, n, key_bits, low_bits, w, rest, status, s, nullptr, true,
+                           defer);
+    if (e == cudaSuccess)
+      e = launch_sort_passes_few(keys, alt, &p, plan, rest + (L.total - L.zero_bytes), status,
+                                 defer, nullptr, s, &result);
+    if (e == cudaSuccess && result != keys)
+      e = launch_chained(copy_gated_kernel, dim3(device_sm_count() * 2), dim3(1024), 0, s, result,
+                         keys, n, defer);
+    if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+    (void)cudaGetLastError();
   }
-  cudaError_t e = cudaMemsetAsync(workspace, 0, p.zero_bytes, s);
-  if (e == cudaSuccess) e = launch_histogram(keys, &p, workspace, s);
-  uint32_t* result = keys;
-  if (e == cudaSuccess) e = launch_sort_passes(keys, alt, &p, workspace, status, s, &result);
+  cudaError_t e = cudaMemsetAsync(w, 0, p.zero_bytes, s);
+  if (e == cudaSuccess) e = launch_histogram(keys, &p, w, s);
+  if (e == cudaSuccess) e = launch_sort_passes(keys, alt, &p, w, status, s, &result);
   if (e == cudaSuccess && result != keys)
     e = cudaMemcpyAsync(keys, result, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToDevice, s);
   return e;
@@ -534,13 +592,13 @@ cudaError_t launch_diag_grid_wait(void* workspace, uint32_t* status, unsigned lo
   return e == cudaSuccess
              ? launch_sort_once(keys, alt, kSoDiagKeys, 30, 30, w,
                                 w + so_layout(kSoDiagKeys).zero_bytes, status, s, nullptr, false,
-                                1u, limit_ns)
+                                nullptr, 1u, limit_ns)
              : e;
 }
 
 bool sort_once_in_plan(const SortPlan& p) {
   const SoLayout L = so_layout(p.n);
-  return sort_once_takes(p.n, kSoMaxN) && msd_plan_ok(p) &&
+  return sort_once_takes(p.n, kSoAny) && msd_plan_ok(p) &&
          p.zero_bytes - p.tile_part_off >= 2 * align_up(L.zero_bytes, 256) &&
          p.bytes - p.tile_hist_off >= L.total - L.zero_bytes;
 }
@@ -558,7 +616,7 @@ size_t sort_keys_gated_zero_bytes(int n) {
 
 size_t sort_keys_gated_bytes(int n) {
   const size_t least = std::max(sort_plan(n, 30).bytes, sort_keys_gated_zero_bytes(n));
-  return n > 1 && n <= kSoMaxN ? std::max(least, so_layout(n).total) : least;
+  return n > 1 && n <= kSoAny ? std::max(least, so_layout(n).total) : least;
 }
 
 // A sort that mostly does not run (gate 0) should cost little then: one launch,
@@ -569,7 +627,7 @@ cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* w
                                    void* lookback, uint32_t* status, const uint32_t* gate,
                                    cudaStream_t s, uint32_t** result) {
   *result = keys;
-  if (sort_once_takes(n, kSoMaxN)) {
+  if (sort_once_takes(n, kSoAny)) {
     const cudaError_t e = launch_sort_once(
         keys, alt, n, 30, 30, workspace, static_cast<char*>(workspace) + so_layout(n).zero_bytes,
         status, s, gate, true);

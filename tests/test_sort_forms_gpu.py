@@ -44,6 +44,10 @@ def codes(kind, n, seed=1):
         return (5 << 20) + some(1 << 20)
     if kind == "one value":
         return torch.full_like(even, low)
+    if kind == "even":
+        return even
+    if kind == "lumps":  # even at the top, not below
+        return (some(4096) << 18) + some(600)
     few = {"nine tenths": lambda: low, "ten values": lambda: some(10) * 100_000_007,
            "narrow": lambda: low + some(1 << 12)}[kind]()
     return torch.where(share < 0.9, few, even)
@@ -93,8 +97,8 @@ def sort_us(src, bits):
     return best_us(run, 10)
 
 
-@pytest.mark.parametrize("kind", ["nine tenths", "ten values", "narrow"])
-@pytest.mark.parametrize("n", [1_000_000, 3_900_000, 8_000_000])
+@pytest.mark.parametrize("kind", ["nine tenths", "ten values", "narrow", "lumps"])
+@pytest.mark.parametrize("n", [1_000_000, 3_900_000, 4_100_000, 8_000_000])
 def test_sorts_of_keys_of_a_few_values(kind, n):
     src = codes(kind, n).to(torch.int32)
     for bits in (30, 32):
@@ -103,11 +107,12 @@ def test_sorts_of_keys_of_a_few_values(kind, n):
         assert sort_us(src, bits) < MARGIN * want
 
 
-@pytest.mark.parametrize("kind", ["nine tenths", "ten values", "narrow", "one bucket", "one value"])
-@pytest.mark.parametrize("n", [(1 << 21) + 1, 3_999_999, 4_000_000, 4_000_001])
+@pytest.mark.parametrize("kind", ["even", "nine tenths", "ten values", "narrow", "one bucket",
+                                  "one value", "lumps"])
+@pytest.mark.parametrize("n", [(1 << 21) + 1, 4_000_000, 4_000_001, 1 << 23, (1 << 23) + 1])
 def test_few_values_sort_like_torch(kind, n):
-    """On both sides of the array sizes from which the keys are looked at first and
-    from which they take launched passes; with bits above key_bits as well."""
+    """On both sides of the array sizes from which the keys are looked at first, may be
+    left to passes, and take passes alone; with bits above key_bits as well."""
     from pipeline_gb300.kernels import k_SimpleRadixSort
 
     src = codes(kind, n).to(torch.int32)
@@ -173,3 +178,23 @@ def test_learned_builds_whose_model_does_not_fit(kind, n):
     assert result["status"] == want["status"] == 0
     for key in ("sorted_unique", "parent", "prefix_sum", "oct_nodes"):
         assert result[key].tobytes() == want[key].tobytes(), key
+
+
+def test_sort_that_may_be_left_to_passes_replayed_from_a_graph():
+    """One graph over keys that the one-launch sort takes, leaves after the look, and
+    leaves after its count (bits above key_bits in keys that look even)."""
+    from pipeline_gb300.kernels import k_SimpleRadixSort
+
+    n = 4_500_001
+    src = torch.zeros(n, dtype=torch.int32, device="cuda")
+    keys, alt = torch.empty_like(src), torch.empty_like(src)
+    k_SimpleRadixSort(keys.zero_(), alt, n, key_bits=30)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        keys.copy_(src)
+        k_SimpleRadixSort(keys, alt, n, key_bits=30)
+    for kind, above in (("even", 0), ("narrow", 0), ("even", 1 << 30), ("one value", 0), ("even", 0)):
+        src.copy_(codes(kind, n).to(torch.int32) + above)
+        graph.replay()
+        assert torch.equal(keys, torch.sort(src).values), (kind, above)

@@ -290,12 +290,13 @@ OCT_API int oct_build_octree(const oct_vec4* points, int n, float min_coord, flo
 #define OCT_SORT_FORM_LSD_FALLBACK 2
 OCT_API int oct_build_sort_form(const void* workspace, int n, int nodes_capacity, int* form);
 
-/* Timed build for measurement: the stage-by-stage launches (those of
- * oct_build_octree for clouds it does not build in one launch), with
- * caller-created CUDA events (cudaEvent_t, passed as void*) recorded on the
+/* Timed build for measurement: the stage-by-stage launches, those of
+ * oct_build_octree for clouds that it does not build in one launch (a cloud that
+ * it does is built stage by stage here), with caller-created CUDA events (cudaEvent_t, passed as void*) recorded on the
  * stream at each step boundary: events[k] after step k of
  * oct_build_step_name(k) for k < oct_build_step_count() (step 0 is the start).
- * Bench tooling derives per-kernel device times from consecutive events. */
+ * A sort without digit passes is timed as "sort pass 0"; a step that a build
+ * does not have takes no time. Bench tooling derives per-kernel device times from consecutive events. */
 OCT_API int oct_build_step_count(void);
 OCT_API const char* oct_build_step_name(int k);
 OCT_API int oct_build_octree_timed(const oct_vec4* points, int n, float min_coord, float range,

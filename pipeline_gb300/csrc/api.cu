@@ -400,18 +400,24 @@ static int build_impl(const oct_vec4* points, int n, float min_coord, float rang
   uint32_t* top_base = reinterpret_cast<uint32_t*>(sort_ctrl + L.sort.base_off) + top_row;
   const uint32_t* lsd_flag = msd ? m.form + 1 : nullptr;
   uint32_t* sorted = keys_a;
-  bool once = !rec && sort_once_in_plan(L.sort);
+  bool once = sort_once_in_plan(L.sort);
   if (once) {
+    mark(rec, s);
     OCT_TRY(cudaMemsetAsync(w, 0, L.ctrl_bytes, s), "build: clear");
+    mark(rec, s);
     OCT_TRY(launch_morton(reinterpret_cast<const float4*>(points), keys_a, n, min_coord, range,
                           nullptr, nullptr, m.status, s),
             "build: morton");
+    mark(rec, s);
+    mark(rec, s);  // no histogram scan
     const cudaError_t e = launch_sort_once_in_plan(keys_a, keys_b, L.sort, sort_ctrl, m.status, s);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       (void)cudaGetLastError();  // a context with fewer SMs: again with the passes
       once = false;
+      if (rec) rec->k = 0;
     } else {
       OCT_TRY(e, "build: sort");
+      for (int k = 0; k < 3; ++k) mark(rec, s);  // in place of three passes
     }
   }
   if (!once) {

@@ -69,6 +69,7 @@ constexpr int kFuMaxCluster = 8;                   // the portable cluster size
 constexpr int kFuMinPer = 1024;                    // points per CTA at least
 static_assert(kFuBuckets + 2 * (kFuMaxGrid * kFuShare / (int)kFuUnit) <= kFuIds,
               "a bucket of c codes has fewer than 2 c / kFuUnit parts");
+static_assert(kFuMaxCluster * kFuMinPer <= (int)kFuCut, "a cluster's codes need no cut");
 
 struct FusedLayout {
   size_t misc_off, hist_off, zero_bytes, ids_off, cta_off, keys_off, min_off, sum_off, d_off, tags_off,
@@ -250,6 +251,7 @@ __device__ uint32_t fused_bitmap_bucket(uint32_t* keys, uint32_t cnt, int bits, 
   return *total;
 }
 
+// CLUSTER: the grid is one cluster, and no bucket is cut.
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -258,12 +260,14 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
   __shared__ uint32_t s_cut[4];  // lo, hi, start of the straddling bucket
   __shared__ uint32_t s_off[kFuMaxGrid];
   __shared__ int s_next, s_ok;
+  __shared__ bool s_parts;
   const int tid = threadIdx.x, lane = tid & 31;
   const uint32_t G = gridDim.x, cta = blockIdx.x;
   uint32_t phase = 0;
 
   // ---- codes and bucket counts
   if (cta == 0 && tid < 4) A.d_counts[tid] = 0;
+  if (tid == 0) s_parts = false;  // (barriers follow)
   const int per = (int)(((uint32_t)A.n + G - 1u) / G);
   const int t0 = (int)min((long long)cta * per, (long long)A.n), t1 = min(t0 + per, A.n);
   uint32_t code[kFuItems];
@@ -280,7 +284,8 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
         *A.max_slot = 0;
       }
     }
-    for (int b = (int)cta * kFuThreads + tid; b < kFuIds; b += (int)G * kFuThreads) A.ids[b] = 0u;
+    for (int b = (int)cta * kFuThreads + tid; !CLUSTER && b < kFuIds; b += (int)G * kFuThreads)
+      A.ids[b] = 0u;
     fill_spread_lut(lut);
     // tile sums and minima start empty (used three barriers later)
     const int pad = (int)align_up((size_t)A.S.tiles, kTtMinBlock);
@@ -339,12 +344,13 @@ __global__ void __launch_bounds__(kFuThreads, 1) fused_build_kernel(FusedArgs A)
     static_assert(kPer == 4, "one 16-byte load of counts per thread");
     const uint4 q = reinterpret_cast<const uint4*>(A.hist)[tid];
     const uint32_t c[kPer] = {q.x, q.y, q.z, q.w};
+    if (max(max(c[0], c[1]), max(c[2], c[3])) > kFuCut) s_parts = true;
     const uint32_t ex =
         block_exclusive_sum<kFuThreads>(c[0] + c[1] + c[2] + c[3], s_warp, &s_total);
     const uint32_t kept = s_total;
     share = (kept + G - 1u) / G;
     const uint32_t w0 = min(cta * share, kept), w1 = min(w0 + share, kept);
-    parts = __syncthreads_or(max(max(c[0], c[1]), max(c[2], c[3])) > kFuCut) != 0;
+    parts = !CLUSTER && s_parts;  // (the sum's barriers)
     if (!parts) {
       fused_starts(M.s, c, ex, w0, w1, kept, s_cut);
     } else {

@@ -299,12 +299,6 @@ cudaError_t launch_tile_counts_scan(int tiles, const int* counts, uint32_t* pref
                                     const uint32_t* gate = nullptr);
 size_t tree_scratch_bytes_tiles(int tiles);
 TreeScratch tree_scratch_carve_tiles(void* base, int tiles);
-// Batched clouds: tiles {first, end, cloud, first tile of cloud} of 4,096
-// positions that never cross clouds; start[C+1]; U per cloud on the device.
-cudaError_t launch_batch_radix_tree(const int4* tiles, int n_tiles, const int* start,
-                                    const int* unique_c, const uint32_t* codes, uint8_t* prefix_n,
-                                    uint8_t* hll, uint8_t* hlr, int* left_child, int* parent,
-                                    int* ec, void* scratch, cudaStream_t s);
 cudaError_t launch_radix_tree_sorted(int n_host, const int* d_unique, const uint32_t* codes,
                                      uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr,
                                      int* left_child, int* parent, int* ec, void* scratch,

@@ -905,11 +905,15 @@ cudaError_t launch_sort_passes_few(uint32_t* keys, uint32_t* alt, const SortPlan
   const int top = plan->passes - 1, ctas = 2 * device_sm_count();
   // (with the MSD form beside, the top digit is counted already)
   const int counted = msd_flag ? top : plan->passes;
-  cudaError_t e = launch_chained(
-      plan->radix_bits == 10 ? histogram_bases_kernel<10> : histogram_bases_kernel<8>, dim3(ctas),
-      dim3(256), sizeof(uint32_t) * plan->bins * counted, s, keys, plan->n, hist, counted,
-      plan->passes, base, counters + 32, reinterpret_cast<uint4*>(lookback),
-      (int)(sort_few_lookback_bytes(*plan) / 16), gate);
+  const size_t sm = sizeof(uint32_t) * plan->bins * counted;
+  uint4* clear = static_cast<uint4*>(lookback);
+  const int words4 = (int)(sort_few_lookback_bytes(*plan) / 16);
+  cudaError_t e =
+      plan->radix_bits == 10
+          ? launch_chained(histogram_bases_kernel<10>, dim3(ctas), dim3(256), sm, s, keys, plan->n,
+                           hist, counted, plan->passes, base, counters + 32, clear, words4, gate)
+          : launch_chained(histogram_bases_kernel<8>, dim3(ctas), dim3(256), sm, s, keys, plan->n,
+                           hist, counted, plan->passes, base, counters + 32, clear, words4, gate);
   if (e != cudaSuccess) return e;
   mark(rec, s);
   DigitAlt a0;

@@ -449,19 +449,4 @@ cudaError_t launch_radix_tree_sorted(int n_host, const int* d_unique, const uint
                         codes, S, o);
 }
 
-cudaError_t launch_batch_radix_tree(const int4* tiles, int n_tiles, const int* start,
-                                    const int* unique_c, const uint32_t* codes, uint8_t* prefix_n,
-                                    uint8_t* hll, uint8_t* hlr, int* left_child, int* parent,
-                                    int* ec, void* scratch, cudaStream_t s) {
-  if (n_tiles <= 0) return cudaSuccess;
-  const TreeScratch S = tree_scratch_carve_tiles(scratch, n_tiles);
-  const CloudTiles map{tiles, start, unique_c};
-  cudaError_t e = launch_chained(tree_tiles_kernel<CloudTiles>, dim3(n_tiles), dim3(kTtAThreads), 0,
-                                 s, map, codes, S);
-  if (e != cudaSuccess) return e;
-  const TreeOut o{prefix_n, hll, hlr, left_child, parent, ec};
-  return launch_chained(tree_nodes_kernel<CloudTiles>, dim3(n_tiles), dim3(kTtBThreads), 0, s, map,
-                        codes, S, o);
-}
-
 }  // namespace octgb

@@ -346,7 +346,7 @@ OCT_API int oct_lcdf_buckets(const void* model, int max_segments, const uint32_t
  * n_buckets). Keys are scattered into model buckets and each bucket is sorted
  * and de-duplicated in shared memory; when more than overflow_threshold of the
  * keys sit in oversized buckets, or a bucket fits no shared-memory form, the
- * same launches fall back to the OneSweep sort + unique (device-side switch).
+ * same launches fall back to a plain sort + unique (device-side switch).
  * d_stats (nullable, 48 bytes): {fallback, failed_buckets, overflow_keys,
  * max_bucket, n, overflow_frac (float), skip, bitmap_buckets, radix_buckets,
  * bitonic_buckets, 0, 0}. On the fallback path `keys`

@@ -161,6 +161,10 @@ cudaError_t launch_sort_keys_gated(uint32_t* keys, uint32_t* alt, int n, void* w
                                    void* lookback, uint32_t* status, const uint32_t* gate,
                                    cudaStream_t s, uint32_t** result);
 
+// src to dst where the device flag gate is set.
+cudaError_t launch_copy_gated(const uint32_t* src, uint32_t* dst, int n, const uint32_t* gate,
+                              cudaStream_t s);
+
 // Whether build stages 2-3 of this plan run without digit passes: the one-launch
 // sort, whose scratch lies in parts of the plan's that the passes would use.
 bool sort_once_in_plan(const SortPlan& p);

@@ -25,7 +25,7 @@
 //
 // If any bucket fits neither form, the overflow fraction exceeds the
 // threshold, or the model's tables were built for another bucket count, the
-// device flag `fallback` is set and the OneSweep sort + unique (launched right
+// device flag `fallback` is set and a plain sort + unique (launched right
 // after, gated on the flag) redo stages 2-3 from the original keys; otherwise
 // those launches return at once. Either way the output is the sorted unique
 // key array, identical to the plain path's.
@@ -881,6 +881,8 @@ cudaError_t launch_lsort(const float4* pts, uint32_t* keys, int n, float min_coo
   if (e != cudaSuccess) return e;
   e = launch_unique_gated(sorted, out, n, d_unique, &p.fallback_unique, ws + p.uniq_ctrl_off,
                           status, gate, s);
+  if (e == cudaSuccess && !pts && sorted != keys)  // the caller's keys: sorted in place
+    e = launch_copy_gated(sorted, keys, n, gate, s);
   mark(rec, s);
   return e;
 }

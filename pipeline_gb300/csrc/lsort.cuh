@@ -7,7 +7,7 @@ namespace octgb {
 
 // Device-side statistics of one learned sort (in the zeroed workspace).
 struct LsortStats {
-  uint32_t fallback;        // 1: the OneSweep path produced the result
+  uint32_t fallback;        // 1: the plain sort produced the result
   uint32_t failed_buckets;  // buckets that fit neither bucket form
   uint32_t overflow_keys;   // keys in buckets above the bitonic capacity
   uint32_t max_bucket;      // largest bucket

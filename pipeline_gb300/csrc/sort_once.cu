@@ -542,6 +542,12 @@ __global__ void __launch_bounds__(1024)
     dst[i] = src[i];
 }
 
+cudaError_t launch_copy_gated(const uint32_t* src, uint32_t* dst, int n, const uint32_t* gate,
+                              cudaStream_t s) {
+  return launch_chained(copy_gated_kernel, dim3(device_sm_count() * 2), dim3(1024), 0, s, src, dst,
+                        n, gate);
+}
+
 cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits, void* workspace,
                              uint32_t* status, cudaStream_t s) {
   const SortPlan p = sort_plan(n, key_bits);
@@ -565,9 +571,7 @@ cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits,
     if (e == cudaSuccess)
       e = launch_sort_passes_few(keys, alt, &p, plan, rest + (L.total - L.zero_bytes), status,
                                  defer, nullptr, s, &result);
-    if (e == cudaSuccess && result != keys)
-      e = launch_chained(copy_gated_kernel, dim3(device_sm_count() * 2), dim3(1024), 0, s, result,
-                         keys, n, defer);
+    if (e == cudaSuccess && result != keys) e = launch_copy_gated(result, keys, n, defer, s);
     if (e != cudaErrorCooperativeLaunchTooLarge) return e;
     (void)cudaGetLastError();
   }

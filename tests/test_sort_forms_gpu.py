@@ -198,3 +198,22 @@ def test_sort_that_may_be_left_to_passes_replayed_from_a_graph():
         src.copy_(codes(kind, n).to(torch.int32) + above)
         graph.replay()
         assert torch.equal(keys, torch.sort(src).values), (kind, above)
+
+
+@pytest.mark.parametrize("digits", [False, True])
+@pytest.mark.parametrize("n", [100_001, 4_100_003])
+def test_lsort_fall_back_sorts_the_keys_in_place(n, digits):
+    """As the header promises, whichever sort the fall-back takes."""
+    from pipeline_gb300.learned import LearnedCDF
+    from pipeline_gb300.pipeline import lsort_unique
+
+    g = torch.Generator(device="cuda").manual_seed(6)
+    other = torch.randint(0, 1 << 30, (100_000,), generator=g, device="cuda").to(torch.int32)
+    model = LearnedCDF(1024).fit(other, n_segments=1024, steps=20, n_buckets=1024)
+    for kind in ("narrow", "one bucket"):
+        keys = codes(kind, n).to(torch.int32)
+        want = torch.sort(keys).values
+        with passes() if digits else contextlib.nullcontext():
+            unique, stats = lsort_unique(keys, model)
+        assert stats["fallback"] == 1
+        assert torch.equal(keys, want) and torch.equal(unique, torch.unique_consecutive(want))

@@ -498,11 +498,12 @@ def build_launches(n: int = 0) -> int:
     12,288 points per SM: one. Otherwise stages 2-3, then tree nodes, tile-sum
     scan + prefix sum (which clears the octree tags), octree emit/finalize and
     counts. Stages 2-3: Morton, the one-launch sort and unique (run-head count,
-    their scan, compaction with the deltas), from 2^22 points on with the MSD
-    form beside them (form gate, top-digit scatter, bucket bitmaps, pack scan +
-    pack); for other sort shapes and more than 2^24 points digit passes (base
-    scan, per pass a tile histogram + tile scan and the pass; the first doubles
-    as the top-digit scatter)."""
+    their scan, compaction with the deltas); past 4,000,000 points and for other
+    sort shapes digit passes in place of the one-launch sort (base scan, per
+    pass a tile histogram + tile scan and the pass), from 2^22 points on with the
+    MSD form beside them (form gate, bucket bitmaps, pack scan + pack; the first
+    pass doubles as the top-digit scatter), there up to 2^24 points as one
+    launch of counts and bases and three passes."""
     import torch
 
     from pipeline_gb300 import autotune
@@ -511,10 +512,15 @@ def build_launches(n: int = 0) -> int:
     if n and n <= 12288 * torch.cuda.get_device_properties(0).multi_processor_count:
         return 1
     passes = (30 + rb - 1) // rb
-    once = (rb, warps, items, scan) == (10, 16, 16, 1) and n <= (1 << 24)
-    sort = 1 if once else 1 + passes * (3 if scan == 1 else 1)
+    default = (rb, warps, items, scan) == (10, 16, 16, 1)
     msd = n >= (1 << 22) and rb == 10 and passes == 3 and scan == 1
-    return 1 + sort + 3 + (4 + once if msd else 0) + 1 + 2 + 2 + 1
+    if default and n <= 4_000_000:
+        sort = 1
+    elif default and msd and n <= (1 << 24):
+        sort = 1 + passes
+    else:
+        sort = 1 + passes * (3 if scan == 1 else 1)
+    return 1 + sort + 3 + (4 if msd else 0) + 1 + 2 + 2 + 1
 
 
 def profile_only(args):

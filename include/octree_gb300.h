@@ -366,8 +366,9 @@ OCT_API int oct_build_octree_learned(const oct_vec4* points, int n, float min_co
                                      oct_stream_t stream);
 /* Radix sort shape used by sort plans made after the call (the autotuner's
  * knob; shapes other than the default 10, 16, 16, 1 also keep digit passes
- * where the default takes one-launch and bucket sorts): radix_bits 10 or 8, warps 16, items 16 or 24, scan 0 (decoupled
- * look-back) or 1 (per-tile histograms + tile scan). */
+ * where the default takes one-launch and bucket sorts): radix_bits 10 or 8,
+ * warps 16, items 16 or 24, scan 0 (decoupled look-back) or 1 (per-tile
+ * histograms + tile scan). */
 OCT_API int oct_set_sort_config(int radix_bits, int warps, int items, int scan);
 OCT_API int oct_get_sort_config(int out[4]);
 

@@ -3,7 +3,8 @@
 Candidates are the sort configurations the library instantiates: digit width
 (10-bit: 3 passes over 30-bit Morton keys; 8-bit: 4 passes), keys per thread
 (16 or 24, i.e. tiles of 8192 or 12288 keys with 16 warps) and the tile-offset
-scheme (0: decoupled look-back, OneSweep; 1: per-tile histograms + tile scan).
+scheme (0: decoupled look-back; 1: per-tile histograms + tile scan). The default
+shape also lets the forms without digit passes run (one-launch and bucket sorts).
 ``tune`` times whole builds of the caller's workload under each candidate
 with CUDA events, applies the fastest (``oct_set_sort_config``) and records it
 in a JSON table keyed by workload kind and size class, so later processes

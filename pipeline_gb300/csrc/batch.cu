@@ -8,9 +8,11 @@
 //
 //   morton    tiles never cross clouds; each CTA walks a contiguous run of
 //             tiles and flushes its shared digit histograms per cloud;
-//   sort      reduce-then-scan radix passes: per-tile digit histograms, a
-//             per-cloud tile-prefix scan, and the pass kernel driven by tile
-//             descriptors (cloud-local positions are absolute indices);
+//   sort      clouds of at most 12,288 points: the top digit's scatter and the
+//             bucket sort (batch_sort.cu); else reduce-then-scan radix passes:
+//             per-tile digit histograms, a per-cloud tile-prefix scan, and the
+//             pass kernel driven by tile descriptors (cloud-local positions are
+//             absolute indices);
 //   unique    the single-cloud run-head count, one scan of all tiles' counts
 //             (a tile's offset is its entry minus that of its cloud's first
 //             tile) and the compaction that also writes each code's delta to
@@ -22,8 +24,8 @@
 //   scan      one scan of the tile sums for all clouds; a tile's prefix is its
 //             entry minus that of its cloud's first tile, so no tile waits;
 //   octree    the tags are cleared by the prefix-sum tiles; then one CTA per
-//             4,096-node tile (emit) and per 256-slot tile (finalize) of a
-//             cloud, reusing the single-cloud node and slot functions on
+//             4,096-node tile (emit) and one wave of CTAs over the written
+//             256-slot blocks (finalize), reusing the single-cloud functions on
 //             per-cloud views.
 //
 // The host plan (tile descriptors, cloud starts) is uploaded once; every

@@ -5,12 +5,13 @@
 // One launch in place of two stable digit passes (tile histogram, scan, ranked
 // scatter each): a key moves once more instead of twice, and its place comes
 // from smem_bin_sort instead of ballots. Two CTAs of 512 threads per SM take
-// units, even stretches of at most kBsUnit positions of a cloud, from a counter:
-// the buckets that start in a unit, as many at a time as fit shared memory. A
-// bucket that does not fit is shared by the units it covers: each counts the
-// bucket's keys by eight further bits, takes the parts that start in its
-// stretch, and gathers their keys from the whole bucket; a part that still does
-// not fit has its 2^12 values counted.
+// units, even stretches of at most kBatchUnit positions of a cloud, from a
+// counter: the buckets that start in a unit, as many at a time as fit shared
+// memory. A bucket that does not fit (bs_large) is the CTA's in whose unit it
+// starts: its keys are counted and scattered by eight further bits, and the parts
+// sorted where they then lie; a part that still does not fit has its 2^12 values
+// counted. That takes some 90 us for 49,152 keys, which is why batch_build keeps
+// larger clouds, whose buckets may be as large, to digit passes.
 #include "kernels.cuh"
 #include "smem_sort.cuh"
 
@@ -53,8 +54,8 @@ __device__ __forceinline__ void bs_each(const uint32_t* src, uint32_t cnt, F f) 
   }
 }
 
-// keys[0, cnt) (in global memory, or in M.b), whose bins follow `start` over
-// values of `span` bits below bucket id_of(key), in order to dst. lo: start's
+// keys[0, cnt) in global memory, whose bins follow `start` over values of `span`
+// bits below bucket id_of(key), in order to dst (keys or elsewhere). lo: start's
 // value at the first key.
 template <class IdOf>
 __device__ __forceinline__ void bs_sort(BsSmem& M, const uint32_t* keys, uint32_t cnt,

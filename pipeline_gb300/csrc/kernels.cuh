@@ -102,7 +102,7 @@ struct SortConfig {
   int radix_bits;  // 10 (3 passes over 30-bit keys) or 8
   int warps;       // warps per tile CTA (16)
   int items;       // keys per thread (16 or 24)
-  int scan;        // 0: decoupled look-back (OneSweep); 1: tile histograms + tile scan
+  int scan;        // 0: decoupled look-back; 1: tile histograms + tile scan
 };
 constexpr SortConfig kSortConfigDefault = {10, 16, 16, 1};
 
@@ -147,7 +147,7 @@ void set_sort_config(const SortConfig& c);
 SortConfig get_sort_config();
 
 // The whole sort of n > 1 keys on their key_bits low bits, in place (sort_once.cu;
-// the digit passes for other sort configurations and very large arrays).
+// the digit passes for other sort configurations, large arrays and uneven ones).
 // workspace: sort_keys_bytes(n, key_bits), 256-byte aligned; alt: n words.
 size_t sort_keys_bytes(int n, int key_bits);
 cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits, void* workspace,

@@ -20,9 +20,13 @@
 //             (a tag names its radix node and step) and writes the 60-byte
 //             node once, coalesced.
 //
-// Sequence tags (32-bit, larger = later):
+// Sequence tags (32-bit, larger = later), of the stage entries and of clouds above
+// kSlotTagMaxPoints points:
 //   MakeOctNodes step j of node i : ((i << 4) | j) + 1        (i < 2^27)
 //   LinkLeafNodes side s of node i: 0x80000000 | (i << 1) | s
+// Whole and batched builds take slot tags (octree.cuh), which name their values:
+// no owner tag, a mask byte per slot, and a CTA emits a tile of radix nodes that
+// bulk copies bring to shared memory.
 #include <algorithm>
 
 #include "octree.cuh"

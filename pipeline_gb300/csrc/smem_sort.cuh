@@ -1,5 +1,6 @@
-// Shared-memory sorting of one CTA's keys: the bucket kernels of the learned
-// sort and the fused build.
+// Shared-memory sorting of one CTA's keys: the one-launch build and sort, the
+// bucket sort of batched builds (bins), the bucket kernels of the learned sort and
+// the digit passes of the one-launch sort (radix).
 #pragma once
 
 #include "common.cuh"
@@ -379,7 +380,7 @@ __device__ __forceinline__ void smem_sort_bins(uint32_t* k, const uint32_t* star
 // key to within its bin's size of its place. Where a bin has more than kBinCut
 // keys, every bin is cut into as many as it has keys, and the keys are counted
 // once more: what is large after that is mostly one value. aux: kBinAux words,
-// s_span: two; the keys may lie in b.
+// s_span: two.
 // (By 1,024 threads 16,384 even keys take 13 us; 22 us with comparisons within
 // the bins and a scan of 16 bins per thread.)
 template <int WARPS, int ITEMS, class PlaceOf>

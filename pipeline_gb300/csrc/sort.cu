@@ -5,15 +5,17 @@
 // (include/kernels/02_sort.hpp:6-7, kernels/02_sort.cpp:13-118; GPU form
 // kernels/cuda/02_sort.cu:208-338, 566-792).
 //
-// Design: the Morton kernel reads the points once with 128-bit streaming loads
-// and, in the same pass, builds the digit histograms of every sort pass in
-// shared memory (so the sort needs no separate histogram read). The sort is a
-// single-pass-per-digit "OneSweep" LSD radix sort: each tile ranks its keys
-// with warp multi-split (match.any), publishes its per-digit counts, resolves
-// its global digit offsets by decoupled look-back over earlier tiles, stages
-// the keys in shared memory in digit order and scatters them in runs.
-// 30-bit Morton keys take 3 passes of 10-bit digits (28 B/key of HBM traffic
-// including the histogram read) instead of the reference's 4 passes of 8.
+// The Morton kernel reads the points once with 128-bit streaming loads and, where
+// a digit pass or the MSD form needs them, counts digits of the codes in shared
+// memory on the way. The digit passes here sort what the other forms do not take
+// (sort_once.cu: arrays up to 4M keys, even ones to 8.4M; msd.cu: large clouds;
+// fused.cu, batch_sort.cu, lsort.cu): other sort shapes, large arrays, uneven large
+// clouds, batches of larger clouds. A tile ranks its keys by warp multi-split from
+// ballots (a first pass by shared-memory atomics), finds its digits' places from a
+// tile histogram and scan, by look-back over earlier tiles, or (a first pass) from
+// bucket cursors, stages the keys in shared memory in digit order and writes them
+// in runs. 30-bit Morton keys take 3 passes of 10-bit digits instead of the
+// reference's 4 passes of 8.
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
@@ -196,12 +198,13 @@ __global__ void __launch_bounds__(1024) hist_scan_kernel(const uint32_t* __restr
 //   !STABLE one shared-memory atomicAdd per key: any order. Only the first
 //           LSD pass may use it (its input order carries no information).
 // Tile offsets (where the tile's keys of each digit start in the output):
-//   SCAN 0  decoupled look-back over earlier tiles (OneSweep): a tile takes
-//           the next id from an atomic counter, publishes its per-digit
+//   SCAN 0  decoupled look-back over earlier tiles: a CTA takes tile after
+//           tile from an atomic counter, publishes its per-digit
 //           counts, sums earlier tiles' counts back to an inclusive prefix
 //           (bounded waits, windowed relaxed loads).
 //   SCAN 1  precomputed: a per-tile digit histogram kernel and a tile-prefix
 //           scan ran before the pass (reduce-then-scan); no inter-tile waits.
+//           A first pass may take cursors instead (DigitAlt).
 //   lookback[tile * BINS + b]: bits 31..30 flag (0 not ready, 1 tile count,
 //   2 inclusive count of tiles 0..tile), bits 29..0 the count.
 // --------------------------------------------------------------------------

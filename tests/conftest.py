@@ -50,3 +50,15 @@ def small_cases(golden):
                 case[key.split("__", 1)[1]] = z[key]
         out[name] = case
     return out
+
+
+def cell_centres(codes):
+    """Points at the centres of Morton cells (unit cells of a 1024 box)."""
+    codes = np.asarray(codes, np.int64)
+    pts = np.ones((len(codes), 4), np.float32)
+    for axis in range(3):
+        cell = np.zeros(len(codes), np.int64)
+        for bit in range(10):
+            cell |= ((codes >> (3 * bit + axis)) & 1) << bit
+        pts[:, axis] = cell + 0.5
+    return pts

@@ -9,23 +9,13 @@ import numpy as np
 import pytest
 import torch
 
+from conftest import cell_centres
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 KEYS = ["sorted_unique", "prefix_n", "has_leaf_left", "has_leaf_right", "left_child", "parent",
         "edge_count", "prefix_sum", "oct_nodes"]
 CUT = 32768  # codes of a top-12-bit bucket (2^18 values)
-
-
-def points(codes):
-    codes = np.asarray(codes, np.int64)
-    pts = np.ones((len(codes), 4), np.float32)
-    for axis in range(3):
-        cell = np.zeros(len(codes), np.int64)
-        for bit in range(10):
-            cell |= ((codes >> (3 * bit + axis)) & 1) << bit
-        pts[:, axis] = cell + 0.5
-    return pts
 
 
 def cloud(kind, n, rng):
@@ -50,7 +40,7 @@ def cloud(kind, n, rng):
         codes = np.concatenate([(b << 18) + rng.integers(0, 1 << s, n // 6)
                                 for b, s in ((0, 18), (1, 9), (2, 18), (4000, 15))]
                                + [rng.integers(0, 1 << 30, n // 3)])
-    return points(rng.permutation(codes))
+    return cell_centres(rng.permutation(codes))
 
 
 def build(pts, timed=False):
@@ -116,5 +106,5 @@ def build_us(pts):
 def test_a_cloud_in_a_corner_costs_no_more_than_twice_an_even_one(kind, n):
     """(One CTA that took a whole bucket: three to seven times.)"""
     rng = np.random.default_rng(1)
-    even = points(rng.integers(0, 1 << 30, n))
+    even = cell_centres(rng.integers(0, 1 << 30, n))
     assert build_us(cloud(kind, n, rng)) < 2 * build_us(even)

@@ -275,10 +275,9 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem<THREADS, ITEMS>& S,
     }
     clear_mask_range(t, (int)ex, (int)hi, tid, THREADS);
   }
-  // (Bounds on run and v: counts of a malformed tree, see emit_slots.)
-  // a tile covers at most its nodes' slots; more than the stage holds only
-  // when many nodes span several levels
-  const bool staged = total <= (uint32_t)kTile;
+  // (Bounds on run, v and total: counts of a malformed tree, see emit_slots.)
+  // The stage takes the tile's slots; there are more than it holds only when many
+  // nodes span several levels, and it then takes them kTile at a time.
   uint32_t run = ex + off;
   int mx = 0;
   uint32_t multi = 0;  // items that span several levels
@@ -298,25 +297,13 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem<THREADS, ITEMS>& S,
     if (i == n - 1) mx = max(mx, (int)run);
   }
   // further steps, one such node of each lane at a time
-  while (staged && multi) {
+  while (multi) {
     const int j = tid * items + __ffs(multi) - 1;
     multi &= multi - 1u;
     const uint32_t q = (uint32_t)S.v[pf_pad(j)] - ex - 1u;
     const uint32_t k = (uint32_t)min(ec[lo + j], kMaxSteps);
-    for (uint32_t h = 1; h < k && q + h < total; ++h)
+    for (uint32_t h = 1; h < k && q + h < min(total, (uint32_t)kTile); ++h)
       atomicMax(&S.node[q + h], ((uint32_t)(j + 1) << 4) | h);
-  }
-  if (!staged) {
-    // the node's own slot only, none for those up to the one before it
-#pragma unroll 1
-    for (int k = 0; k < items; ++k) {
-      const int j = tid * items + k;
-      const uint32_t r = (uint32_t)S.v[pf_pad(j)];
-      const int kk = j < valid && lo + j > 0 ? min(ec[lo + j], kMaxSteps) : 0;
-      for (int h = 1; h < kk; ++h)
-        if (r - (uint32_t)h < cap) t.node[r - (uint32_t)h] = 0u;
-      if (kk > 0 && r < cap) t.node[r] = (uint32_t)(lo + j) << 4;
-    }
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
   if ((tid & 31) == 0 && mx > 0) atomicMax(&S.max_slot, mx);
@@ -328,13 +315,38 @@ __device__ __forceinline__ void prefix_slots_tile(PrefixSmem<THREADS, ITEMS>& S,
     const int j = k * THREADS + tid;
     if (j < valid) ps[lo + j] = S.v[pf_pad(j)];
   }
-  if (staged) {
-    for (uint32_t q = tid; q < total; q += THREADS) {
-      const uint32_t slot = ex + 1u + q;
-      const uint32_t e = S.node[q];
-      // the tile before may reach its first few slots: left open
-      const uint32_t none = q < (uint32_t)kMaxSteps && lo > 0 ? 0u : kNoNode;
-      if (slot < cap) t.node[slot] = e ? e + ((uint32_t)(lo - 1) << 4) : none;
+  for (uint32_t q = tid; q < min(total, (uint32_t)kTile); q += THREADS) {
+    const uint32_t slot = ex + 1u + q;
+    const uint32_t e = S.node[q];
+    // the tile before may reach its first few slots: left open
+    const uint32_t none = q < (uint32_t)kMaxSteps && lo > 0 ? 0u : kNoNode;
+    if (slot < cap) t.node[slot] = e ? e + ((uint32_t)(lo - 1) << 4) : none;
+  }
+  // (6M points in pairs of neighbours: 127 us and 215 in finalize when such a tile
+  // left its slots to finalize's search, 88 and 153 this way)
+#pragma unroll 1
+  for (uint32_t w = kTile; w < min(total, (uint32_t)(kTile * kMaxSteps)); w += kTile) {
+    __syncthreads();
+    for (int q = tid; q < kTile / 4; q += THREADS)
+      reinterpret_cast<uint4*>(S.node)[q] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < items; ++k) {
+      const int j = tid * items + k;
+      if (j >= valid || lo + j == 0) continue;
+      const uint32_t q = (uint32_t)S.v[pf_pad(j)] - ex - 1u;
+      if (q >= w + (uint32_t)kTile || q + (uint32_t)kMaxSteps <= w) continue;
+      const int steps = min(ec[lo + j], kMaxSteps);
+      for (int h = 0; h < steps; ++h) {
+        const uint32_t s = q + (uint32_t)h;
+        if (s - w < (uint32_t)kTile && s < total)
+          atomicMax(&S.node[s - w], ((uint32_t)(j + 1) << 4) | (uint32_t)h);
+      }
+    }
+    __syncthreads();
+    for (uint32_t q = tid; q < min(total - w, (uint32_t)kTile); q += THREADS) {
+      const uint32_t slot = ex + 1u + w + q, e = S.node[q];
+      if (slot < cap) t.node[slot] = e ? e + ((uint32_t)(lo - 1) << 4) : kNoNode;
     }
   }
   // slot 0 (the root's) and the slots after the last node's prefix have none
@@ -580,8 +592,8 @@ __device__ __forceinline__ void finalize_slots(int p, const OctArgs& a, const Sl
   const uint32_t m = t.mask[(uint32_t)t.at + (uint32_t)p];
   uint32_t own = p > 0 ? t.node[p] : 0u;
   if (own == 0u && p > 0) {
-    // not in a tile's own slots (a tile's first few, or one with more slots
-    // than it stages): the nearest node before it whose slots reach p
+    // not in a tile's own slots (a tile's first few): the nearest node before it
+    // whose slots reach p
     for (int d = 1; d < kMaxSteps && d < p; ++d) {
       const uint32_t e = t.node[p - d];
       if ((e & 15u) == 0u && e != 0u && a.counts[min(e >> 4, last)] > d) {

@@ -34,6 +34,9 @@ def cloud(kind, n, rng):
     elif kind == "few values":
         codes = np.concatenate([rng.choice(low + rng.integers(0, 1 << 18, 3), n - n // 4),
                                 rng.integers(0, 1 << 30, n // 4)])
+    elif kind == "pairs":  # nodes that span several levels: more slots than a tile has nodes
+        codes = rng.integers(0, 1 << 27, n // 2) << 3
+        codes = np.concatenate([codes, codes | 1])
     elif kind == "last bucket":
         codes = (4095 << 18) + (1 << 18) - 1 - rng.integers(0, 1 << 17, n)
     else:  # a few buckets, sparse and dense, and scattered codes
@@ -60,7 +63,8 @@ def build(pts, timed=False):
     return b.result()
 
 
-KINDS = ["at the cut", "one bucket", "dense", "dense part", "few values", "last bucket", "mixed"]
+KINDS = ["at the cut", "one bucket", "dense", "dense part", "few values", "pairs", "last bucket",
+         "mixed"]
 
 
 @pytest.mark.parametrize("kind", KINDS)

@@ -59,13 +59,20 @@ constexpr int kSoMinPer = 1024;   // keys per CTA at least
 // 1% of the passes alone). Larger arrays take passes alone (16.7M: even keys would
 // gain an eighth, uneven ones lose 4%).
 constexpr int kSoAny = 4000000;
+// Keys of one digit (10 bits) take a single launched pass, as fast for any of them
+// (45 us up to 250,000, 54 at 1M): the launch is faster for even ones (26 to 50) but
+// not where a value holds half of them or more (35 to 66), so it takes arrays up to
+// kSoOneDigit, those of one cluster. Two digits are worth it throughout: 70 us up to
+// 250,000 by passes and 24 to 72 here, 81 at 1.5M and 38 to 72.
+constexpr int kSoOneDigit = kSoMaxCluster * kSoMinPer;
 constexpr int kSoEven = 1 << 23;
 // The look: 1,024 keys of the array. Few values hold much of it if more than kSoFew
 // are alike in all but 12 bits; such keys take the digit passes in here at once, not
-// after two counts (20 us of 155 at 4M; fewer than kSoLook keys lose little). It is
-// uneven, for kSoEven, if more than kSoTopMost are alike in the top 10 bits or
-// kSoPairs meet another in a cell of 2^12 values (even keys: 32 by the table's size).
-constexpr int kSoLook = 1 << 21;
+// after two counts (20 us of 155 at 4M and of 106 at 1.5M; even keys lose 1 us, and
+// smaller arrays little by the counts). It is uneven, for kSoEven, if more than
+// kSoTopMost are alike in the top 10 bits or kSoPairs meet another in a cell of 2^12
+// values (even keys: 32 by the table's size).
+constexpr int kSoLook = 1 << 20;
 constexpr uint32_t kSoFew = 16;
 constexpr uint32_t kSoTopMost = 14;
 constexpr int kSoPairs = 80;
@@ -555,12 +562,12 @@ cudaError_t launch_sort_keys(uint32_t* keys, uint32_t* alt, int n, int key_bits,
   const int low_bits = std::min(32, p.passes * p.radix_bits);
   char* w = static_cast<char*>(workspace);
   uint32_t* result = keys;
-  if (sort_once_takes(n, kSoAny)) {
+  if (sort_once_takes(n, p.passes > 1 ? kSoAny : kSoOneDigit)) {
     const cudaError_t e =
         launch_sort_once(keys, alt, n, key_bits, low_bits, w, w + L.zero_bytes, status, s);
     if (e != cudaErrorCooperativeLaunchTooLarge) return e;
     (void)cudaGetLastError();  // a context with fewer SMs: the passes
-  } else if (sort_once_takes(n, kSoEven) && sort_few_ok(p)) {
+  } else if (n > kSoAny && sort_once_takes(n, kSoEven) && sort_few_ok(p)) {
     char* plan = w + align_up(L.zero_bytes, 256);
     char* rest = plan + align_up(p.bytes, 256);
     uint32_t* defer = reinterpret_cast<uint32_t*>(w) + 3;

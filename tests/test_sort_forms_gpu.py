@@ -124,6 +124,31 @@ def test_few_values_sort_like_torch(kind, n):
         assert int(status[0]) == 0 and torch.equal(keys, want)
 
 
+def narrow(kind, n, bits):
+    g = torch.Generator(device="cuda").manual_seed(4)
+    some = torch.randint(0, 1 << bits, (n,), generator=g, device="cuda")
+    share = torch.rand(n, generator=g, device="cuda")
+    part = {"even": 0.0, "half": 0.5, "nine tenths": 0.9, "one value": 1.0}[kind]
+    return torch.where(share < part, torch.full_like(some, 3), some).to(torch.int32)
+
+
+@pytest.mark.parametrize("bits", [4, 8, 10, 11, 16, 20])
+@pytest.mark.parametrize("kind", ["even", "half", "nine tenths", "one value"])
+def test_sorts_of_narrow_keys(kind, bits):
+    """One and two digit passes are little to be faster than: sizes on both sides of a
+    cluster's, of the first look's, and near the largest array of one launch."""
+    from pipeline_gb300.kernels import k_SimpleRadixSort
+
+    for n in (8192, 8193, 16_000, 130_000, 1 << 20, (1 << 20) + 1, 1_800_000, 3_900_000):
+        src = narrow(kind, n, bits)
+        keys, alt = src.clone(), torch.empty_like(src)
+        k_SimpleRadixSort(keys, alt, n, key_bits=bits)
+        assert torch.equal(keys, torch.sort(src).values)
+        with passes():
+            want = sort_us(src, bits)
+        assert sort_us(src, bits) < MARGIN * want, n
+
+
 def build_us(pts):
     from pipeline_gb300.pipeline import OctreeBuilder
 

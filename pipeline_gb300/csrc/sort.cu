@@ -9,13 +9,13 @@
 // a digit pass or the MSD form needs them, counts digits of the codes in shared
 // memory on the way. The digit passes here sort what the other forms do not take
 // (sort_once.cu: arrays up to 4M keys, even ones to 8.4M; msd.cu: large clouds;
-// fused.cu, batch_sort.cu, lsort.cu): other sort shapes, large arrays, uneven large
-// clouds, batches of larger clouds. A tile ranks its keys by warp multi-split from
-// ballots (a first pass by shared-memory atomics), finds its digits' places from a
-// tile histogram and scan, by look-back over earlier tiles, or (a first pass) from
-// bucket cursors, stages the keys in shared memory in digit order and writes them
-// in runs. 30-bit Morton keys take 3 passes of 10-bit digits instead of the
-// reference's 4 passes of 8.
+// fused.cu, batch_sort.cu, lsort.cu): other sort shapes, keys of one digit, large
+// arrays, uneven large clouds, batches of larger clouds. A tile ranks its keys by
+// warp multi-split from ballots (a first pass by shared-memory atomics), finds its
+// digits' places from a tile histogram and scan, by look-back over earlier tiles, or
+// (a first pass) from bucket cursors, stages the keys in shared memory in digit order
+// and writes them in runs. 30-bit Morton keys take 3 passes of 10-bit digits instead
+// of the reference's 4 passes of 8.
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>

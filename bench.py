@@ -498,10 +498,10 @@ def build_launches(n: int = 0) -> int:
     12,288 points per SM: one. Otherwise stages 2-3, then tree nodes, tile-sum
     scan + prefix sum (which clears the octree tags), octree emit/finalize and
     counts. Stages 2-3: Morton, the one-launch sort and unique (run-head count,
-    their scan, compaction with the deltas); past 4,000,000 points and for other
-    sort shapes digit passes in place of the one-launch sort (base scan, per
-    pass a tile histogram + tile scan and the pass), from 2^22 points on with the
-    MSD form beside them (form gate, bucket bitmaps, pack scan + pack; the first
+    their scan, compaction with the deltas); for other sort shapes and from 2^22
+    points on digit passes in place of the one-launch sort (base scan, per pass
+    a tile histogram + tile scan and the pass), with the MSD form beside them
+    from 2^22 points on (form gate, bucket bitmaps, pack scan + pack; the first
     pass doubles as the top-digit scatter), there up to 2^24 points as one
     launch of counts and bases and three passes."""
     import torch
@@ -514,7 +514,7 @@ def build_launches(n: int = 0) -> int:
     passes = (30 + rb - 1) // rb
     default = (rb, warps, items, scan) == (10, 16, 16, 1)
     msd = n >= (1 << 22) and rb == 10 and passes == 3 and scan == 1
-    if default and n <= 4_000_000:
+    if default and not msd:
         sort = 1
     elif default and msd and n <= (1 << 24):
         sort = 1 + passes

@@ -59,6 +59,11 @@ constexpr int kSoMinPer = 1024;   // keys per CTA at least
 // 1% of the passes alone). Larger arrays take passes alone (16.7M: even keys would
 // gain an eighth, uneven ones lose 4%).
 constexpr int kSoAny = 4000000;
+// Whole builds take it to where the MSD form begins (4,190,000 points, build: even 373
+// us by passes and 299, codes around 64 centres 357 and 333, a few values 240 and 234;
+// at that end alone a cloud in one sixteenth of one axis has its 256 buckets just above
+// what a CTA sorts: 313 and 336, at 4.1M 307 and 274).
+constexpr int kSoBuild = (1 << 22) - 1;
 // Keys of one digit (10 bits) take a single launched pass, as fast for any of them
 // (45 us up to 250,000, 54 at 1M): the launch is faster for even ones (26 to 50) but
 // not where a value holds half of them or more (35 to 66), so it takes arrays up to
@@ -609,7 +614,7 @@ cudaError_t launch_diag_grid_wait(void* workspace, uint32_t* status, unsigned lo
 
 bool sort_once_in_plan(const SortPlan& p) {
   const SoLayout L = so_layout(p.n);
-  return sort_once_takes(p.n, kSoAny) && msd_plan_ok(p) &&
+  return sort_once_takes(p.n, kSoBuild) && msd_plan_ok(p) &&
          p.zero_bytes - p.tile_part_off >= 2 * align_up(L.zero_bytes, 256) &&
          p.bytes - p.tile_hist_off >= L.total - L.zero_bytes;
 }

@@ -173,6 +173,25 @@ def test_builds_of_clouds_that_the_msd_form_refuses(kind, n):
     assert build_us(pts) < MARGIN * want
 
 
+@pytest.mark.parametrize("kind,most", [("even", 0.9), ("nine tenths", MARGIN), ("lumps", 0.9)])
+@pytest.mark.parametrize("n", [4_000_001, (1 << 22) - 1])
+def test_builds_up_to_the_msd_size_take_one_sort(kind, most, n):
+    """Between the sizes from which sorts alone may take passes and builds the MSD form."""
+    from pipeline_gb300.pipeline import OctreeBuilder
+
+    pts = points(codes(kind, n))
+
+    def nodes():
+        b = OctreeBuilder(n)
+        b.build(pts, 0.0, 1024.0)
+        return b.result()["oct_nodes"].tobytes()
+
+    with passes():
+        want, tree = build_us(pts), nodes()
+    assert nodes() == tree
+    assert build_us(pts) < most * want
+
+
 @pytest.mark.parametrize("kind", ["nine tenths", "one bucket"])
 @pytest.mark.parametrize("n", [1_000_000, 8_300_000, 16_700_000])
 def test_learned_builds_whose_model_does_not_fit(kind, n):
